@@ -143,6 +143,7 @@ struct vfem_problem {
     // constants for the kernels
     double op64[45 + 576];
     float op32[45 + 576];
+    FxOperand fx;  // the structured FP64 product in block fixed point (matvec_fx.cu)
     // the tensor-core FP32 CG product (matvec_tc.cu), opt-in, when Ke admits an exact BF16 scaling
     TcOperand tc;
     bool tcReady = false;
@@ -705,6 +706,7 @@ vfem_status createImpl(const uint8_t* vox, int nx, int ny, int nz, const double*
         p->op64[45 + i] = p->ke.Ke[i];
         p->op32[45 + i] = (float)p->ke.Ke[i];
     }
+    fxPrepare(p->ke, p->fx);
     auto bail = [&](vfem_status s) {
         freeProblem(p);
         return s;
@@ -718,6 +720,7 @@ vfem_status createImpl(const uint8_t* vox, int nx, int ny, int nz, const double*
     } while (0)
     CKP(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
     CKP(setKernelAttributes());
+    CKP(fxSetAttributes());
     // VFEM_TENSOR_CORE_PRODUCT=1: the FP32 CG product on the tensor cores (slower
     // than the CUDA-core kernel on GB300; kept as a measured alternative)
     p->tcReady = envInt("VFEM_TENSOR_CORE_PRODUCT", 0) != 0 && tcPrepare(p->ke.Ke, p->tc) &&
@@ -835,6 +838,11 @@ template <typename T>
 int matvec(vfem_problem* p, const MatvecArgs<T>& a, bool allowTc = true) {
     if constexpr (std::is_same<T, float>::value) {
         if (allowTc && p->tcReady && tcEligible(a)) return launchMatvecTC(ctx(p), a, p->tc);
+    } else {
+        if (fxEligible(p->fx, a.scale)) {
+            launchMatvecFx(p->stream, a, p->fx, p->op64, p->S, p->rb);
+            return 1;
+        }
     }
     return launchMatvec<T>(ctx(p), a, p->ke.structured, opc<T>(p));
 }
@@ -1534,7 +1542,7 @@ vfem_status vfem_apply_operator_device_noalloc(vfem_problem* p, const double* x_
     CK(cudaSetDevice(p->device));  // the scratch set-up below runs with the problem's device current
     MatvecArgs<double> a = mvArgs<double>(p, 0, x_device, y_device, MV_AX);
     bool tooLarge = false;
-    CK(launchMatvecNoAlloc(static_cast<cudaStream_t>(stream), a, p->ke.structured, p->op64, xKx_device, &tooLarge));
+    CK(launchMatvecNoAlloc(static_cast<cudaStream_t>(stream), a, p->ke.structured, p->op64, p->fx, xKx_device, &tooLarge));
     if (tooLarge)
         return fail(VFEM_ERR_INVALID_ARGUMENT,
                     "grid too large for the no-allocation scratch (at most 65536 product blocks of 31x7x32 "

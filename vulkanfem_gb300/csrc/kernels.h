@@ -123,6 +123,20 @@ cudaError_t setKernelAttributes();
 template <typename T>
 int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, const void* opconst);
 
+// The structured FP64 product in block fixed point (matvec_fx.cu): the cube's
+// 8 constants as 62-bit integers.  fxEligible: the operand is ready and `scale` a power of two.
+struct FxOperand {
+    int32_t k1[8], k0[8];
+    int outExp;
+    bool ready = false;
+};
+bool fxPrepare(const KeData& ke, FxOperand& op);
+cudaError_t fxSetAttributes();
+bool fxEligible(const FxOperand& op, double scale);
+int fxLayers(const Grid& g);  // node layers a block marches
+void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOperand& op, const double* ks,
+                    Scalars* S, const RedBuf& rb);
+
 // The same product on FP64 vectors in double-float arithmetic (FP32 instructions,
 // ~48-bit significands): the mixed-precision true residual.  a.y may be null.
 int launchMatvecDF(const LaunchCtx& c, const MatvecArgs<double>& a, bool structured, const double* opconst);
@@ -258,7 +272,7 @@ int launchInitScalars(cudaStream_t s, Scalars* S, double tol, long long maxIter,
 // nothing launched) when the product's grid needs more reduction blocks than
 // the array holds.  xKx is a device pointer.
 cudaError_t launchMatvecNoAlloc(cudaStream_t s, const MatvecArgs<double>& a, bool structured, const void* opconst,
-                                double* xKx, bool* tooLarge);
+                                const FxOperand& fx, double* xKx, bool* tooLarge);
 
 // Tensor-core FP32 CG product (matvec_tc.cu): B = q Ke in BF16 as K-major core
 // matrices, invScale = 1 / q.  tcPrepare fails (false) when no integer

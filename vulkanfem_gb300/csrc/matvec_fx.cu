@@ -1,0 +1,499 @@
+// matvec_fx.cu -- the structured FP64 product in block fixed point.
+//
+// GB300 issues FP64 at 1/64 of its FP32 rate: measured 1.7 FP64 operations per
+// clock and SM against 58 64-bit integer additions and 29 multiply-adds 32 x 32
+// -> 64.  The FP64 march (walshMarch, matvec_march.cuh) is bound by its ~190
+// FP64 operations per element.  This kernel does the same element product in
+// 64-bit integers and leaves three conversions and the dot of a node to the
+// FP64 pipe.  Measured on a 191^3 grid with voids and log-normal moduli:
+// 3.72 -> 0.49 ms; on 33 x 17 x 17 nodes 262 -> 20 us (of it 262 -> 25 us from
+// this form with the shorter marches of fxLayers).  Bound now: instruction
+// issue (1,100 warp instructions per element row, 59% of the issue slots, ALU
+// 56%, wide multiply-adds 54% of their pipe), two 8-warp blocks per SM for
+// their registers.  Tiles of 12 rows in one block per SM (168 registers) or 6
+// rows in two measured 14% slower.
+//
+// Numbers.  A node's three components are staged as 58-bit integers under the
+// node's largest exponent.  An element reads its 24 values on a grid S with
+// S - 3 <= (exponent of its largest value) <= S and 2^-57 of 2^S as the unit;
+// the Walsh transforms are then exact.  The largest of the 20 combinations that
+// Khat scales is shifted up to 2^61..2^62 (lz), multiplied by 62-bit constants
+// in two 32-bit digits, and by the modulus' 24-bit significand, with rounding;
+// what leaves the element has the unit 2^(O + 9 - f), O = S + exponent(E) - lz,
+// at most 2^-56 of C E times that largest combination (C, f: fxPrepare).
+// Outputs with different O are aligned to the larger one where they meet.
+// Against 113-bit arithmetic the result's relative error is 3e-16 to 6e-16
+// (random, smooth, graded and point vectors, moduli 1, log-normal or spread
+// over e^20), where the FP64 march has 5e-16 to 4e-15.
+//
+// No sum can overflow: the combinations are below 2^62, so a component's corner
+// value is at most C 2^f 2^62 / 2^64 / 2 <= 2^59 per element, and a node sums 8
+// of them; sums in between are taken modulo 2^64.  Values the grid cannot take
+// (non-finite ones or exponents beyond 2^+-575 next to a filled voxel, subnormal
+// moduli) make the block repeat its march in FP64, so that results for those
+// are what the FP64 march gives.
+#include <cmath>
+
+#include "matvec_march.cuh"
+
+namespace vfem {
+
+namespace {
+
+constexpr int FX_EMIN = 448, FX_EMAX = 1600;  // biased exponents the integer march takes
+constexpr int FX_BAD = 4000;                  // a node outside of them
+constexpr int FX_NONE = -(1 << 20);           // exponent of a zero contribution
+constexpr int FX_SLACK = 3;
+
+struct FxArgs {
+    long long kb[8];   // start of a middle digit sum: 2^31 (rounding) + 2^31 k1
+    int k1[8], k0[8];  // the cube's constants (fxPrepare) times 2^f = k1 2^32 + k0, signed digits
+    int scaleExp;        // log2 of the level's operator scale
+    int outExp;          // exponent-field offset of an output at O
+};
+
+struct FxNode {
+    long long v[3];
+    int e;
+};
+
+// Three FP64 components on their common grid.
+__device__ __forceinline__ FxNode fxNode(double x, double y, double z) {
+    const double d[3] = {x, y, z};
+    FxNode n;
+    int e = 0, ec[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        ec[c] = (__double2hiint(d[c]) >> 20) & 0x7ff;
+        e = max(e, ec[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const int hi = __double2hiint(d[c]);
+        const unsigned long long m =
+            (((unsigned long long)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(d[c])) << 5;
+        // a zero or subnormal component (field 0) is shifted out: e >= FX_EMIN below
+        const unsigned long long q = m >> min(e - ec[c], 63);
+        const long long s = (long long)(hi >> 31);
+        n.v[c] = ((long long)q ^ s) - s;
+    }
+    if ((unsigned)(e - FX_EMIN) > (unsigned)(FX_EMAX - FX_EMIN)) {
+        const bool zero = (((__double2hiint(x) | __double2hiint(y) | __double2hiint(z)) & 0x7fffffff) |
+                           __double2loint(x) | __double2loint(y) | __double2loint(z)) == 0;
+        n.v[0] = n.v[1] = n.v[2] = 0;
+        e = zero ? 0 : FX_BAD;
+    }
+    n.e = e;
+    return n;
+}
+
+__device__ __forceinline__ long long fxShr(long long v, int by) { return v >> (int)min((unsigned)by, 63u); }
+
+__device__ __forceinline__ void fwht4x3i(long long (&v)[12]) {
+#pragma unroll
+    for (int s = 1; s < 4; s <<= 1)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (q & s) continue;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const long long p = v[3 * q + c], r = v[3 * (q + s) + c];
+                v[3 * q + c] = p + r;
+                v[3 * (q + s) + c] = p - r;
+            }
+        }
+}
+
+template <int TY>
+constexpr size_t fxSmemBytes() {
+    // staged nodes (two layers) and exported corners (three), 32 bytes each; the
+    // FP64 march of a block that falls back uses the same memory
+    constexpr size_t fx = 32 * (2 * (size_t)(TY + 1) * (MV_TX + 1) + 3 * (size_t)TY * MV_TX);
+    constexpr size_t fp = (size_t)(kSuElems + kSyElems) * sizeof(double);
+    return fx > fp ? fx : fp;
+}
+
+// One block's march, the counterpart of walshMarch<double, double, OUT> with the
+// same tile, halo and pipelining.  Returns true when a value did not fit (the
+// outputs and dots are then to be recomputed).
+template <int OUT, int TY>
+__device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const FxArgs& K, int zc, unsigned char* smem,
+                                        DotAcc<double>& d0, DotAcc<double>& d1) {
+    // 16-byte halves of the 32-byte slots in arrays of their own: conflict-free
+    longlong2* suA = reinterpret_cast<longlong2*>(smem);           // {v0, v1}
+    longlong2* suB = suA + 2 * (TY + 1) * (MV_TX + 1);             // {v2, exponent}
+    longlong2* syA = suB + 2 * (TY + 1) * (MV_TX + 1);
+    longlong2* syB = syA + 3 * TY * MV_TX;
+    const Grid g = a.g;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int x0 = blockIdx.x * (MV_TX - 1), y0 = blockIdx.y * (TY - 1), z0 = blockIdx.z * zc;
+    const int zend = min(z0 + zc, g.nz);
+    const int64_t plane = (int64_t)g.nx * g.ny;
+    const int ecx = x0 + tx - 1, ecy = y0 + ty - 1;
+    const int onx = x0 + tx, ony = y0 + ty;
+    const bool owner = (tx < MV_TX - 1) && (ty < TY - 1) && onx < g.nx && ony < g.ny;
+    const bool ecxy = ecx >= 0 && ecx < g.ex && ecy >= 0 && ecy < g.ey;
+    const int eCol = ecy * g.nx + ecx, oCol = ony * g.nx + onx;
+    // the tile's extra row (ty == 0 threads) and column (row-1 threads): at most one extra node a thread
+    const bool hasR = ty == 0, hasC = (ty == 1) && (tx <= TY);
+    const int exX = hasR ? x0 - 1 + tx : x0 - 1 + MV_TX, exY = hasR ? y0 - 1 + TY : y0 - 1 + tx;
+    const int exSlot = hasR ? TY * (MV_TX + 1) + tx : tx * (MV_TX + 1) + MV_TX;
+    const bool hasX = hasR || hasC;
+    const bool ok0 = ecx >= 0 && ecx < g.nx && ecy >= 0 && ecy < g.ny;
+    const bool okX = hasX && exX >= 0 && exX < g.nx && exY >= 0 && exY < g.ny;
+    const int exCol = exY * g.nx + exX;
+#define SLOT(b, iy, ix) (((b) * (TY + 1) + (iy)) * (MV_TX + 1) + (ix))
+#define YSLOT(k, iy, ix) (((k) * TY + (iy)) * MV_TX + (ix))
+    double pf[6];
+    auto gload = [&](int zl) {
+        const bool zok = zl >= 0 && zl < g.nz;
+        const int64_t zoff = (int64_t)zl * plane;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) pf[i] = 0.0;
+        if (ok0 && zok) {
+            const double* p = a.x + 3 * ((int64_t)eCol + zoff);
+            pf[0] = p[0]; pf[1] = p[1]; pf[2] = p[2];
+        }
+        if (okX && zok) {
+            const double* p = a.x + 3 * ((int64_t)exCol + zoff);
+            pf[3] = p[0]; pf[4] = p[1]; pf[5] = p[2];
+        }
+    };
+    auto put = [&](int slot, const FxNode& n) {
+        suA[slot] = make_longlong2(n.v[0], n.v[1]);
+        suB[slot] = make_longlong2(n.v[2], n.e);
+    };
+    auto sstore = [&](int zl) {
+        const int b = zl & 1;
+        put(SLOT(b, ty, tx), fxNode(pf[0], pf[1], pf[2]));
+        if (hasX) put(SLOT(b, 0, 0) + exSlot, fxNode(pf[3], pf[4], pf[5]));
+    };
+    auto eload = [&](int k) -> float {
+        return (ecxy && k >= 0 && k < g.ez) ? a.E[(int64_t)eCol + (int64_t)k * plane] : 0.f;
+    };
+    auto fload = [&](int k) -> uint8_t {
+        return (owner && k >= z0 && k < zend) ? a.flags[(int64_t)oCol + (int64_t)k * plane] : (uint8_t)0;
+    };
+    // A staged node layer's quad: the second halves of its slots, the largest exponent ...
+    auto quadB = [&](int b, longlong2 (&vb)[4]) {
+        int e = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            vb[q] = suB[SLOT(b, ty + (q >> 1), tx + (q & 1))];
+            e = max(e, (int)vb[q].y);
+        }
+        return e;
+    };
+    // ... and its Walsh transform on the grid S.
+    auto quad = [&](int b, int S, const longlong2 (&vb)[4], long long (&v)[12]) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const longlong2 va = suA[SLOT(b, ty + (q >> 1), tx + (q & 1))];
+            const int by = S - (int)vb[q].y;
+            v[3 * q] = fxShr(va.x, by);
+            v[3 * q + 1] = fxShr(va.y, by);
+            v[3 * q + 2] = fxShr(vb[q].x, by);
+        }
+        fwht4x3i(v);
+    };
+    long long qb[12], carry[12];  // bottom quad and the previous element's top-face output, Walsh domain
+#pragma unroll
+    for (int i = 0; i < 12; ++i) qb[i] = carry[i] = 0;
+    int S = 0, qS = -1, eb = 0, cO = FX_NONE;  // grid, the grid qb is on (-1: none), exponent of qb, of the carry
+    bool bad = false;
+    double dAx = 0.0;
+    gload(z0 - 1);
+    sstore(z0 - 1);
+    gload(z0);
+    float Enext = eload(z0 - 1);
+    uint8_t flNext = fload(z0 - 1);
+    for (int k = z0 - 1; k < zend; ++k) {
+        sstore(k + 1);
+        const float Ee = Enext;
+        const uint8_t fl = flNext;
+        __syncthreads();
+        gload(k + 2);
+        Enext = eload(k + 1);
+        flNext = fload(k + 1);
+        if (k == z0 - 1) {
+            longlong2 vb[4];
+            eb = quadB(k & 1, vb);
+        }
+        longlong2 vt[4];
+        const int et = quadB((k + 1) & 1, vt), el = max(eb, et);
+        const int eBits = __float_as_int(Ee);
+        bool act = Ee != 0.f && el != 0;
+        if (act && (el > FX_EMAX || (eBits >> 23) == 0)) {
+            bad = true;
+            act = false;
+        }
+        long long nb[12];
+        int nO = cO;
+        if (__any_sync(0xffffffffu, act)) {
+            if (act && (el > S || S > el + FX_SLACK || qS != S)) {
+                longlong2 vb[4];
+                quadB(k & 1, vb);
+                S = el + 1;
+                quad(k & 1, S, vb, qb);
+            }
+            long long qt[12];
+            quad((k + 1) & 1, S, vt, qt);
+            qS = et <= S ? S : -1;
+            // The 20 combinations of the modes 1..7 that the cube's Khat scales (FxArgs).
+            long long v[20];
+            {
+                long long u[24];
+#pragma unroll
+                for (int i = 0; i < 12; ++i) {
+                    u[i] = qb[i] + qt[i];
+                    u[12 + i] = qb[i] - qt[i];
+                    qb[i] = qt[i];
+                }
+                v[0] = u[3]; v[1] = u[7]; v[2] = u[14]; v[3] = u[3] + u[7] + u[14];
+                v[4] = u[6] + u[4]; v[5] = u[12] + u[5]; v[6] = u[13] + u[8];
+                v[7] = u[23]; v[8] = u[22]; v[9] = u[21];
+                v[10] = u[10] + u[17]; v[11] = u[10] - u[17];
+                v[12] = u[9] + u[20]; v[13] = u[9] - u[20];
+                v[14] = u[15] + u[19]; v[15] = u[15] - u[19];
+                v[16] = u[18]; v[17] = u[16]; v[18] = u[11]; v[19] = u[18] + u[16] + u[11];
+            }
+            unsigned mag = 0;
+#pragma unroll
+            for (int i = 0; i < 20; ++i) {
+                const int h = (int)(v[i] >> 32);
+                mag |= (unsigned)(h ^ (h >> 31));
+            }
+            const int lz = max(__clz((int)mag) - 2, 0);
+            cO = act ? S + (eBits >> 23) + K.scaleExp - lz : FX_NONE;
+            const unsigned m = act ? (unsigned)((eBits & 0x7fffff) | 0x800000) << 7 : 0u;
+            // k_j v 2^lz in 2^64 units as a leading (A) and a middle digit sum (B); v 2^lz = v1 2^32 + v0 + 2^31
+            auto mul = [&](long long w, int j, long long& A, long long& B) {
+                const int v1 = (int)__funnelshift_l((unsigned)w, (unsigned)(w >> 32), lz);
+                const int v0 = (int)(((unsigned)w << lz) ^ 0x80000000u);
+                A += (long long)v1 * K.k1[j];
+                B += (long long)v1 * K.k0[j] + (long long)v0 * K.k1[j];
+            };
+            // times the modulus, rounded
+            auto scaled = [&](long long A, long long B) {
+                const long long y1 = A + (B >> 32);
+                const unsigned long long lo = (unsigned long long)(unsigned)y1 * m + 0x80000000ull;
+                return (long long)(int)(y1 >> 32) * (int)m + (long long)(lo >> 32);
+            };
+            auto one = [&](long long w, int j) {
+                long long A = 0, B = K.kb[j];
+                mul(w, j, A, B);
+                return scaled(A, B);
+            };
+            long long y[24];
+            y[0] = y[1] = y[2] = 0;
+            // a common part of three outputs plus each one's own
+            auto three = [&](int at, int j, long long& ya, long long& yb, long long& yc) {
+                long long As = 0, Bs = K.kb[j] + K.kb[j + 1] - 0x80000000ll;
+                mul(v[at + 3], j + 1, As, Bs);
+                long long A = As, B = Bs;
+                mul(v[at], j, A, B);
+                ya = scaled(A, B);
+                A = As, B = Bs;
+                mul(v[at + 1], j, A, B);
+                yb = scaled(A, B);
+                mul(v[at + 2], j, As, Bs);
+                yc = scaled(As, Bs);
+            };
+            three(0, 0, y[3], y[7], y[14]);
+            y[6] = y[4] = one(v[4], 2);
+            y[12] = y[5] = one(v[5], 2);
+            y[13] = y[8] = one(v[6], 2);
+            y[23] = one(v[7], 3);
+            y[22] = one(v[8], 3);
+            y[21] = one(v[9], 3);
+            auto two = [&](int at, long long& ya, long long& yb) {
+                const long long sum = one(v[at], 4), dif = one(v[at + 1], 5);
+                ya = sum + dif;
+                yb = sum - dif;
+            };
+            two(10, y[10], y[17]);
+            two(12, y[9], y[20]);
+            two(14, y[15], y[19]);
+            three(16, 6, y[18], y[16], y[11]);
+            // fold with the carry on the coarser of the two units
+            const int mO = max(nO, cO), sc = mO - nO, sy = mO - cO;
+            nO = mO;
+#pragma unroll
+            for (int i = 0; i < 12; ++i) {
+                nb[i] = fxShr(carry[i], sc) + fxShr(y[i] + y[12 + i], sy);
+                carry[i] = y[i] - y[12 + i];
+            }
+        } else {
+            qS = -1;
+            cO = FX_NONE;
+#pragma unroll
+            for (int i = 0; i < 12; ++i) {
+                nb[i] = carry[i];
+                carry[i] = 0;
+            }
+        }
+        eb = et;
+        double xo[3] = {0.0, 0.0, 0.0};  // in flight across the transform and the barrier
+        if (owner && k >= z0 && (OUT == OUT_CG || a.mode == MV_SMOOTH || a.dot0 == DOT_X_OUT)) {
+            const double* p = a.x + 3 * ((int64_t)oCol + (int64_t)k * plane);
+            xo[0] = p[0]; xo[1] = p[1]; xo[2] = p[2];
+        }
+        fwht4x3i(nb);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            syA[YSLOT(q, ty, tx)] = make_longlong2(nb[3 * q], nb[3 * q + 1]);
+            syB[YSLOT(q, ty, tx)] = make_longlong2(nb[3 * q + 2], nO);
+        }
+        __syncthreads();
+        if (owner && k >= z0) {
+            const int64_t s = (int64_t)oCol + (int64_t)k * plane;
+            const longlong2 a1 = syA[YSLOT(2, ty, tx + 1)], b1 = syB[YSLOT(2, ty, tx + 1)];
+            const longlong2 a2 = syA[YSLOT(1, ty + 1, tx)], b2 = syB[YSLOT(1, ty + 1, tx)];
+            const longlong2 a3 = syA[YSLOT(0, ty + 1, tx + 1)], b3 = syB[YSLOT(0, ty + 1, tx + 1)];
+            const int o1 = (int)b1.y, o2 = (int)b2.y, o3 = (int)b3.y;
+            const int o = max(max(nO, o1), max(o2, o3));
+            const long long t[3] = {
+                fxShr(nb[9], o - nO) + fxShr(a1.x, o - o1) + fxShr(a2.x, o - o2) + fxShr(a3.x, o - o3),
+                fxShr(nb[10], o - nO) + fxShr(a1.y, o - o1) + fxShr(a2.y, o - o2) + fxShr(a3.y, o - o3),
+                fxShr(nb[11], o - nO) + fxShr(b1.x, o - o1) + fxShr(b2.x, o - o2) + fxShr(b3.x, o - o3)};
+            double sum[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double r = __ll2double_rn(t[c]);
+                sum[c] = t[c] == 0 ? 0.0
+                                   : __hiloint2double(__double2hiint(r) + ((o + K.outExp) << 20), __double2loint(r));
+            }
+            if constexpr (OUT == OUT_CG) {
+                // (x at unused nodes may be anything: it must not reach the dot)
+                const bool fixed = (fl & FLAG_FIXED) != 0, live = (fl & FLAG_USED) && !fixed;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const double out = fixed ? 0.0 : sum[c];
+                    a.y[3 * s + c] = out;
+                    if (live) dAx = fma(xo[c], out, dAx);
+                }
+            } else {
+                mvOutput<double, double>(a, s, sum, fl, xo, d0, d1);
+            }
+        }
+    }
+#undef SLOT
+#undef YSLOT
+    if constexpr (OUT == OUT_CG) d0.add(dAx);
+    return bad;
+}
+
+// The block's march in FP64, out of line: its registers must not weigh on the integer march.
+template <int OUT>
+__device__ __noinline__ void fp64March(const MatvecArgs<double>* a, const Ks<double>* kp, int zc,
+                                       Scalars* S, unsigned char* smem, DotAcc<double>* d) {
+    d[0] = d[1] = DotAcc<double>();
+    walshMarch<double, double, OUT>(*a, *kp, S, smem, d[0], d[1], zc);
+}
+
+constexpr int FX_TY = MV_TY;
+
+template <int OUT>
+__global__ void __launch_bounds__(MV_TX* FX_TY, 2)
+    kMatvecFx(const __grid_constant__ MatvecArgs<double> a, const __grid_constant__ FxArgs K,
+              const __grid_constant__ Ks<double> kp, int zc, Scalars* S, RedBuf rb) {
+    if (a.checkDone && S->done) return;
+    if (a.condTrue && !trueResidualDue(S)) return;
+    extern __shared__ __align__(16) unsigned char smemRaw[];
+    DotAcc<double> d[2];
+    if (__syncthreads_or(fxMarch<OUT, FX_TY>(a, K, zc, smemRaw, d[0], d[1])))
+        fp64March<OUT>(&a, &kp, zc, S, smemRaw, d);
+    if (a.epi != EPI_NONE) {
+        double v[2] = {d[0].get(), d[1].get()}, t[2];
+        if (gridReduce<MV_TX * FX_TY, 2>(v, rb, t)) applyEpi(a.epi, S, t[0], t[1]);
+    }
+}
+
+}  // namespace
+
+// Khat of a cube, whose axes are interchangeable, has one constant per kind of
+// entry (a: diagonal, b: off-diagonal): normal strains (a, b), in-plane shears
+// (a = b: a rotation has no energy), bending pairs (a, b), the mode-7 terms and
+// the (1,1,1)-class triples (a, b).  Rows then need 20 products instead of 45:
+// a u_i + b (u_j + u_k) = (a - b) u_i + b (u_i + u_j + u_k), and a pair's sum and
+// difference scale by a + b and a - b, halved when they are recombined.
+bool fxPrepare(const KeData& ke, FxOperand& op) {
+    op.ready = false;
+    if (!ke.structured) return false;
+    static const int kind[45] = {0, 1, 1, 1, 0, 1, 1, 1, 0, 2, 2, 2, 2, 3, 2, 2, 2, 2, 3, 2, 2, 2, 2,
+                                 3, 4, 5, 5, 4, 4, 5, 5, 4, 4, 5, 5, 4, 6, 7, 7, 7, 6, 7, 7, 7, 6};
+    double c[8] = {}, cnt[8] = {}, top = 0.0;
+    for (int n = 0; n < 45; ++n) {
+        c[kind[n]] += ke.ks[n];
+        cnt[kind[n]] += 1.0;
+        top = std::fmax(top, std::fabs(ke.ks[n]));
+    }
+    for (int i = 0; i < 8; ++i) c[i] /= cnt[i];
+    for (int n = 0; n < 45; ++n)  // equal up to the rounding of Khat itself
+        if (!(std::fabs(ke.ks[n] - c[kind[n]]) <= 1e-15 * top)) return false;
+    const double k[8] = {c[0] - c[1], c[1], c[2], c[3], 0.5 * (c[4] + c[5]), 0.5 * (c[4] - c[5]), c[6] - c[7], c[7]};
+    // a component's rows: one normal strain, two shears, one mode-7 term, two of pairs, one of a triple
+    const double C = std::fabs(k[0]) + std::fabs(k[1]) + 2 * std::fabs(k[2]) + std::fabs(k[3]) +
+                     2 * (std::fabs(k[4]) + std::fabs(k[5])) + std::fabs(k[6]) + std::fabs(k[7]);
+    if (!(C > 0.0) || !std::isfinite(C)) return false;
+    int e = 0;
+    std::frexp(C, &e);  // C <= 2^e
+    if (std::abs(e) > 150) return false;
+    const int f = 62 - e;
+    for (int n = 0; n < 8; ++n) {
+        const long long v = std::llrint(std::ldexp(k[n], f));
+        op.k0[n] = (int32_t)(uint32_t)(v & 0xffffffffll);
+        op.k1[n] = (int32_t)((v - op.k0[n]) >> 32);
+    }
+    // field of 2^(S' + E' + 9 - f) with S' and E' the unbiased exponents of S and E
+    op.outExp = 9 - f - 1023 - 127;
+    op.ready = true;
+    return true;
+}
+
+cudaError_t fxSetAttributes() {
+    const cudaFuncAttribute A = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(kMatvecFx<OUT_CG>, A, (int)fxSmemBytes<FX_TY>());
+    return e ? e : cudaFuncSetAttribute(kMatvecFx<OUT_ANY>, A, (int)fxSmemBytes<FX_TY>());
+}
+
+// The operator scale of a level is a power of two (planLevels); other scales stay with the FP64 march.
+bool fxEligible(const FxOperand& op, double scale) {
+    int e = 0;
+    return op.ready && scale > 0.0 && std::frexp(scale, &e) == 0.5 && std::abs(e) <= 64;
+}
+
+void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOperand& op, const double* ks,
+                    Scalars* S, const RedBuf& rb) {
+    const int zc = fxLayers(a.g);
+    const Grid& g = a.g;
+    const dim3 block(MV_TX, FX_TY),
+        grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + FX_TY - 2) / (FX_TY - 1), (g.nz + zc - 1) / zc);
+    FxArgs K;
+    Ks<double> k;
+    for (int i = 0; i < 45; ++i) k.v[i] = ks[i];
+    for (int i = 0; i < 8; ++i) {
+        K.k1[i] = op.k1[i];
+        K.k0[i] = op.k0[i];
+        K.kb[i] = ((long long)op.k1[i] + 1) * (1ll << 31);
+    }
+    int e = 0;
+    std::frexp(a.scale, &e);
+    K.scaleExp = e - 1;
+    K.outExp = op.outExp;
+    if (a.mode == MV_AX && a.dot0 == DOT_X_OUT && !a.dot1 && !a.y32)
+        kMatvecFx<OUT_CG><<<grid, block, fxSmemBytes<FX_TY>(), stream>>>(a, K, k, zc, S, rb);
+    else
+        kMatvecFx<OUT_ANY><<<grid, block, fxSmemBytes<FX_TY>(), stream>>>(a, K, k, zc, S, rb);
+}
+
+int fxLayers(const Grid& g) {
+    // Few blocks: shorter marches (each repeats one element layer) until every SM has two blocks.
+    // 33 x 17 x 17 nodes: 6 blocks of 17 layers take 60 us, 54 blocks of 2 layers 20 us.
+    const int64_t tiles = (int64_t)((g.nx + MV_TX - 2) / (MV_TX - 1)) * ((g.ny + FX_TY - 2) / (FX_TY - 1));
+    int zc = MV_ZC;
+    while (zc > 2 && tiles * ((g.nz + zc - 1) / zc) < 2 * 152) zc /= 2;
+    return zc;
+}
+
+}  // namespace vfem
