@@ -6,6 +6,8 @@ is off by at most 2^-50 of C E sum|x| (its 24 values; C = the largest sum of
 |Khat| over one component's rows): 2^-51 from the inputs (each within 2^-54 of
 the largest, doubled three times by the transform), 14 roundings of 2^-56 each;
 aligning outputs and the final rounding to FP64 at most double that: 2^-49.
+Any other Ke is multiplied as it is; C is then its largest row sum of |Ke| and
+the same 2^-49 holds (no transform, one rounding per row and two of its modulus).
 """
 import numpy as np
 import pytest
@@ -31,7 +33,7 @@ def _corners(g, shape):
     return [g[a >> 2:(a >> 2) + nz, (a >> 1 & 1):(a >> 1 & 1) + ny, (a & 1):(a & 1) + nx] for a in range(8)]
 
 
-def _reference(vox, E, ke, x, fixed):
+def _reference(vox, E, ke, x, fixed, C=None):
     """K x and the entrywise tolerance."""
     mask = domains.used_nodes_mask(vox)
     g = np.zeros(mask.shape + (3,), LD)
@@ -42,7 +44,8 @@ def _reference(vox, E, ke, x, fixed):
     for i in range(24):
         for j in range(24):
             w[..., i] += LD(ke[i, j]) * u[..., j]
-    C = max(np.abs(_khat(ke))[c::3].sum() for c in range(3))
+    if C is None:
+        C = max(np.abs(_khat(ke))[c::3].sum() for c in range(3))
     t = LD(2.0) ** -49 * LD(C) * (np.abs(u).sum(axis=-1) * e)
     y, tol = np.zeros_like(g), np.zeros(g.shape, LD)
     for a, (v, b) in enumerate(zip(_corners(y, vox.shape), _corners(tol, vox.shape))):
@@ -110,14 +113,28 @@ def test_non_finite_values_stay_local():
     A.close()
 
 
-def test_other_structured_matrices_keep_the_fp64_march():
-    """A box's Ke (components scaled) has the cube's zero pattern but not its constants."""
-    shape = (9, 10, 33)
+@pytest.mark.parametrize("kind", ["reference_order", "box", "general"])
+def test_other_matrices(kind):
+    """Ke in the reference's corner order, a box's (components scaled: the cube's
+    zero pattern, not its constants) and a symmetric matrix without structure."""
+    shape = (5, 8, 32)
     vox, fixed, P = _domain(shape, 7)
-    s = np.tile([1.0, 2.0, 0.5], 8)
-    ke = domains.hex8_stiffness() * s[:, None] * s[None, :]
-    A = api.assembleSystemMatrix(vox, ke, fixed, 2)
-    x = np.random.default_rng(2).standard_normal(P.size)
-    ref, _ = _reference(vox, None, ke, x, fixed)
-    assert np.linalg.norm(((A @ x).astype(LD) - ref).astype(float)) <= 1e-14 * np.linalg.norm(ref.astype(float))
+    rng = np.random.default_rng(3)
+    E = rng.lognormal(0, 0.5, shape).astype(np.float32)
+    ke = domains.hex8_stiffness()
+    if kind == "reference_order":
+        dof = [3 * p + c for p in domains.KE0_NODE_PERM for c in range(3)]
+        ke = ke[np.ix_(dof, dof)]
+    elif kind == "box":
+        s = np.tile([1.0, 2.0, 0.5], 8)
+        ke = ke * s[:, None] * s[None, :]
+    else:
+        B = rng.standard_normal((24, 24))
+        ke = 1e-4 * (B @ B.T)
+    A = api.assembleSystemMatrix(vox, ke, fixed, 2, E=E)
+    C = np.abs(ke).sum(axis=1).max()
+    for name in ("random", "smooth", "graded_z", "wide", "huge"):
+        x = VECTORS[name](rng, P).reshape(-1)
+        ref, tol = _reference(vox, E, ke, x, fixed, C)
+        assert (np.abs((A @ x).astype(LD) - ref) <= tol).all(), name
     A.close()

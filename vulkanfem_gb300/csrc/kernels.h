@@ -123,18 +123,20 @@ cudaError_t setKernelAttributes();
 template <typename T>
 int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, const void* opconst);
 
-// The structured FP64 product in block fixed point (matvec_fx.cu): the cube's
-// 8 constants as 62-bit integers.  fxEligible: the operand is ready and `scale` a power of two.
+// The FP64 product in block fixed point (matvec_fx.cu): the 8 constants of a
+// cube's Ke, or the 576 entries of any other, as 62-bit integers.  fxEligible:
+// the operand is ready and `scale` a power of two.  opconst: the problem's
+// 45 + 576 FP64 constants.
 struct FxOperand {
-    int32_t k1[8], k0[8];
+    int32_t k1[576], k0[576];
     int outExp;
-    bool ready = false;
+    bool cube = false, ready = false;
 };
 bool fxPrepare(const KeData& ke, FxOperand& op);
 cudaError_t fxSetAttributes();
 bool fxEligible(const FxOperand& op, double scale);
 int fxLayers(const Grid& g);  // node layers a block marches
-void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOperand& op, const double* ks,
+void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOperand& op, const double* opconst,
                     Scalars* S, const RedBuf& rb);
 
 // The same product on FP64 vectors in double-float arithmetic (FP32 instructions,

@@ -1,17 +1,21 @@
-// matvec_fx.cu -- the structured FP64 product in block fixed point.
+// matvec_fx.cu -- the FP64 product in block fixed point.
 //
 // GB300 issues FP64 at 1/64 of its FP32 rate: measured 1.7 FP64 operations per
 // clock and SM against 58 64-bit integer additions and 29 multiply-adds 32 x 32
-// -> 64.  The FP64 march (walshMarch, matvec_march.cuh) is bound by its ~190
-// FP64 operations per element.  This kernel does the same element product in
-// 64-bit integers and leaves three conversions and the dot of a node to the
-// FP64 pipe.  Measured on a 191^3 grid with voids and log-normal moduli:
-// 3.72 -> 0.49 ms; on 33 x 17 x 17 nodes 262 -> 20 us (of it 262 -> 25 us from
-// this form with the shorter marches of fxLayers).  Bound now: instruction
-// issue (1,100 warp instructions per element row, 59% of the issue slots, ALU
-// 56%, wide multiply-adds 54% of their pipe), two 8-warp blocks per SM for
-// their registers.  Tiles of 12 rows in one block per SM (168 registers) or 6
-// rows in two measured 14% slower.
+// -> 64.  The FP64 marches (walshMarch and denseMarch, matvec_march.cuh) are
+// bound by their ~190 and ~600 FP64 operations per element.  This kernel does
+// the same element products in 64-bit integers and leaves three conversions and
+// the dot of a node to the FP64 pipe.
+//
+// Measured: 191^3 with voids and log-normal moduli 3.72 -> 0.49 ms; 33 x 17 x 17
+// nodes 262 -> 20 us (shorter marches by fxLayers among it); a Ke in another
+// corner order, as the dense 24 x 24 product, 96 x 80 x 72 half full, 1.56 ->
+// 0.26 ms.  Bound now: instruction issue (1,100 warp instructions per element
+// row, 59% of the issue slots, ALU 56%, wide multiply-adds 54% of their pipe)
+// with two 8-warp blocks per SM for their registers; the dense form by its 1,728
+// wide multiply-adds an element.  Cube tiles of 12 rows in one block per SM (168
+// registers) or of 6 rows in two measured 14% slower; the dense form with two
+// blocks per SM (128 registers, 240 bytes spilled) the same as with one.
 //
 // Numbers.  A node's three components are staged as 58-bit integers under the
 // node's largest exponent.  An element reads its 24 values on a grid S with
@@ -24,15 +28,18 @@
 // Outputs with different O are aligned to the larger one where they meet.
 // Against 113-bit arithmetic the result's relative error is 3e-16 to 6e-16
 // (random, smooth, graded and point vectors, moduli 1, log-normal or spread
-// over e^20), where the FP64 march has 5e-16 to 4e-15.
+// over e^20), where the FP64 march has 5e-16 to 4e-15; the dense form's 5e-17 to
+// 8e-16, where the FP64 one has 1e-16 to 2.5e-15.
 //
 // No sum can overflow: the combinations are below 2^62, so a component's corner
 // value is at most C 2^f 2^62 / 2^64 / 2 <= 2^59 per element, and a node sums 8
-// of them; sums in between are taken modulo 2^64.  Values the grid cannot take
+// of them; sums in between are taken modulo 2^64.  A middle digit sum has at
+// most two (dense: 24, hence the coarser k0) products of 2^61 and 2^62 besides.  Values the grid cannot take
 // (non-finite ones or exponents beyond 2^+-575 next to a filled voxel, subnormal
 // moduli) make the block repeat its march in FP64, so that results for those
 // are what the FP64 march gives.
 #include <cmath>
+#include <cstring>
 
 #include "matvec_march.cuh"
 
@@ -45,11 +52,18 @@ constexpr int FX_BAD = 4000;                  // a node outside of them
 constexpr int FX_NONE = -(1 << 20);           // exponent of a zero contribution
 constexpr int FX_SLACK = 3;
 
-struct FxArgs {
-    long long kb[8];   // start of a middle digit sum: 2^31 (rounding) + 2^31 k1
-    int k1[8], k0[8];  // the cube's constants (fxPrepare) times 2^f = k1 2^32 + k0, signed digits
-    int scaleExp;        // log2 of the level's operator scale
-    int outExp;          // exponent-field offset of an output at O
+// Constants times 2^f = k1 2^32 + k0, signed digits.  kb: start of a middle digit
+// sum, 2^31 (rounding) + 2^31 k1.
+struct FxArgs {        // the cube's 8 constants (cubeConstants)
+    long long kb[8];
+    int k1[8], k0[8];
+    int scaleExp;      // log2 of the level's operator scale
+    int outExp;        // exponent-field offset of an output at O
+};
+struct FxDenseArgs {   // Ke, row-major; k0 in units of 2^3, so that 24 of its products fit their sum
+    long long kb[24];
+    int k1[576], k0[576];
+    int scaleExp, outExp;
 };
 
 struct FxNode {
@@ -113,12 +127,16 @@ constexpr size_t fxSmemBytes() {
     return fx > fp ? fx : fp;
 }
 
-// One block's march, the counterpart of walshMarch<double, double, OUT> with the
-// same tile, halo and pipelining.  Returns true when a value did not fit (the
-// outputs and dots are then to be recomputed).
-template <int OUT, int TY>
-__device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const FxArgs& K, int zc, unsigned char* smem,
+// One block's march, the counterpart of walshMarch<double, double, OUT> (KA =
+// FxArgs) and denseMarch<double, double> (FxDenseArgs) with the same tile, halo
+// and pipelining.  Returns true when a value did not fit (the outputs and dots
+// are then to be recomputed).  The dense form has the 24 values themselves in
+// place of the Walsh combinations and reads both quads every layer, to keep
+// their digits in registers.
+template <int OUT, int TY, typename KA>
+__device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const KA& K, int zc, unsigned char* smem,
                                         DotAcc<double>& d0, DotAcc<double>& d1) {
+    constexpr bool DENSE = std::is_same<KA, FxDenseArgs>::value;
     // 16-byte halves of the 32-byte slots in arrays of their own: conflict-free
     longlong2* suA = reinterpret_cast<longlong2*>(smem);           // {v0, v1}
     longlong2* suB = suA + 2 * (TY + 1) * (MV_TX + 1);             // {v2, exponent}
@@ -194,9 +212,9 @@ __device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const FxArg
             v[3 * q + 1] = fxShr(va.y, by);
             v[3 * q + 2] = fxShr(vb[q].x, by);
         }
-        fwht4x3i(v);
+        if constexpr (!DENSE) fwht4x3i(v);
     };
-    long long qb[12], carry[12];  // bottom quad and the previous element's top-face output, Walsh domain
+    long long qb[12], carry[12];  // bottom quad and the previous element's top-face output (Walsh domain)
 #pragma unroll
     for (int i = 0; i < 12; ++i) qb[i] = carry[i] = 0;
     int S = 0, qS = -1, eb = 0, cO = FX_NONE;  // grid, the grid qb is on (-1: none), exponent of qb, of the carry
@@ -230,98 +248,133 @@ __device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const FxArg
         long long nb[12];
         int nO = cO;
         if (__any_sync(0xffffffffu, act)) {
-            if (act && (el > S || S > el + FX_SLACK || qS != S)) {
+            if constexpr (DENSE) {
+                if (act && (el > S || S > el + FX_SLACK)) S = el + 1;
+            } else if (act && (el > S || S > el + FX_SLACK || qS != S)) {
                 longlong2 vb[4];
                 quadB(k & 1, vb);
                 S = el + 1;
                 quad(k & 1, S, vb, qb);
             }
-            long long qt[12];
+            long long qt[12], y[24];
             quad((k + 1) & 1, S, vt, qt);
             qS = et <= S ? S : -1;
-            // The 20 combinations of the modes 1..7 that the cube's Khat scales (FxArgs).
-            long long v[20];
-            {
-                long long u[24];
-#pragma unroll
-                for (int i = 0; i < 12; ++i) {
-                    u[i] = qb[i] + qt[i];
-                    u[12 + i] = qb[i] - qt[i];
-                    qb[i] = qt[i];
-                }
-                v[0] = u[3]; v[1] = u[7]; v[2] = u[14]; v[3] = u[3] + u[7] + u[14];
-                v[4] = u[6] + u[4]; v[5] = u[12] + u[5]; v[6] = u[13] + u[8];
-                v[7] = u[23]; v[8] = u[22]; v[9] = u[21];
-                v[10] = u[10] + u[17]; v[11] = u[10] - u[17];
-                v[12] = u[9] + u[20]; v[13] = u[9] - u[20];
-                v[14] = u[15] + u[19]; v[15] = u[15] - u[19];
-                v[16] = u[18]; v[17] = u[16]; v[18] = u[11]; v[19] = u[18] + u[16] + u[11];
-            }
-            unsigned mag = 0;
-#pragma unroll
-            for (int i = 0; i < 20; ++i) {
-                const int h = (int)(v[i] >> 32);
-                mag |= (unsigned)(h ^ (h >> 31));
-            }
-            const int lz = max(__clz((int)mag) - 2, 0);
-            cO = act ? S + (eBits >> 23) + K.scaleExp - lz : FX_NONE;
             const unsigned m = act ? (unsigned)((eBits & 0x7fffff) | 0x800000) << 7 : 0u;
-            // k_j v 2^lz in 2^64 units as a leading (A) and a middle digit sum (B); v 2^lz = v1 2^32 + v0 + 2^31
-            auto mul = [&](long long w, int j, long long& A, long long& B) {
-                const int v1 = (int)__funnelshift_l((unsigned)w, (unsigned)(w >> 32), lz);
-                const int v0 = (int)(((unsigned)w << lz) ^ 0x80000000u);
-                A += (long long)v1 * K.k1[j];
-                B += (long long)v1 * K.k0[j] + (long long)v0 * K.k1[j];
-            };
             // times the modulus, rounded
             auto scaled = [&](long long A, long long B) {
                 const long long y1 = A + (B >> 32);
                 const unsigned long long lo = (unsigned long long)(unsigned)y1 * m + 0x80000000ull;
                 return (long long)(int)(y1 >> 32) * (int)m + (long long)(lo >> 32);
             };
-            auto one = [&](long long w, int j) {
-                long long A = 0, B = K.kb[j];
-                mul(w, j, A, B);
-                return scaled(A, B);
+            auto spread = [](long long w) {
+                const int h = (int)(w >> 32);
+                return (unsigned)(h ^ (h >> 31));
             };
-            long long y[24];
-            y[0] = y[1] = y[2] = 0;
-            // a common part of three outputs plus each one's own
-            auto three = [&](int at, int j, long long& ya, long long& yb, long long& yc) {
-                long long As = 0, Bs = K.kb[j] + K.kb[j + 1] - 0x80000000ll;
-                mul(v[at + 3], j + 1, As, Bs);
-                long long A = As, B = Bs;
-                mul(v[at], j, A, B);
-                ya = scaled(A, B);
-                A = As, B = Bs;
-                mul(v[at + 1], j, A, B);
-                yb = scaled(A, B);
-                mul(v[at + 2], j, As, Bs);
-                yc = scaled(As, Bs);
+            // w 2^lz = w1 2^32 + w0 + 2^31
+            auto digits = [](long long w, int lz, int& w1, int& w0) {
+                w1 = (int)__funnelshift_l((unsigned)w, (unsigned)(w >> 32), lz);
+                w0 = (int)(((unsigned)w << lz) ^ 0x80000000u);
             };
-            three(0, 0, y[3], y[7], y[14]);
-            y[6] = y[4] = one(v[4], 2);
-            y[12] = y[5] = one(v[5], 2);
-            y[13] = y[8] = one(v[6], 2);
-            y[23] = one(v[7], 3);
-            y[22] = one(v[8], 3);
-            y[21] = one(v[9], 3);
-            auto two = [&](int at, long long& ya, long long& yb) {
-                const long long sum = one(v[at], 4), dif = one(v[at + 1], 5);
-                ya = sum + dif;
-                yb = sum - dif;
-            };
-            two(10, y[10], y[17]);
-            two(12, y[9], y[20]);
-            two(14, y[15], y[19]);
-            three(16, 6, y[18], y[16], y[11]);
+            if constexpr (DENSE) {
+                longlong2 vb[4];
+                quadB(k & 1, vb);
+                quad(k & 1, S, vb, qb);
+                unsigned mag = 0;
+#pragma unroll
+                for (int i = 0; i < 12; ++i) mag |= spread(qb[i]) | spread(qt[i]);
+                const int lz = max(__clz((int)mag) - 2, 0);
+                cO = act ? S + (eBits >> 23) + K.scaleExp - lz : FX_NONE;
+                int u1[24], u0[24];
+#pragma unroll
+                for (int i = 0; i < 12; ++i) {
+                    digits(qb[i], lz, u1[i], u0[i]);
+                    digits(qt[i], lz, u1[12 + i], u0[12 + i]);
+                }
+#pragma unroll
+                for (int r = 0; r < 24; ++r) {
+                    long long A = 0, B = K.kb[r], B3 = 0;
+#pragma unroll
+                    for (int c = 0; c < 24; ++c) {
+                        A += (long long)u1[c] * K.k1[24 * r + c];
+                        B += (long long)u0[c] * K.k1[24 * r + c];
+                        B3 += (long long)u1[c] * K.k0[24 * r + c];
+                    }
+                    y[r] = scaled(A + (B3 >> 29), B);
+                }
+            } else {
+                // The 20 combinations of the modes 1..7 that the cube's Khat scales (FxArgs).
+                long long v[20];
+                {
+                    long long u[24];
+#pragma unroll
+                    for (int i = 0; i < 12; ++i) {
+                        u[i] = qb[i] + qt[i];
+                        u[12 + i] = qb[i] - qt[i];
+                        qb[i] = qt[i];
+                    }
+                    v[0] = u[3]; v[1] = u[7]; v[2] = u[14]; v[3] = u[3] + u[7] + u[14];
+                    v[4] = u[6] + u[4]; v[5] = u[12] + u[5]; v[6] = u[13] + u[8];
+                    v[7] = u[23]; v[8] = u[22]; v[9] = u[21];
+                    v[10] = u[10] + u[17]; v[11] = u[10] - u[17];
+                    v[12] = u[9] + u[20]; v[13] = u[9] - u[20];
+                    v[14] = u[15] + u[19]; v[15] = u[15] - u[19];
+                    v[16] = u[18]; v[17] = u[16]; v[18] = u[11]; v[19] = u[18] + u[16] + u[11];
+                }
+                unsigned mag = 0;
+#pragma unroll
+                for (int i = 0; i < 20; ++i) mag |= spread(v[i]);
+                const int lz = max(__clz((int)mag) - 2, 0);
+                cO = act ? S + (eBits >> 23) + K.scaleExp - lz : FX_NONE;
+                // k_j v 2^lz in 2^64 units as a leading (A) and a middle digit sum (B)
+                auto mul = [&](long long w, int j, long long& A, long long& B) {
+                    int v1, v0;
+                    digits(w, lz, v1, v0);
+                    A += (long long)v1 * K.k1[j];
+                    B += (long long)v1 * K.k0[j] + (long long)v0 * K.k1[j];
+                };
+                auto one = [&](long long w, int j) {
+                    long long A = 0, B = K.kb[j];
+                    mul(w, j, A, B);
+                    return scaled(A, B);
+                };
+                y[0] = y[1] = y[2] = 0;
+                // a common part of three outputs plus each one's own
+                auto three = [&](int at, int j, long long& ya, long long& yb, long long& yc) {
+                    long long As = 0, Bs = K.kb[j] + K.kb[j + 1] - 0x80000000ll;
+                    mul(v[at + 3], j + 1, As, Bs);
+                    long long A = As, B = Bs;
+                    mul(v[at], j, A, B);
+                    ya = scaled(A, B);
+                    A = As, B = Bs;
+                    mul(v[at + 1], j, A, B);
+                    yb = scaled(A, B);
+                    mul(v[at + 2], j, As, Bs);
+                    yc = scaled(As, Bs);
+                };
+                three(0, 0, y[3], y[7], y[14]);
+                y[6] = y[4] = one(v[4], 2);
+                y[12] = y[5] = one(v[5], 2);
+                y[13] = y[8] = one(v[6], 2);
+                y[23] = one(v[7], 3);
+                y[22] = one(v[8], 3);
+                y[21] = one(v[9], 3);
+                auto two = [&](int at, long long& ya, long long& yb) {
+                    const long long sum = one(v[at], 4), dif = one(v[at + 1], 5);
+                    ya = sum + dif;
+                    yb = sum - dif;
+                };
+                two(10, y[10], y[17]);
+                two(12, y[9], y[20]);
+                two(14, y[15], y[19]);
+                three(16, 6, y[18], y[16], y[11]);
+            }
             // fold with the carry on the coarser of the two units
             const int mO = max(nO, cO), sc = mO - nO, sy = mO - cO;
             nO = mO;
 #pragma unroll
             for (int i = 0; i < 12; ++i) {
-                nb[i] = fxShr(carry[i], sc) + fxShr(y[i] + y[12 + i], sy);
-                carry[i] = y[i] - y[12 + i];
+                nb[i] = fxShr(carry[i], sc) + fxShr(DENSE ? y[i] : y[i] + y[12 + i], sy);
+                carry[i] = DENSE ? y[12 + i] : y[i] - y[12 + i];
             }
         } else {
             qS = -1;
@@ -338,7 +391,7 @@ __device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const FxArg
             const double* p = a.x + 3 * ((int64_t)oCol + (int64_t)k * plane);
             xo[0] = p[0]; xo[1] = p[1]; xo[2] = p[2];
         }
-        fwht4x3i(nb);
+        if constexpr (!DENSE) fwht4x3i(nb);
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             syA[YSLOT(q, ty, tx)] = make_longlong2(nb[3 * q], nb[3 * q + 1]);
@@ -385,18 +438,24 @@ __device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const FxArg
 
 // The block's march in FP64, out of line: its registers must not weigh on the integer march.
 template <int OUT>
-__device__ __noinline__ void fp64March(const MatvecArgs<double>* a, const Ks<double>* kp, int zc,
-                                       Scalars* S, unsigned char* smem, DotAcc<double>* d) {
+__device__ __noinline__ void fp64March(const MatvecArgs<double>* a, const Ks<double>* kp, int zc, Scalars* S,
+                                       unsigned char* smem, DotAcc<double>* d) {
     d[0] = d[1] = DotAcc<double>();
     walshMarch<double, double, OUT>(*a, *kp, S, smem, d[0], d[1], zc);
+}
+template <int OUT>
+__device__ __noinline__ void fp64March(const MatvecArgs<double>* a, const Kd<double>* kp, int zc, Scalars*,
+                                       unsigned char* smem, DotAcc<double>* d) {
+    d[0] = d[1] = DotAcc<double>();
+    denseMarch<double, double>(*a, *kp, smem, d[0], d[1], zc);
 }
 
 constexpr int FX_TY = MV_TY;
 
-template <int OUT>
-__global__ void __launch_bounds__(MV_TX* FX_TY, 2)
-    kMatvecFx(const __grid_constant__ MatvecArgs<double> a, const __grid_constant__ FxArgs K,
-              const __grid_constant__ Ks<double> kp, int zc, Scalars* S, RedBuf rb) {
+template <int OUT, typename KA, typename KP>
+__global__ void __launch_bounds__(MV_TX* FX_TY, std::is_same<KA, FxArgs>::value ? 2 : 1)
+    kMatvecFx(const __grid_constant__ MatvecArgs<double> a, const __grid_constant__ KA K,
+              const __grid_constant__ KP kp, int zc, Scalars* S, RedBuf rb) {
     if (a.checkDone && S->done) return;
     if (a.condTrue && !trueResidualDue(S)) return;
     extern __shared__ __align__(16) unsigned char smemRaw[];
@@ -411,14 +470,33 @@ __global__ void __launch_bounds__(MV_TX* FX_TY, 2)
 
 }  // namespace
 
+namespace {
+// Digits and f of k[0..n), k0 in units of 2^low.  C: a bound of the sum of |k|
+// over what one node component collects from an element.
+bool fxDigits(const double* k, int n, double C, int low, int32_t* k1, int32_t* k0, int& outExp) {
+    if (!(C > 0.0) || !std::isfinite(C)) return false;
+    int e = 0;
+    std::frexp(C, &e);  // C <= 2^e
+    if (std::abs(e) > 150) return false;
+    const int f = 62 - e;
+    for (int i = 0; i < n; ++i) {
+        const long long v = std::llrint(std::ldexp(k[i], f));
+        const int32_t rest = (int32_t)(uint32_t)(v & 0xffffffffll);
+        k1[i] = (int32_t)((v - rest) >> 32);
+        k0[i] = low ? (int32_t)std::lrint(std::ldexp((double)rest, -low)) : rest;
+    }
+    // field of 2^(S' + E' + 9 - f) with S' and E' the unbiased exponents of S and E
+    outExp = 9 - f - 1023 - 127;
+    return true;
+}
+
 // Khat of a cube, whose axes are interchangeable, has one constant per kind of
 // entry (a: diagonal, b: off-diagonal): normal strains (a, b), in-plane shears
 // (a = b: a rotation has no energy), bending pairs (a, b), the mode-7 terms and
 // the (1,1,1)-class triples (a, b).  Rows then need 20 products instead of 45:
 // a u_i + b (u_j + u_k) = (a - b) u_i + b (u_i + u_j + u_k), and a pair's sum and
 // difference scale by a + b and a - b, halved when they are recombined.
-bool fxPrepare(const KeData& ke, FxOperand& op) {
-    op.ready = false;
+bool cubeConstants(const KeData& ke, double (&k)[8], double& C) {
     if (!ke.structured) return false;
     static const int kind[45] = {0, 1, 1, 1, 0, 1, 1, 1, 0, 2, 2, 2, 2, 3, 2, 2, 2, 2, 3, 2, 2, 2, 2,
                                  3, 4, 5, 5, 4, 4, 5, 5, 4, 4, 5, 5, 4, 6, 7, 7, 7, 6, 7, 7, 7, 6};
@@ -431,30 +509,37 @@ bool fxPrepare(const KeData& ke, FxOperand& op) {
     for (int i = 0; i < 8; ++i) c[i] /= cnt[i];
     for (int n = 0; n < 45; ++n)  // equal up to the rounding of Khat itself
         if (!(std::fabs(ke.ks[n] - c[kind[n]]) <= 1e-15 * top)) return false;
-    const double k[8] = {c[0] - c[1], c[1], c[2], c[3], 0.5 * (c[4] + c[5]), 0.5 * (c[4] - c[5]), c[6] - c[7], c[7]};
+    const double v[8] = {c[0] - c[1], c[1], c[2], c[3], 0.5 * (c[4] + c[5]), 0.5 * (c[4] - c[5]), c[6] - c[7], c[7]};
+    for (int i = 0; i < 8; ++i) k[i] = v[i];
     // a component's rows: one normal strain, two shears, one mode-7 term, two of pairs, one of a triple
-    const double C = std::fabs(k[0]) + std::fabs(k[1]) + 2 * std::fabs(k[2]) + std::fabs(k[3]) +
-                     2 * (std::fabs(k[4]) + std::fabs(k[5])) + std::fabs(k[6]) + std::fabs(k[7]);
-    if (!(C > 0.0) || !std::isfinite(C)) return false;
-    int e = 0;
-    std::frexp(C, &e);  // C <= 2^e
-    if (std::abs(e) > 150) return false;
-    const int f = 62 - e;
-    for (int n = 0; n < 8; ++n) {
-        const long long v = std::llrint(std::ldexp(k[n], f));
-        op.k0[n] = (int32_t)(uint32_t)(v & 0xffffffffll);
-        op.k1[n] = (int32_t)((v - op.k0[n]) >> 32);
-    }
-    // field of 2^(S' + E' + 9 - f) with S' and E' the unbiased exponents of S and E
-    op.outExp = 9 - f - 1023 - 127;
-    op.ready = true;
+    C = std::fabs(k[0]) + std::fabs(k[1]) + 2 * std::fabs(k[2]) + std::fabs(k[3]) +
+        2 * (std::fabs(k[4]) + std::fabs(k[5])) + std::fabs(k[6]) + std::fabs(k[7]);
     return true;
+}
+}  // namespace
+
+bool fxPrepare(const KeData& ke, FxOperand& op) {
+    double k[8], C = 0.0;
+    op.cube = cubeConstants(ke, k, C);
+    if (op.cube) return op.ready = fxDigits(k, 8, C, 0, op.k1, op.k0, op.outExp);
+    for (int r = 0; r < 24; ++r) {
+        double row = 0.0;
+        for (int c = 0; c < 24; ++c) row += std::fabs(ke.Ke[24 * r + c]);
+        C = std::fmax(C, row);
+    }
+    return op.ready = fxDigits(ke.Ke, 576, C, 3, op.k1, op.k0, op.outExp);
 }
 
 cudaError_t fxSetAttributes() {
-    const cudaFuncAttribute A = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(kMatvecFx<OUT_CG>, A, (int)fxSmemBytes<FX_TY>());
-    return e ? e : cudaFuncSetAttribute(kMatvecFx<OUT_ANY>, A, (int)fxSmemBytes<FX_TY>());
+    cudaError_t e = cudaSuccess;
+    auto set = [&](auto kern) {
+        if (!e) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fxSmemBytes<FX_TY>());
+    };
+    set(kMatvecFx<OUT_CG, FxArgs, Ks<double>>);
+    set(kMatvecFx<OUT_ANY, FxArgs, Ks<double>>);
+    set(kMatvecFx<OUT_CG, FxDenseArgs, Kd<double>>);
+    set(kMatvecFx<OUT_ANY, FxDenseArgs, Kd<double>>);
+    return e;
 }
 
 // The operator scale of a level is a power of two (planLevels); other scales stay with the FP64 march.
@@ -463,28 +548,35 @@ bool fxEligible(const FxOperand& op, double scale) {
     return op.ready && scale > 0.0 && std::frexp(scale, &e) == 0.5 && std::abs(e) <= 64;
 }
 
-void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOperand& op, const double* ks,
+void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOperand& op, const double* opconst,
                     Scalars* S, const RedBuf& rb) {
     const int zc = fxLayers(a.g);
     const Grid& g = a.g;
     const dim3 block(MV_TX, FX_TY),
         grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + FX_TY - 2) / (FX_TY - 1), (g.nz + zc - 1) / zc);
-    FxArgs K;
-    Ks<double> k;
-    for (int i = 0; i < 45; ++i) k.v[i] = ks[i];
-    for (int i = 0; i < 8; ++i) {
-        K.k1[i] = op.k1[i];
-        K.k0[i] = op.k0[i];
-        K.kb[i] = ((long long)op.k1[i] + 1) * (1ll << 31);
-    }
-    int e = 0;
-    std::frexp(a.scale, &e);
-    K.scaleExp = e - 1;
-    K.outExp = op.outExp;
-    if (a.mode == MV_AX && a.dot0 == DOT_X_OUT && !a.dot1 && !a.y32)
-        kMatvecFx<OUT_CG><<<grid, block, fxSmemBytes<FX_TY>(), stream>>>(a, K, k, zc, S, rb);
+    const bool cg = a.mode == MV_AX && a.dot0 == DOT_X_OUT && !a.dot1 && !a.y32;
+    auto go = [&](auto K, int rows, int cols, auto k, const double* src, auto kernCg, auto kernAny) {
+        for (int i = 0; i < rows * cols; ++i) {
+            K.k1[i] = op.k1[i];
+            K.k0[i] = op.k0[i];
+        }
+        for (int r = 0; r < rows; ++r) {
+            K.kb[r] = 1ll << 31;
+            for (int c = 0; c < cols; ++c) K.kb[r] += (long long)op.k1[r * cols + c] * (1ll << 31);
+        }
+        int e = 0;
+        std::frexp(a.scale, &e);
+        K.scaleExp = e - 1;
+        K.outExp = op.outExp;
+        std::memcpy(k.v, src, sizeof(k.v));
+        (cg ? kernCg : kernAny)<<<grid, block, fxSmemBytes<FX_TY>(), stream>>>(a, K, k, zc, S, rb);
+    };
+    if (op.cube)
+        go(FxArgs(), 8, 1, Ks<double>(), opconst, kMatvecFx<OUT_CG, FxArgs, Ks<double>>,
+           kMatvecFx<OUT_ANY, FxArgs, Ks<double>>);
     else
-        kMatvecFx<OUT_ANY><<<grid, block, fxSmemBytes<FX_TY>(), stream>>>(a, K, k, zc, S, rb);
+        go(FxDenseArgs(), 24, 24, Kd<double>(), opconst + 45, kMatvecFx<OUT_CG, FxDenseArgs, Kd<double>>,
+           kMatvecFx<OUT_ANY, FxDenseArgs, Kd<double>>);
 }
 
 int fxLayers(const Grid& g) {

@@ -218,6 +218,161 @@ __device__ __forceinline__ void mvOutput(const MatvecArgs<T>& a, int64_t s, cons
     }
 }
 
+// Element-by-element product with a general (dense 24 x 24) Ke, for element
+// matrices without the isotropic-cube symmetry (for example the reference's
+// Ke0.dat in its own node order); structured Ke use kMatvecH below.
+// A 2.5-D tile: a block of 32 x 8 threads marches
+// up a z-range; at each element layer thread (tx,ty) computes the element whose
+// lower corner is node (x0+tx-1, y0+ty-1) and owns node (x0+tx, y0+ty), which is
+// the (1,1) corner of its own element and a corner of the three neighbouring
+// threads' elements.  Element outputs pass through shared memory once; each
+// owned node sums its four in-layer contributions for the bottom face (node
+// layer k) and the top face (node layer k+1), so no atomics are needed.
+// The march is software-pipelined: while layer k is computed, the node values
+// of layer k+2, the modulus of element layer k+1 and the owned node's flags
+// are already in flight to registers.  The 33 x 9 node tile of a layer is
+// loaded without integer division: every thread loads its own slot, row 8
+// comes from the ty == 0 threads and column 32 from nine threads of row 1.
+//
+// T is the storage type of the vectors, TC the arithmetic type (T, or df for
+// the true residual of the mixed-precision solve: FP64 vectors, df arithmetic).
+// One block's march: fills d0 and d1 (this thread's dots).
+template <typename T, typename TC>
+__device__ __forceinline__ void denseMarch(const MatvecArgs<T>& a, const Kd<TC>& kp, unsigned char* smemRaw,
+                                           DotAcc<TC>& d0, DotAcc<TC>& d1, [[maybe_unused]] int layers = MV_ZC) {
+    typedef Cvt<T, TC> C;
+    TC* su = reinterpret_cast<TC*>(smemRaw);
+    TC* sy = su + kSuElems;
+    const Grid g = a.g;
+    const int zc = std::is_same<TC, double>::value ? layers : MV_ZC;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int x0 = blockIdx.x * (MV_TX - 1), y0 = blockIdx.y * (MV_TY - 1), z0 = blockIdx.z * zc;
+    const int zend = min(z0 + zc, g.nz);
+    const int64_t plane = (int64_t)g.nx * g.ny;
+    const int ecx = x0 + tx - 1, ecy = y0 + ty - 1;
+    const int onx = x0 + tx, ony = y0 + ty;
+    const bool owner = (tx < MV_TX - 1) && (ty < MV_TY - 1) && onx < g.nx && ony < g.ny;
+    const bool ecxy = ecx >= 0 && ecx < g.ex && ecy >= 0 && ecy < g.ey;
+    const int eCol = ecy * g.nx + ecx;   // in-plane offsets fit in 32 bits for every accepted grid
+    const int oCol = ony * g.nx + onx;
+    const TC sc = TC(a.scale);
+    // Extra tile slots: row MV_TY (ty == 0 threads), column MV_TX (row-1 threads tx <= MV_TY).
+    const bool hasR = ty == 0, hasC = (ty == 1) && (tx <= MV_TY);
+    const int rX = x0 - 1 + tx, rY = y0 - 1 + MV_TY;
+    const int cX = x0 - 1 + MV_TX, cY = y0 - 1 + tx;
+    const bool ok0 = ecx >= 0 && ecx < g.nx && ecy >= 0 && ecy < g.ny;
+    const bool okR = hasR && rX >= 0 && rX < g.nx && rY >= 0 && rY < g.ny;
+    const bool okC = hasC && cX >= 0 && cX < g.nx && cY >= 0 && cY < g.ny;
+#define SU(b, iy, ix) (su + (((((b) * (MV_TY + 1)) + (iy)) * (MV_TX + 1) + (ix)) << 2))
+#define SY(k, iy, ix) (sy + (((((k) * MV_TY) + (iy)) * MV_TX + (ix)) << 2))
+    T pf[9];
+    auto gload = [&](int zl) {
+        const bool zok = zl >= 0 && zl < g.nz;
+        const int64_t zoff = (int64_t)zl * plane;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) pf[i] = T(0);
+        if (ok0 && zok) {
+            const T* p = a.x + 3 * ((int64_t)eCol + zoff);
+            pf[0] = p[0]; pf[1] = p[1]; pf[2] = p[2];
+        }
+        if (okR && zok) {
+            const T* p = a.x + 3 * ((int64_t)(rY * g.nx + rX) + zoff);
+            pf[3] = p[0]; pf[4] = p[1]; pf[5] = p[2];
+        }
+        if (okC && zok) {
+            const T* p = a.x + 3 * ((int64_t)(cY * g.nx + cX) + zoff);
+            pf[6] = p[0]; pf[7] = p[1]; pf[8] = p[2];
+        }
+    };
+    auto sstore = [&](int zl) {
+        const int b = zl & 1;
+        stSlot<TC>(SU(b, ty, tx), C::in(pf[0]), C::in(pf[1]), C::in(pf[2]));
+        if (hasR) stSlot<TC>(SU(b, MV_TY, tx), C::in(pf[3]), C::in(pf[4]), C::in(pf[5]));
+        if (hasC) stSlot<TC>(SU(b, tx, MV_TX), C::in(pf[6]), C::in(pf[7]), C::in(pf[8]));
+    };
+    auto eload = [&](int k) -> float {
+        return (ecxy && k >= 0 && k < g.ez) ? a.E[(int64_t)eCol + (int64_t)k * plane] : 0.f;
+    };
+    auto fload = [&](int k) -> uint8_t {
+        return (owner && k >= z0 && k < zend) ? a.flags[(int64_t)oCol + (int64_t)k * plane] : (uint8_t)0;
+    };
+    TC acc[3] = {TC(0), TC(0), TC(0)};
+    gload(z0 - 1);
+    sstore(z0 - 1);
+    gload(z0);
+    float Enext = eload(z0 - 1);
+    uint8_t flNext = fload(z0 - 1);
+    for (int k = z0 - 1; k < zend; ++k) {
+        sstore(k + 1);
+        const float Ee = Enext;
+        const uint8_t fl = flNext;
+        __syncthreads();
+        gload(k + 2);           // consumed by the next iteration
+        Enext = eload(k + 1);
+        flNext = fload(k + 1);
+        // x at the owned node of layer k, read now: the next iteration's store
+        // overwrites this layer's buffer without waiting for the output phase.
+        TC xo[3];
+        ldSlot<TC>(SU(k & 1, ty + 1, tx + 1), xo[0], xo[1], xo[2]);
+        TC ye[24];
+        if (Ee != 0.f) {
+            TC u[24];
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+                const int dx = n & 1, dy = (n >> 1) & 1, dz = n >> 2;
+                ldSlot<TC>(SU((k + dz) & 1, ty + dy, tx + dx), u[3 * n], u[3 * n + 1], u[3 * n + 2]);
+            }
+            elemDense<TC>(u, ye, kp, sc * TC(Ee));
+        } else {
+#pragma unroll
+            for (int i = 0; i < 24; ++i) ye[i] = TC(0);
+        }
+        stSlot<TC>(SY(0, ty, tx), ye[0], ye[1], ye[2]);     // a = 0
+        stSlot<TC>(SY(1, ty, tx), ye[3], ye[4], ye[5]);     // a = 1
+        stSlot<TC>(SY(2, ty, tx), ye[6], ye[7], ye[8]);     // a = 2
+        stSlot<TC>(SY(3, ty, tx), ye[12], ye[13], ye[14]);  // a = 4
+        stSlot<TC>(SY(4, ty, tx), ye[15], ye[16], ye[17]);  // a = 5
+        stSlot<TC>(SY(5, ty, tx), ye[18], ye[19], ye[20]);  // a = 6
+        __syncthreads();
+        if (owner) {
+            TC lo[3], hi[3], q[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                lo[c] = ye[9 + c];
+                hi[c] = ye[21 + c];
+            }
+            ldSlot<TC>(SY(2, ty, tx + 1), q[0], q[1], q[2]);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) lo[c] += q[c];
+            ldSlot<TC>(SY(1, ty + 1, tx), q[0], q[1], q[2]);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) lo[c] += q[c];
+            ldSlot<TC>(SY(0, ty + 1, tx + 1), q[0], q[1], q[2]);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) lo[c] += q[c];
+            ldSlot<TC>(SY(5, ty, tx + 1), q[0], q[1], q[2]);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) hi[c] += q[c];
+            ldSlot<TC>(SY(4, ty + 1, tx), q[0], q[1], q[2]);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) hi[c] += q[c];
+            ldSlot<TC>(SY(3, ty + 1, tx + 1), q[0], q[1], q[2]);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) hi[c] += q[c];
+            if (k >= z0) {
+                TC sum[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) sum[c] = acc[c] + lo[c];
+                mvOutput<T, TC>(a, (int64_t)oCol + (int64_t)k * plane, sum, fl, xo, d0, d1);
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) acc[c] = hi[c];
+        }
+    }
+#undef SU
+#undef SY
+}
+
 // 4-point Walsh-Hadamard transform of a node quad (corner q = dx + 2 dy), per
 // component: v[3m+c] = sum_q (-1)^popcount(m&q) u[3q+c].
 template <typename T>
