@@ -847,11 +847,6 @@ int matvec(vfem_problem* p, const MatvecArgs<T>& a, bool allowTc = true) {
     return launchMatvec<T>(ctx(p), a, p->ke.structured, opc<T>(p));
 }
 
-// FP64 vectors, double-float arithmetic (the mixed solve's true residual).
-int matvecDF(vfem_problem* p, const MatvecArgs<double>& a) {
-    return launchMatvecDF(ctx(p), a, p->ke.structured, p->op64);
-}
-
 // z = M^-1 r on level `lv` (r, z given); returns kernels; on level 0 the final
 // pass produces r.z (and z.aux) with epilogue `epi`.  *outZ receives the buffer
 // holding the result (it differs from z in the multiplicative cycle when the
@@ -1009,7 +1004,7 @@ int iteration(vfem_problem* p, const vfem_options& o, double** zOut64, float** z
             k += launchUpdateR(c, n, r, p->Ap32);
         }
         k += launchFlushX(c, n, p->x64, p->x32, p->p32, p->p32b, 1);
-        // True residual f - K x64 in double-float; only its FP32 rounding (the new
+        // True residual f - K x64 of the FP64 solution; only its FP32 rounding (the new
         // recursive residual) and its norm are kept.
         MatvecArgs<double> t = mvArgs<double>(p, 0, p->x64, nullptr, MV_RESID);
         t.f = p->f64;
@@ -1017,7 +1012,7 @@ int iteration(vfem_problem* p, const vfem_options& o, double** zOut64, float** z
         t.dot0 = DOT_OUT_OUT;
         t.epi = EPI_TRUE;
         t.condTrue = 1;
-        k += matvecDF(p, t);
+        k += matvec<double>(p, t);
         // a replaced residual is restricted again
         if (fused) k += launchRestrict<float>(c, l0.g, p->L[1].g, 2, r, p->L[1].r32, 2);
         float* z = nullptr;
@@ -1062,12 +1057,8 @@ vfem_status solvePhase(vfem_problem* p, const vfem_options& o, bool haveX0, vfem
         MatvecArgs<double> a = mvArgs<double>(p, 0, p->x64, l0.r64, MV_RESID);
         a.f = p->f64;
         a.checkDone = 0;
-        if (mixed) {
-            a.y32 = l0.r32;
-            launches += matvecDF(p, a);
-        } else {
-            launches += matvec<double>(p, a);
-        }
+        if (mixed) a.y32 = l0.r32;
+        launches += matvec<double>(p, a);
     } else {
         launches += launchFill<double>(p->stream, n, p->x64, 0.0);
         launches += launchConvert<double, double>(p->stream, n, p->f64, l0.r64);
@@ -1727,7 +1718,7 @@ vfem_status vfem_profile_kernels(vfem_problem* p, int32_t reps, double* ms) {
                     a.y32 = l0.t32;
                     a.dot0 = DOT_OUT_OUT;
                     a.epi = EPI_STORE;
-                    return matvecDF(p, a);
+                    return matvec<double>(p, a);
                 }
             }
         };

@@ -1171,7 +1171,6 @@ inline dim3 nodeGrid(const Grid& g) {
 
 cudaError_t setKernelAttributes() {
     const int s64 = (kSuElems + kSyElems) * (int)sizeof(double), s32 = (kSuElems + kSyElems) * (int)sizeof(float);
-    const int sdf = (kSuElems + kSyElems) * (int)sizeof(df);
     const cudaFuncAttribute A = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e;
     if ((e = cudaFuncSetAttribute(kMatvecH<double, double>, A, s64))) return e;
@@ -1179,11 +1178,8 @@ cudaError_t setKernelAttributes() {
     if ((e = cudaFuncSetAttribute(kMatvecH<float, float, OUT_CG>, A, s32))) return e;
     if ((e = cudaFuncSetAttribute(kMatvecH<float, float, OUT_CG_PX>, A, s32))) return e;
     if ((e = cudaFuncSetAttribute(kMatvecH<double, double, OUT_CG>, A, s64))) return e;
-    if ((e = cudaFuncSetAttribute(kMatvecH<double, df, OUT_TRUE>, A, sdf))) return e;
-    if ((e = cudaFuncSetAttribute(kMatvecH<double, df>, A, sdf))) return e;
     if ((e = cudaFuncSetAttribute(kMatvec<double>, A, s64))) return e;
-    if ((e = cudaFuncSetAttribute(kMatvec<float>, A, s32))) return e;
-    return cudaFuncSetAttribute(kMatvec<double, df>, A, sdf);
+    return cudaFuncSetAttribute(kMatvec<float>, A, s32);
 }
 
 template <typename T>
@@ -1217,26 +1213,6 @@ int launchMatvecPX(const LaunchCtx& c, const MatvecArgs<float>& a, const float* 
     Ks<float> k;
     for (int i = 0; i < 45; ++i) k.v[i] = opconst[i];
     kMatvecH<float, float, OUT_CG_PX><<<grid, block, smem, c.stream>>>(a, k, c.S, c.rb);
-    return 1;
-}
-
-int launchMatvecDF(const LaunchCtx& c, const MatvecArgs<double>& a, bool structured, const double* opconst) {
-    const Grid& g = a.g;
-    dim3 grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + MV_TY - 2) / (MV_TY - 1), (g.nz + MV_ZC - 1) / MV_ZC);
-    dim3 block(MV_TX, MV_TY);
-    size_t smem = (size_t)(kSuElems + kSyElems) * sizeof(df);
-    if (structured) {
-        Ks<df> k;
-        for (int i = 0; i < 45; ++i) k.v[i] = df(opconst[i]);
-        if (a.mode == MV_RESID && a.dot0 == DOT_OUT_OUT && !a.dot1 && a.y32)
-            kMatvecH<double, df, OUT_TRUE><<<grid, block, smem, c.stream>>>(a, k, c.S, c.rb);
-        else
-            kMatvecH<double, df><<<grid, block, smem, c.stream>>>(a, k, c.S, c.rb);
-    } else {
-        Kd<df> k;
-        for (int i = 0; i < 576; ++i) k.v[i] = df(opconst[45 + i]);
-        kMatvec<double, df><<<grid, block, smem, c.stream>>>(a, k, c.S, c.rb);
-    }
     return 1;
 }
 

@@ -139,10 +139,6 @@ int fxLayers(const Grid& g);  // node layers a block marches
 void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOperand& op, const double* opconst,
                     Scalars* S, const RedBuf& rb);
 
-// The same product on FP64 vectors in double-float arithmetic (FP32 instructions,
-// ~48-bit significands): the mixed-precision true residual.  a.y may be null.
-int launchMatvecDF(const LaunchCtx& c, const MatvecArgs<double>& a, bool structured, const double* opconst);
-
 // checkDone: 1 = skip once the solve is done; 2 = also skip unless the true
 // residual replaced r in this iteration (2x coarsening only).
 template <typename T>

@@ -386,10 +386,17 @@ __device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const KA& K
             }
         }
         eb = et;
-        double xo[3] = {0.0, 0.0, 0.0};  // in flight across the transform and the barrier
-        if (owner && k >= z0 && (OUT == OUT_CG || a.mode == MV_SMOOTH || a.dot0 == DOT_X_OUT)) {
-            const double* p = a.x + 3 * ((int64_t)oCol + (int64_t)k * plane);
-            xo[0] = p[0]; xo[1] = p[1]; xo[2] = p[2];
+        // x or f at the owned node, in flight across the transform and the barrier
+        double xo[3] = {0.0, 0.0, 0.0}, fo[3] = {0.0, 0.0, 0.0};
+        if (owner && k >= z0) {
+            const int64_t i = 3 * ((int64_t)oCol + (int64_t)k * plane);
+            if (OUT == OUT_TRUE) {
+                const double* p = a.f + i;
+                fo[0] = p[0]; fo[1] = p[1]; fo[2] = p[2];
+            } else if (OUT == OUT_CG || a.mode == MV_SMOOTH || a.dot0 == DOT_X_OUT) {
+                const double* p = a.x + i;
+                xo[0] = p[0]; xo[1] = p[1]; xo[2] = p[2];
+            }
         }
         if constexpr (!DENSE) fwht4x3i(nb);
 #pragma unroll
@@ -424,6 +431,15 @@ __device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const KA& K
                     const double out = fixed ? 0.0 : sum[c];
                     a.y[3 * s + c] = out;
                     if (live) dAx = fma(xo[c], out, dAx);
+                }
+            } else if constexpr (OUT == OUT_TRUE) {
+                const bool fixed = (fl & FLAG_FIXED) != 0;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const double out = fo[c] - (fixed ? 0.0 : sum[c]);
+                    if (a.y) a.y[3 * s + c] = out;
+                    a.y32[3 * s + c] = (float)out;
+                    d0.add(out * out);
                 }
             } else {
                 mvOutput<double, double>(a, s, sum, fl, xo, d0, d1);
@@ -537,6 +553,7 @@ cudaError_t fxSetAttributes() {
     };
     set(kMatvecFx<OUT_CG, FxArgs, Ks<double>>);
     set(kMatvecFx<OUT_ANY, FxArgs, Ks<double>>);
+    set(kMatvecFx<OUT_TRUE, FxArgs, Ks<double>>);
     set(kMatvecFx<OUT_CG, FxDenseArgs, Kd<double>>);
     set(kMatvecFx<OUT_ANY, FxDenseArgs, Kd<double>>);
     return e;
@@ -555,7 +572,8 @@ void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOp
     const dim3 block(MV_TX, FX_TY),
         grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + FX_TY - 2) / (FX_TY - 1), (g.nz + zc - 1) / zc);
     const bool cg = a.mode == MV_AX && a.dot0 == DOT_X_OUT && !a.dot1 && !a.y32;
-    auto go = [&](auto K, int rows, int cols, auto k, const double* src, auto kernCg, auto kernAny) {
+    const bool tr = a.mode == MV_RESID && a.dot0 == DOT_OUT_OUT && !a.dot1 && a.y32;
+    auto go = [&](auto K, int rows, int cols, auto k, const double* src, auto kern) {
         for (int i = 0; i < rows * cols; ++i) {
             K.k1[i] = op.k1[i];
             K.k0[i] = op.k0[i];
@@ -569,14 +587,15 @@ void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOp
         K.scaleExp = e - 1;
         K.outExp = op.outExp;
         std::memcpy(k.v, src, sizeof(k.v));
-        (cg ? kernCg : kernAny)<<<grid, block, fxSmemBytes<FX_TY>(), stream>>>(a, K, k, zc, S, rb);
+        kern<<<grid, block, fxSmemBytes<FX_TY>(), stream>>>(a, K, k, zc, S, rb);
     };
     if (op.cube)
-        go(FxArgs(), 8, 1, Ks<double>(), opconst, kMatvecFx<OUT_CG, FxArgs, Ks<double>>,
-           kMatvecFx<OUT_ANY, FxArgs, Ks<double>>);
+        go(FxArgs(), 8, 1, Ks<double>(), opconst,
+           cg ? kMatvecFx<OUT_CG, FxArgs, Ks<double>>
+              : tr ? kMatvecFx<OUT_TRUE, FxArgs, Ks<double>> : kMatvecFx<OUT_ANY, FxArgs, Ks<double>>);
     else
-        go(FxDenseArgs(), 24, 24, Kd<double>(), opconst + 45, kMatvecFx<OUT_CG, FxDenseArgs, Kd<double>>,
-           kMatvecFx<OUT_ANY, FxDenseArgs, Kd<double>>);
+        go(FxDenseArgs(), 24, 24, Kd<double>(), opconst + 45,
+           cg ? kMatvecFx<OUT_CG, FxDenseArgs, Kd<double>> : kMatvecFx<OUT_ANY, FxDenseArgs, Kd<double>>);
 }
 
 int fxLayers(const Grid& g) {

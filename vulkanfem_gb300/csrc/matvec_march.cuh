@@ -1,8 +1,8 @@
 // matvec_march.cuh -- the element-by-element product's building blocks shared by
-// its translation units: double-float arithmetic, the Walsh-basis element
-// product, the output stage and the march up a z range (kernels.cu: FP32, FP64
-// and double-float kernels; matvec_fx.cu: the fixed-point FP64 product, which
-// hands blocks it cannot represent to the FP64 march).  Everything here has
+// its translation units: the Walsh-basis and dense element products, the output
+// stage and the march up a z range (kernels.cu: FP32 and FP64 kernels;
+// matvec_fx.cu: the fixed-point FP64 product, which hands blocks it cannot
+// represent to the FP64 march).  Everything here has
 // internal linkage (one copy per translation unit).
 #pragma once
 
@@ -16,61 +16,9 @@ namespace {
 
 constexpr int MV_TX = 32, MV_TY = 8, MV_ZC = 32;  // z layers per product block (32: 5% faster than 16)
 
-// Double-float ("df") numbers: the unevaluated sum hi + lo of two FP32 values,
-// about 48 significant bits, computed with FP32 instructions only (Dekker 1971:
-// TwoSum / FastTwoSum; the product error from one FMA).  GB300 issues FP64 at
-// about 1/64 of its FP32 rate, so the mixed-precision solve evaluates its true
-// residual f - K x in df: relative rounding ~1e-14 of the summed magnitudes,
-// several times faster than the FP64 product.  Addition is the "sloppy" variant
-// (error bounded by ~2^-44 (|a| + |b|)), ample for a residual that is compared
-// with 1e-6 |f|.  The compiler must not re-associate these expressions, which
-// nvcc does not do without fast-math flags.
-struct df {
-    float hi, lo;
-    df() = default;
-    __host__ __device__ constexpr df(float h, float l) : hi(h), lo(l) {}
-    __host__ __device__ constexpr explicit df(int v) : hi((float)v), lo(0.f) {}
-    __host__ __device__ constexpr explicit df(float v) : hi(v), lo(0.f) {}
-    __host__ __device__ explicit df(double v) : hi((float)v), lo((float)(v - (double)(float)v)) {}
-};
-
-__device__ __forceinline__ df dfTwoSum(float a, float b) {
-    const float s = a + b;
-    const float bb = s - a;
-    return df(s, (a - (s - bb)) + (b - bb));
-}
-__device__ __forceinline__ df dfFastTwoSum(float a, float b) {  // |a| >= |b|
-    const float s = a + b;
-    return df(s, b - (s - a));
-}
-__device__ __forceinline__ df operator+(df a, df b) {
-    const df s = dfTwoSum(a.hi, b.hi);
-    return dfFastTwoSum(s.hi, s.lo + (a.lo + b.lo));
-}
-__device__ __forceinline__ df operator-(df a, df b) { return a + df(-b.hi, -b.lo); }
-__device__ __forceinline__ df operator*(df a, df b) {
-    const float p = a.hi * b.hi;
-    float e = fmaf(a.hi, b.hi, -p);
-    e = fmaf(a.hi, b.lo, e);
-    e = fmaf(a.lo, b.hi, e);
-    return dfFastTwoSum(p, e);
-}
-__device__ __forceinline__ df& operator+=(df& a, df b) { return a = a + b; }
-__device__ __forceinline__ df& operator*=(df& a, df b) { return a = a * b; }
-// The df overload below would hide the global fma from unqualified calls in
-// this namespace; these restore the FP32 and FP64 forms.
+// One name for both FP32 and FP64 multiply-adds in the templates below.
 __device__ __forceinline__ float fma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma(double a, double b, double c) { return ::fma(a, b, c); }
-// a * b + c with one renormalisation.
-__device__ __forceinline__ df fma(df a, df b, df c) {
-    const float p = a.hi * b.hi;
-    const float pe = fmaf(a.hi, b.hi, -p);
-    const df s = dfTwoSum(p, c.hi);
-    float t = s.lo + (pe + c.lo);
-    t = fmaf(a.hi, b.lo, t);
-    t = fmaf(a.lo, b.hi, t);
-    return dfFastTwoSum(s.hi, t);
-}
 
 // Conversions between a storage type T and a compute type TC of the matvec.
 template <typename T, typename TC>
@@ -78,24 +26,8 @@ struct Cvt {
     static __device__ __forceinline__ TC in(T v) { return TC(v); }
     static __device__ __forceinline__ T out(TC v) { return T(v); }
 };
-template <>
-struct Cvt<double, df> {
-    static __device__ __forceinline__ df in(double v) {
-        const float h = __double2float_rn(v);
-        return df(h, __double2float_rn(v - (double)h));
-    }
-    static __device__ __forceinline__ double out(df v) { return (double)v.hi + (double)v.lo; }
-};
 __device__ __forceinline__ float toF(float v) { return v; }
 __device__ __forceinline__ float toF(double v) { return (float)v; }
-__device__ __forceinline__ float toF(df v) { return v.hi; }  // hi is v rounded to FP32
-
-template <>
-struct DotAcc<df> {
-    df s = df(0.f, 0.f);
-    __device__ __forceinline__ void add(df v) { s = s + v; }
-    __device__ __forceinline__ double get() const { return (double)s.hi + (double)s.lo; }
-};
 
 template <typename T>
 struct Ks {
@@ -154,20 +86,8 @@ __device__ __forceinline__ void stSlot<double>(double* p, double a, double b, do
     reinterpret_cast<double2*>(p)[0] = make_double2(a, b);
     reinterpret_cast<double2*>(p)[1] = make_double2(c, 0.0);
 }
-template <>
-__device__ __forceinline__ void stSlot<df>(df* p, df a, df b, df c) {
-    reinterpret_cast<float4*>(p)[0] = make_float4(a.hi, a.lo, b.hi, b.lo);
-    reinterpret_cast<float4*>(p)[1] = make_float4(c.hi, c.lo, 0.f, 0.f);
-}
 template <typename T>
 __device__ __forceinline__ void ldSlot(const T* p, T& a, T& b, T& c);
-template <>
-__device__ __forceinline__ void ldSlot<df>(const df* p, df& a, df& b, df& c) {
-    const float4 v0 = reinterpret_cast<const float4*>(p)[0], v1 = reinterpret_cast<const float4*>(p)[1];
-    a = df(v0.x, v0.y);
-    b = df(v0.z, v0.w);
-    c = df(v1.x, v1.y);
-}
 template <>
 __device__ __forceinline__ void ldSlot<float>(const float* p, float& a, float& b, float& c) {
     const float4 v = *reinterpret_cast<const float4*>(p);
@@ -208,8 +128,7 @@ __device__ __forceinline__ void mvOutput(const MatvecArgs<T>& a, int64_t s, cons
             case MV_RESID0: out = fixed ? TC(0) : fv - ax; break;
             default: out = fixed ? TC(0) : xv + TC(a.omega) * C::in(a.dinv[3 * s + c]) * (fv - ax); break;
         }
-        if constexpr (std::is_same<T, TC>::value) a.y[3 * s + c] = out;
-        else if (a.y) a.y[3 * s + c] = C::out(out);
+        if (std::is_same<T, float>::value || a.y) a.y[3 * s + c] = C::out(out);
         if (a.y32) a.y32[3 * s + c] = toF(out);
         if (a.dot0 == DOT_X_OUT) d0.add(live ? xv * out : TC(0));
         else if (a.dot0 == DOT_OUT_OUT) d0.add(out * out);
@@ -234,8 +153,7 @@ __device__ __forceinline__ void mvOutput(const MatvecArgs<T>& a, int64_t s, cons
 // loaded without integer division: every thread loads its own slot, row 8
 // comes from the ty == 0 threads and column 32 from nine threads of row 1.
 //
-// T is the storage type of the vectors, TC the arithmetic type (T, or df for
-// the true residual of the mixed-precision solve: FP64 vectors, df arithmetic).
+// T is the storage type of the vectors, TC the arithmetic type.
 // One block's march: fills d0 and d1 (this thread's dots).
 template <typename T, typename TC>
 __device__ __forceinline__ void denseMarch(const MatvecArgs<T>& a, const Kd<TC>& kp, unsigned char* smemRaw,
@@ -486,7 +404,7 @@ __device__ __forceinline__ void foldCarry<float>(const float (&y)[24], float (&c
 // Same tile, pipelining and output stage as kMatvec.  The two Walsh-domain
 // carries stay in registers across the z march.  Launch bounds, measured on
 // the 256^3 workload: FP32 3 blocks per SM (80 registers, no spills; 4 blocks
-// spill and run 33% slower); FP64 and df 2 blocks per SM (128 registers, a few
+// spill and run 33% slower); FP64 2 blocks per SM (128 registers, a few
 // spilled values; 20% faster than 1 block without spills).
 //
 // OUT selects the output stage at compile time (runtime mode switches in the
