@@ -58,96 +58,178 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 }
 
 // ----------------------------------------------------------------------------- convolution
-// Implicit GEMM: out[v][co] = sum_{tap, ci} in[v + off(tap)][ci] * W[tap][ci][co] (+ bias, relu).
-// Block: 128 threads (4 warps) computes 64 consecutive voxels x 64 output channels
-// (or Cout if smaller).  K loop over 27 taps x Cin/16 chunks; A (64 x 16) and B
-// (16 x 64) staged in shared memory; each warp owns 16 voxel rows.
-constexpr int CT_M = 64, CT_N = 64, CT_K = 16;
+// Implicit GEMM: out[v][co] = sum_{tap, ci} in[v + off(tap)][ci] * W[tap][ci][co] (+ bias, relu),
+// summed tap by tap and 16 channels at a time (the order every shape keeps).
+//
+// A block stages the halo of an 8 x 8 x TZ voxel tile, all channels, in shared
+// memory once and reads the 27 shifted operands from there with ldmatrix: a
+// voxel's 16 channels are one 32-byte row, so a shift is only an address.  A row
+// of 16 voxels is two x rows of 8; the voxel stride of 32 CK + 16 bytes puts any
+// 8 of them in different banks.  Each of the 2 TZ warps owns 32 voxels and all
+// 8 NT output channels of the block.  Weights pass through shared memory in
+// stages of TG taps, double-buffered; where all 27 fit (TG = 27) they stay for
+// the block's further tiles.  The input may be two tensors: channels [0, Ca)
+// from `a` at half resolution (nearest upsampling) and the rest from `b`, which
+// spares writing the decoder's concatenation.
+//
+// The earlier kernel staged 64 x 16 operands for every tap and 16 channels from
+// global memory (index arithmetic, two barriers and 2 to 8 MMAs a step).
+// Measured on GB300, 16 -> 16 channels at 136^3: 687 -> 134 us; 48 -> 16 there with
+// the concatenation: 2,480 -> 441 us; 192 -> 64 at 34^3: 396 -> 138 us; same bits.
+// Bound: shared-memory reads of A (512 bytes for 2 NT MMAs) where NT = 2.
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+// 16-byte asynchronous copy; zeros when !ok (src must be a valid address all the same).
+__device__ __forceinline__ void cpAsync16(uint32_t dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cpCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cpWait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
-template <bool OUT_F32>
-__global__ void __launch_bounds__(128) kConvFwd(const bf16* __restrict__ in, const bf16* __restrict__ W,
-                                                const float* __restrict__ bias, void* __restrict__ out, int n, int Cin,
-                                                int Cout, int relu) {
-    __shared__ __align__(16) bf16 sA[CT_M][CT_K + 8];   // +8: break bank conflicts
-    __shared__ __align__(16) bf16 sB[CT_K][CT_N + 8];
-    __shared__ int sxyz[CT_M][3];
+// An activation tensor read by the GEMM kernels: channels [0, Ca) of `a` at half
+// resolution, then Cb of `b` (Ca = 0: b alone).
+struct Input {
+    const bf16* a;
+    const bf16* b;
+    int Ca, Cb;
+};
+
+constexpr int HALO = 10;  // tile edge 8 and one voxel on each side
+template <int CK>
+__host__ __device__ constexpr int rowBytes() { return 32 * CK + 16; }
+
+// Copies the halo of the tile at (x0, y0, z0), TZ + 2 layers of 10 x 10 voxels, zeros outside the grid.
+template <int CK, int TZ, int NTH>
+__device__ __forceinline__ void stageHalo(uint32_t dst, const Input& in, int n, int x0, int y0, int z0) {
+    constexpr int Q = 2 * CK, TOT = HALO * HALO * (TZ + 2) * Q;
+    const int C = 16 * CK, nh = n >> 1;
+    for (int i = threadIdx.x; i < TOT; i += NTH) {
+        const int q = i % Q, h = i / Q;
+        const int hx = h % HALO, hy = (h / HALO) % HALO, hz = h / (HALO * HALO);
+        const int x = x0 + hx - 1, y = y0 + hy - 1, z = z0 + hz - 1;
+        const bool ok = x >= 0 && x < n && y >= 0 && y < n && z >= 0 && z < n;
+        const bf16* src = in.b;
+        if (ok) {
+            if (8 * q < in.Ca)
+                src = in.a + ((((int64_t)(z >> 1) * nh + (y >> 1)) * nh + (x >> 1)) * in.Ca + 8 * q);
+            else
+                src = in.b + ((((int64_t)z * n + y) * n + x) * (C - in.Ca) + 8 * q - in.Ca);
+        }
+        cpAsync16(dst + (uint32_t)(h * rowBytes<CK>() + 16 * q), src, ok);
+    }
+}
+
+template <int CK, int NT, int TG, int TZ>
+constexpr size_t convSmem() {
+    return (size_t)HALO * HALO * (TZ + 2) * rowBytes<CK>() +
+           (size_t)(TG == 27 ? 1 : 2) * TG * 16 * CK * (16 * NT + 16);
+}
+
+template <int CK, int NT, int TG, int TZ, bool OUT_F32>
+__global__ void __launch_bounds__(64 * TZ) kConv(const Input in, const bf16* __restrict__ W,
+                                                 const float* __restrict__ bias, void* __restrict__ out, int n,
+                                                 int Cout, int relu) {
+    constexpr int NTH = 64 * TZ, NS = 27 / TG, ROW = rowBytes<CK>(), WROW = 16 * NT + 16;
+    constexpr uint32_t haloBytes = HALO * HALO * (TZ + 2) * ROW, stageBytes = TG * 16 * CK * WROW;
+    extern __shared__ __align__(16) unsigned char convSm[];
+    const uint32_t sA = (uint32_t)__cvta_generic_to_shared(convSm), sB = sA + haloBytes;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t V = (int64_t)n * n * n;
-    const int64_t v0 = (int64_t)blockIdx.x * CT_M;
-    const int n0 = blockIdx.y * CT_N;
-    const int nt = min(CT_N, Cout - n0);  // multiple of 16
-    if (tid < CT_M) {
-        const int64_t v = v0 + tid;
-        sxyz[tid][0] = (int)(v % n);
-        sxyz[tid][1] = (int)((v / n) % n);
-        sxyz[tid][2] = (int)(v / ((int64_t)n * n));
-    }
-    float acc[CT_N / 8][4];
+    const int n0 = blockIdx.y * (8 * NT);
+    const int tx = (n + 7) >> 3, tz = (n + TZ - 1) / TZ, tiles = tx * tx * tz;
+    auto stageW = [&](int s, int buf) {
+        constexpr int Q = NT, TOT = TG * 16 * CK * Q;  // 16-byte pieces
+        for (int i = tid; i < TOT; i += NTH) {
+            const int q = i % Q, k = i / Q;
+            cpAsync16(sB + buf * stageBytes + k * WROW + 16 * q,
+                      W + ((int64_t)s * TG * 16 * CK + k) * Cout + n0 + 8 * q, true);
+        }
+    };
+    // ldmatrix addresses of this lane: A row (lane & 15) of the warp's first 16 voxels,
+    // channel half lane >> 4; B row k, column half
+    const int wz = warp >> 1, wy = (warp & 1) * 4;
+    const uint32_t aLane =
+        sA + (uint32_t)(((wz * HALO + wy + ((lane >> 3) & 1)) * HALO + (lane & 7)) * ROW + 16 * (lane >> 4));
+    const uint32_t bLane = sB + (uint32_t)(((lane & 7) + 8 * ((lane >> 3) & 1)) * WROW + 16 * (lane >> 4));
+    if (NS == 1) stageW(0, 0);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int x0 = (tile % tx) * 8, y0 = (tile / tx) % tx * 8, z0 = tile / (tx * tx) * TZ;
+        stageHalo<CK, TZ, NTH>(sA, in, n, x0, y0, z0);
+        if (NS > 1) stageW(0, 0);
+        cpCommit();
+        float acc[2][NT][4];
 #pragma unroll
-    for (int j = 0; j < CT_N / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    __syncthreads();
-    const int g = lane >> 2, t4 = lane & 3;
-    for (int tap = 0; tap < 27; ++tap) {
-        const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-        for (int c0 = 0; c0 < Cin; c0 += CT_K) {
-            // A: 64 voxels x 16 channels, one 8-channel half per thread.
-            {
-                const int r = tid >> 1, h = tid & 1;
-                const int x = sxyz[r][0] + dx, y = sxyz[r][1] + dy, z = sxyz[r][2] + dz;
-                uint4 val = make_uint4(0, 0, 0, 0);
-                if (v0 + r < V && x >= 0 && x < n && y >= 0 && y < n && z >= 0 && z < n) {
-                    const int64_t src = ((int64_t)z * n + y) * n + x;
-                    val = *reinterpret_cast<const uint4*>(in + src * Cin + c0 + 8 * h);
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[m][j][e] = 0.f;
+        for (int s = 0; s < NS; ++s) {
+            cpWait<0>();
+            __syncthreads();
+            if (s + 1 < NS) {
+                stageW(s + 1, (s + 1) & 1);
+                cpCommit();
+            }
+            const uint32_t b0 = bLane + (NS > 1 ? (s & 1) * stageBytes : 0);
+#pragma unroll 3
+            for (int t = 0; t < TG; ++t) {
+                const int tap = s * TG + t;
+                const uint32_t aTap =
+                    aLane + (uint32_t)((((tap / 9) * HALO + (tap / 3) % 3) * HALO + tap % 3) * ROW);
+#pragma unroll
+                for (int c = 0; c < CK; ++c) {
+                    uint32_t A[2][4];
+                    ldsm4(A[0], aTap + 32 * c);
+                    ldsm4(A[1], aTap + 32 * c + 2 * HALO * ROW);
+#pragma unroll
+                    for (int j = 0; j < NT; j += 2) {
+                        uint32_t B[4];
+                        ldsm4t(B, b0 + (uint32_t)((t * CK + c) * 16 * WROW + 16 * j));
+#pragma unroll
+                        for (int m = 0; m < 2; ++m) {
+                            mma16816(acc[m][j], A[m][0], A[m][1], A[m][2], A[m][3], B[0], B[1]);
+                            mma16816(acc[m][j + 1], A[m][0], A[m][1], A[m][2], A[m][3], B[2], B[3]);
+                        }
+                    }
                 }
-                *reinterpret_cast<uint4*>(&sA[r][8 * h]) = val;
-            }
-            // B: 16 input channels x nt output channels.
-            for (int i = tid; i < CT_K * (nt / 8); i += 128) {
-                const int k = i / (nt / 8), q = i % (nt / 8);
-                *reinterpret_cast<uint4*>(&sB[k][8 * q]) =
-                    *reinterpret_cast<const uint4*>(W + ((int64_t)tap * Cin + c0 + k) * Cout + n0 + 8 * q);
-            }
-            __syncthreads();
-            const int rb = warp * 16;
-            const uint32_t a0 = pack2(sA[rb + g][2 * t4], sA[rb + g][2 * t4 + 1]);
-            const uint32_t a1 = pack2(sA[rb + g + 8][2 * t4], sA[rb + g + 8][2 * t4 + 1]);
-            const uint32_t a2 = pack2(sA[rb + g][2 * t4 + 8], sA[rb + g][2 * t4 + 9]);
-            const uint32_t a3 = pack2(sA[rb + g + 8][2 * t4 + 8], sA[rb + g + 8][2 * t4 + 9]);
-#pragma unroll
-            for (int j = 0; j < CT_N / 8; ++j) {
-                if (8 * j >= nt) break;
-                const uint32_t b0 = pack2(sB[2 * t4][8 * j + g], sB[2 * t4 + 1][8 * j + g]);
-                const uint32_t b1 = pack2(sB[2 * t4 + 8][8 * j + g], sB[2 * t4 + 9][8 * j + g]);
-                mma16816(acc[j], a0, a1, a2, a3, b0, b1);
-            }
-            __syncthreads();
-        }
-    }
-    const int rb = warp * 16;
-#pragma unroll
-    for (int j = 0; j < CT_N / 8; ++j) {
-        if (8 * j >= nt) break;
-#pragma unroll
-        for (int hrow = 0; hrow < 2; ++hrow) {
-            const int64_t v = v0 + rb + g + 8 * hrow;
-            if (v >= V) continue;
-            const int co = n0 + 8 * j + 2 * t4;
-            float y0 = acc[j][2 * hrow] + (bias ? bias[co] : 0.f);
-            float y1 = acc[j][2 * hrow + 1] + (bias ? bias[co + 1] : 0.f);
-            if (relu) {
-                y0 = fmaxf(y0, 0.f);
-                y1 = fmaxf(y1, 0.f);
-            }
-            if (OUT_F32) {
-                float* o = static_cast<float*>(out) + v * Cout + co;
-                o[0] = y0;
-                o[1] = y1;
-            } else {
-                bf16* o = static_cast<bf16*>(out) + v * Cout + co;
-                o[0] = __float2bfloat16(y0);
-                o[1] = __float2bfloat16(y1);
             }
         }
+        const int g = lane >> 2, t4 = lane & 3, x = x0 + g, z = z0 + wz;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int hrow = 0; hrow < 2; ++hrow) {
+                const int y = y0 + wy + 2 * m + hrow;
+                if (x >= n || y >= n || z >= n) continue;
+                const int64_t v = ((int64_t)z * n + y) * n + x;
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    const int co = n0 + 8 * j + 2 * t4;
+                    float r0 = acc[m][j][2 * hrow] + (bias ? bias[co] : 0.f);
+                    float r1 = acc[m][j][2 * hrow + 1] + (bias ? bias[co + 1] : 0.f);
+                    if (relu) {
+                        r0 = fmaxf(r0, 0.f);
+                        r1 = fmaxf(r1, 0.f);
+                    }
+                    if (OUT_F32)
+                        *reinterpret_cast<float2*>(static_cast<float*>(out) + v * Cout + co) = make_float2(r0, r1);
+                    else
+                        *reinterpret_cast<__nv_bfloat162*>(static_cast<bf16*>(out) + v * Cout + co) =
+                            __floats2bfloat162_rn(r0, r1);
+                }
+            }
+        __syncthreads();  // the halo is free for the next tile
     }
 }
 
@@ -451,34 +533,88 @@ cudaError_t nalloc(T** p, int64_t n) {
     return cudaStreamSynchronize(cudaStreamLegacy);
 }
 
-void conv(vfem_net* N, const bf16* in, const bf16* W, const float* b, void* out, int lvl, int Cin, int Cout, int relu,
-          bool f32) {
-    const int n = N->n >> lvl;
-    dim3 grid((unsigned)((N->V[lvl] + CT_M - 1) / CT_M), (unsigned)((Cout + CT_N - 1) / CT_N));
-    if (f32) kConvFwd<true><<<grid, 128, 0, N->stream>>>(in, W, b, out, n, Cin, Cout, relu);
-    else kConvFwd<false><<<grid, 128, 0, N->stream>>>(in, W, b, out, n, Cin, Cout, relu);
+// One convolution at level lvl: (Cin, Cout) as the network has them, forward and data gradient.
+// TZ: 8 x 8 x 4 tiles, or 8 x 8 x 2 where the halo is large (Cin >= 128) or the level
+// has too few voxels to fill the GPU's 152 SMs with the taller ones.
+template <int CK, int NT, int TG, int TZ, bool F32>
+void launchConv(vfem_net* N, const Input& in, const bf16* W, const float* b, void* out, int n, int Cout, int relu) {
+    constexpr size_t smem = convSmem<CK, NT, TG, TZ>();
+    static_assert(smem <= 227 * 1024, "tile too large");
+    auto kern = kConv<CK, NT, TG, TZ, F32>;
+    static const int perSm = [&] {
+        int k = 0;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, 64 * TZ, smem);
+        return std::max(1, k);
+    }();
+    const int tx = (n + 7) / 8, tiles = tx * tx * ((n + TZ - 1) / TZ), parts = Cout / (8 * NT);
+    const dim3 grid((unsigned)std::min(tiles, std::max(1, 152 * perSm / parts)), (unsigned)parts);
+    kern<<<grid, 64 * TZ, smem, N->stream>>>(in, W, b, out, n, Cout, relu);
+}
+
+template <bool F32>
+void conv(vfem_net* N, const Input& in, const bf16* W, const float* b, void* out, int lvl, int Cout, int relu) {
+    const int n = N->n >> lvl, Cin = in.Ca + in.Cb;
+    const bool low = (int64_t)n * n * n < 152 * 256;  // fewer tall tiles than SMs
+#define CONV_CASE(ci, co, nt, tg, tz)                                                                  \
+    if (Cin == ci && Cout == co) {                                                                     \
+        if (low) return launchConv<ci / 16, nt, tg, 2, F32>(N, in, W, b, out, n, Cout, relu);          \
+        return launchConv<ci / 16, nt, tg, tz, F32>(N, in, W, b, out, n, Cout, relu);                  \
+    }
+    if constexpr (!F32) {
+        CONV_CASE(16, 32, 4, 27, 4)
+        CONV_CASE(32, 64, 8, 3, 4)
+        CONV_CASE(64, 128, 8, 1, 4)
+        CONV_CASE(192, 64, 8, 1, 2)
+        CONV_CASE(96, 32, 4, 1, 4)
+        CONV_CASE(48, 16, 2, 3, 4)
+    } else {
+        CONV_CASE(16, 48, 6, 27, 4)
+        CONV_CASE(32, 96, 6, 3, 4)
+        CONV_CASE(64, 192, 8, 1, 4)
+        CONV_CASE(128, 64, 8, 1, 2)
+        CONV_CASE(64, 32, 4, 1, 4)
+        CONV_CASE(32, 16, 2, 27, 4)
+    }
+    CONV_CASE(16, 16, 2, 27, 4)
+#undef CONV_CASE
+}
+
+// BF16 working weights of the current master weights (after set_params and every Adam step).
+void castWeights(vfem_net* N) {
+    for (int l = 0; l < kLayers; ++l)
+        kCastWeights<<<blocks(27LL * kCin[l] * kCout[l]), 256, 0, N->stream>>>(N->w + N->woff[l], N->wb[l], N->wt[l],
+                                                                                 kCin[l], kCout[l]);
+}
+
+// The input of convolution l.
+Input layerInput(const vfem_net* N, int l) {
+    switch (l) {
+        case 0: return {nullptr, N->x, 0, 16};
+        case 1: case 2: case 3: return {nullptr, N->p[l], 0, kCin[l]};
+        case 4: return {N->e[3], N->e[2], 128, 64};
+        case 5: return {N->d[2], N->e[1], 64, 32};
+        case 6: return {N->d[1], N->e[0], 32, 16};
+        default: return {nullptr, N->d[0], 0, 16};
+    }
 }
 
 void forward(vfem_net* N) {
     const int64_t* V = N->V;
-    for (int l = 0; l < kLayers; ++l)
-        kCastWeights<<<blocks(27LL * kCin[l] * kCout[l]), 256, 0, N->stream>>>(N->w + N->woff[l], N->wb[l], N->wt[l],
-                                                                                 kCin[l], kCout[l]);
-    auto B = [&](int l) { return N->w + N->boff[l]; };
-    conv(N, N->x, N->wb[0], B(0), N->e[0], 0, 16, 16, 1, false);
+    auto layer = [&](int l, bf16* out) {
+        conv<false>(N, layerInput(N, l), N->wb[l], N->w + N->boff[l], out, kLevel[l], kCout[l], 1);
+    };
+    layer(0, N->e[0]);
     kPool<<<blocks(V[1] * 16), 256, 0, N->stream>>>(N->e[0], N->p[1], N->n / 2, 16);
-    conv(N, N->p[1], N->wb[1], B(1), N->e[1], 1, 16, 32, 1, false);
+    layer(1, N->e[1]);
     kPool<<<blocks(V[2] * 32), 256, 0, N->stream>>>(N->e[1], N->p[2], N->n / 4, 32);
-    conv(N, N->p[2], N->wb[2], B(2), N->e[2], 2, 32, 64, 1, false);
+    layer(2, N->e[2]);
     kPool<<<blocks(V[3] * 64), 256, 0, N->stream>>>(N->e[2], N->p[3], N->n / 8, 64);
-    conv(N, N->p[3], N->wb[3], B(3), N->e[3], 3, 64, 128, 1, false);
-    kUpConcat<<<blocks(V[2] * 192), 256, 0, N->stream>>>(N->e[3], N->e[2], N->c[2], N->n / 4, 128, 64);
-    conv(N, N->c[2], N->wb[4], B(4), N->d[2], 2, 192, 64, 1, false);
-    kUpConcat<<<blocks(V[1] * 96), 256, 0, N->stream>>>(N->d[2], N->e[1], N->c[1], N->n / 2, 64, 32);
-    conv(N, N->c[1], N->wb[5], B(5), N->d[1], 1, 96, 32, 1, false);
-    kUpConcat<<<blocks(V[0] * 48), 256, 0, N->stream>>>(N->d[1], N->e[0], N->c[0], N->n, 32, 16);
-    conv(N, N->c[0], N->wb[6], B(6), N->d[0], 0, 48, 16, 1, false);
-    conv(N, N->d[0], N->wb[7], B(7), N->y, 0, 16, 16, 0, true);
+    layer(3, N->e[3]);
+    layer(4, N->d[2]);
+    layer(5, N->d[1]);
+    layer(6, N->d[0]);
+    conv<true>(N, layerInput(N, 7), N->wb[7], N->w + N->boff[7], N->y, 0, 16, 0);
 }
 
 // Backward of one convolution: given dL/d(out) in gout (f32, [V][Cout]) and the
@@ -495,11 +631,14 @@ void convBwd(vfem_net* N, int l, const bf16* in, const bf16* out, const float* g
     kConvWGrad<<<gw, 128, 0, N->stream>>>(in, N->gmask, N->wgPart, n, Cin, Cout);
     const int64_t per = 27LL * Cin * Cout;
     kWGradSum<<<blocks(per), 256, 0, N->stream>>>(N->wgPart, N->gw + N->woff[l], per, chunks);
-    if (wantIn) conv(N, N->gmask, N->wt[l], nullptr, gin, lvl, Cout, Cin, 0, true);
+    if (wantIn) conv<true>(N, Input{nullptr, N->gmask, 0, Cout}, N->wt[l], nullptr, gin, lvl, Cin, 0);
 }
 
 void backward(vfem_net* N) {
     const int64_t* V = N->V;
+    kUpConcat<<<blocks(V[2] * 192), 256, 0, N->stream>>>(N->e[3], N->e[2], N->c[2], N->n / 4, 128, 64);
+    kUpConcat<<<blocks(V[1] * 96), 256, 0, N->stream>>>(N->d[2], N->e[1], N->c[1], N->n / 2, 64, 32);
+    kUpConcat<<<blocks(V[0] * 48), 256, 0, N->stream>>>(N->d[1], N->e[0], N->c[0], N->n, 32, 16);
     // y = conv7(d0)
     convBwd(N, 7, N->d[0], nullptr, N->gy, N->gd[0], true);
     // d0 = relu(conv6(c0))
@@ -617,6 +756,7 @@ vfem_status vfem_net_set_params(vfem_net* N, const float* params) {
     NCK(cudaMemcpyAsync(N->w, params, sizeof(float) * N->nparam, cudaMemcpyHostToDevice, N->stream));
     NCK(cudaMemsetAsync(N->m, 0, sizeof(float) * N->nparam, N->stream));
     NCK(cudaMemsetAsync(N->v, 0, sizeof(float) * N->nparam, N->stream));
+    castWeights(N);
     N->step = 0;
     NCK(cudaStreamSynchronize(N->stream));
     return VFEM_OK;
@@ -686,6 +826,7 @@ vfem_status vfem_net_train_batch(vfem_net* N, const float* inputs, const float* 
         const float c1 = 1.f - std::pow(b1, (float)N->step), c2 = 1.f - std::pow(b2, (float)N->step);
         kAdam<<<blocks(N->nparam), 256, 0, N->stream>>>(N->w, N->gw, N->m, N->v, N->nparam, lr, b1, b2, 1e-8f, c1, c2,
                                                         1.f / (float)batch);
+        castWeights(N);
         NCK(cudaGetLastError());
         NCK(cudaStreamSynchronize(N->stream));
     }
