@@ -16,9 +16,10 @@
 //   d1 = relu(conv([up2(d2), e1],  96->32))  @ n/2
 //   d0 = relu(conv([up2(d1), e0],  48->16))  @ n
 //   y  = conv(d0, 16->16)  (channels 0..2 are the prediction)
-// Kernels: kConvFwd (implicit GEMM; also the data gradient with flipped,
-// transposed weights), kConvWGrad (weight gradient, split over voxels), pooling,
-// nearest upsampling, concat/split, ReLU mask, bias gradient, masked MSE, Adam.
+// Kernels: kConv (implicit GEMM; also the data gradient with flipped, transposed
+// weights; reads [up2(a), b] in place), kWGrad (weight and bias gradient, split
+// over voxels), pooling, split of the decoder's gradient, ReLU mask, masked MSE,
+// Adam.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -43,10 +44,6 @@ constexpr int kLevel[kLayers] = {0, 1, 2, 3, 2, 1, 0, 0};
 constexpr int kRelu[kLayers] = {1, 1, 1, 1, 1, 1, 1, 0};
 
 typedef __nv_bfloat16 bf16;
-
-__device__ __forceinline__ uint32_t pack2(bf16 lo, bf16 hi) {
-    return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
-}
 
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
@@ -109,11 +106,12 @@ constexpr int HALO = 10;  // tile edge 8 and one voxel on each side
 template <int CK>
 __host__ __device__ constexpr int rowBytes() { return 32 * CK + 16; }
 
-// Copies the halo of the tile at (x0, y0, z0), TZ + 2 layers of 10 x 10 voxels, zeros outside the grid.
+// Copies 16 CK channels from c0 of the halo of the tile at (x0, y0, z0), TZ + 2 layers of 10 x 10
+// voxels, zeros outside the grid.
 template <int CK, int TZ, int NTH>
-__device__ __forceinline__ void stageHalo(uint32_t dst, const Input& in, int n, int x0, int y0, int z0) {
+__device__ __forceinline__ void stageHalo(uint32_t dst, const Input& in, int c0, int n, int x0, int y0, int z0) {
     constexpr int Q = 2 * CK, TOT = HALO * HALO * (TZ + 2) * Q;
-    const int C = 16 * CK, nh = n >> 1;
+    const int nh = n >> 1;
     for (int i = threadIdx.x; i < TOT; i += NTH) {
         const int q = i % Q, h = i / Q;
         const int hx = h % HALO, hy = (h / HALO) % HALO, hz = h / (HALO * HALO);
@@ -121,10 +119,9 @@ __device__ __forceinline__ void stageHalo(uint32_t dst, const Input& in, int n, 
         const bool ok = x >= 0 && x < n && y >= 0 && y < n && z >= 0 && z < n;
         const bf16* src = in.b;
         if (ok) {
-            if (8 * q < in.Ca)
-                src = in.a + ((((int64_t)(z >> 1) * nh + (y >> 1)) * nh + (x >> 1)) * in.Ca + 8 * q);
-            else
-                src = in.b + ((((int64_t)z * n + y) * n + x) * (C - in.Ca) + 8 * q - in.Ca);
+            const int c = c0 + 8 * q;
+            if (c < in.Ca) src = in.a + ((((int64_t)(z >> 1) * nh + (y >> 1)) * nh + (x >> 1)) * in.Ca + c);
+            else src = in.b + ((((int64_t)z * n + y) * n + x) * in.Cb + c - in.Ca);
         }
         cpAsync16(dst + (uint32_t)(h * rowBytes<CK>() + 16 * q), src, ok);
     }
@@ -164,7 +161,7 @@ __global__ void __launch_bounds__(64 * TZ) kConv(const Input in, const bf16* __r
     if (NS == 1) stageW(0, 0);
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int x0 = (tile % tx) * 8, y0 = (tile / tx) % tx * 8, z0 = tile / (tx * tx) * TZ;
-        stageHalo<CK, TZ, NTH>(sA, in, n, x0, y0, z0);
+        stageHalo<CK, TZ, NTH>(sA, in, 0, n, x0, y0, z0);
         if (NS > 1) stageW(0, 0);
         cpCommit();
         float acc[2][NT][4];
@@ -233,91 +230,136 @@ __global__ void __launch_bounds__(64 * TZ) kConv(const Input in, const bf16* __r
     }
 }
 
-// Weight gradient: dW[tap][ci][co] += sum_v in[v + off(tap)][ci] * g[v][co].
-// Grid (voxel chunks, taps, ci tiles x co tiles); block 128 threads computes a
-// 64(ci) x 64(co) tile over its voxel chunk in steps of 16 voxels and stores it
-// in the chunk's slice of part ([chunk][27][Cin][Cout]); kWGradSum then adds
-// the chunks to dW in a fixed order, so the gradient is bit-reproducible.
-constexpr int WG_CHUNK = 2048;
+// Weight and bias gradient: dW[tap][ci][co] = sum_v in[v + off(tap)][ci] g[v][co], db[co] = sum_v g[v][co].
+//
+// A block owns 16 MT x 8 NT (ci, co) of all 27 taps and walks 8 x 8 x 2 tiles
+// (blockIdx.x, + gridDim.x, ...): halo of the input and the tile of g, double-
+// buffered in shared memory.  Warp w = 3 dz + dy holds the three dx taps in
+// registers; a step is 16 voxels (two x rows) as the MMA's K, both operands by
+// transposing ldmatrix.  The bias is one more MMA against ones, in warp 4 of the
+// first ci block.  Each block writes its sums to a slice of part ([block][27 Cin
+// Cout weights, Cout biases], the parameters' layout); kGradSum adds the slices
+// in a fixed order, so the gradient is bit-reproducible.
+//
+// The earlier kernel (a block per 2,048 voxels, tap and 64 x 64 channels) staged
+// both operands for every tap, element by element for the transpose, and the
+// bias ran in one block per channel.  Measured on GB300 at 72^3, weights and
+// bias: 16 x 16 channels 855 -> 40 us, 48 x 16 1,024 -> 106 us, 96 x 32 (36^3) 297 -> 58 us.
+constexpr int WG_TZ = 2, WG_THREADS = 288;
 
-__global__ void __launch_bounds__(128) kConvWGrad(const bf16* __restrict__ in, const bf16* __restrict__ gout,
-                                                  float* __restrict__ part, int n, int Cin, int Cout) {
-    __shared__ __align__(16) bf16 sA[64][16 + 8];   // [ci][v]
-    __shared__ __align__(16) bf16 sB[16][64 + 8];   // [v][co]
+template <int MT, int NT>
+__host__ __device__ constexpr int wgStageBytes() { return HALO * HALO * (WG_TZ + 2) * rowBytes<MT>() + 64 * WG_TZ * (16 * NT + 16); }
+
+template <int MT, int NT>
+__global__ void __launch_bounds__(WG_THREADS) kWGrad(const Input in, const bf16* __restrict__ g,
+                                                     float* __restrict__ part, int n, int Cout) {
+    constexpr int ROW = rowBytes<MT>(), GROW = 16 * NT + 16, STAGE = wgStageBytes<MT, NT>();
+    constexpr uint32_t haloBytes = HALO * HALO * (WG_TZ + 2) * ROW;
+    extern __shared__ __align__(16) unsigned char wgSm[];
+    const uint32_t sm = (uint32_t)__cvta_generic_to_shared(wgSm);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t4 = lane & 3;
-    const int tap = blockIdx.y;
-    const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-    const int ciTiles = (Cin + 63) / 64;
-    const int ci0 = (blockIdx.z % ciTiles) * 64, co0 = (blockIdx.z / ciTiles) * 64;
-    const int mt = min(64, Cin - ci0), nt = min(64, Cout - co0);
-    const int64_t V = (int64_t)n * n * n;
-    const int64_t vb = (int64_t)blockIdx.x * WG_CHUNK;
-    const int64_t ve = min(V, vb + WG_CHUNK);
-    float acc[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    for (int64_t vs = vb; vs < ve; vs += 16) {
-        // A^T tile: 16 voxels x mt channels of the shifted input.
-        for (int i = tid; i < 16 * (mt / 8); i += 128) {
-            const int vv = i / (mt / 8), q = i % (mt / 8);
-            const int64_t v = vs + vv;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (v < ve) {
-                const int x = (int)(v % n) + dx, y = (int)((v / n) % n) + dy, z = (int)(v / ((int64_t)n * n)) + dz;
-                if (x >= 0 && x < n && y >= 0 && y < n && z >= 0 && z < n)
-                    val = *reinterpret_cast<const uint4*>(in + (((int64_t)z * n + y) * n + x) * Cin + ci0 + 8 * q);
-            }
-            const bf16* e = reinterpret_cast<const bf16*>(&val);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) sA[8 * q + u][vv] = e[u];
+    const int Cin = in.Ca + in.Cb, coParts = Cout / (8 * NT);
+    const int ci0 = (int)(blockIdx.y / coParts) * 16 * MT, co0 = (int)(blockIdx.y % coParts) * 8 * NT;
+    const int tx = (n + 7) >> 3, tiles = tx * tx * ((n + WG_TZ - 1) / WG_TZ);
+    auto stage = [&](int tile, int buf) {
+        const int x0 = (tile % tx) * 8, y0 = (tile / tx) % tx * 8, z0 = tile / (tx * tx) * WG_TZ;
+        stageHalo<MT, WG_TZ, WG_THREADS>(sm + buf * STAGE, in, ci0, n, x0, y0, z0);
+        for (int i = tid; i < 64 * WG_TZ * NT; i += WG_THREADS) {
+            const int q = i % NT, v = i / NT;
+            const int x = x0 + (v & 7), y = y0 + ((v >> 3) & 7), z = z0 + (v >> 6);
+            const bool ok = x < n && y < n && z < n;
+            cpAsync16(sm + buf * STAGE + haloBytes + v * GROW + 16 * q,
+                      ok ? g + (((int64_t)z * n + y) * n + x) * Cout + co0 + 8 * q : g, ok);
         }
-        for (int i = tid; i < 16 * (nt / 8); i += 128) {
-            const int vv = i / (nt / 8), q = i % (nt / 8);
-            const int64_t v = vs + vv;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (v < ve) val = *reinterpret_cast<const uint4*>(gout + v * Cout + co0 + 8 * q);
-            *reinterpret_cast<uint4*>(&sB[vv][8 * q]) = val;
+        cpCommit();
+    };
+    float acc[3][MT][NT][4], accB[NT][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            accB[j][e] = 0.f;
+#pragma unroll
+            for (int t = 0; t < 3; ++t)
+#pragma unroll
+                for (int m = 0; m < MT; ++m) acc[t][m][j][e] = 0.f;
+        }
+    const bool bias = warp == 4 && ci0 == 0;
+    const uint32_t aLane =
+        (uint32_t)((((warp / 3) * HALO + warp % 3 + (lane >> 4)) * HALO + (lane & 7)) * ROW + 16 * ((lane >> 3) & 1));
+    const uint32_t bLane = haloBytes + (uint32_t)(((lane & 7) + 8 * ((lane >> 3) & 1)) * GROW + 16 * (lane >> 4));
+    int buf = 0;
+    if ((int)blockIdx.x < tiles) stage(blockIdx.x, 0);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, buf ^= 1) {
+        if (tile + (int)gridDim.x < tiles) {
+            stage(tile + gridDim.x, buf ^ 1);
+            cpWait<1>();
+        } else {
+            cpWait<0>();
         }
         __syncthreads();
-        const int rb = warp * 16;
-        if (rb < mt) {
-            const uint32_t a0 = pack2(sA[rb + g][2 * t4], sA[rb + g][2 * t4 + 1]);
-            const uint32_t a1 = pack2(sA[rb + g + 8][2 * t4], sA[rb + g + 8][2 * t4 + 1]);
-            const uint32_t a2 = pack2(sA[rb + g][2 * t4 + 8], sA[rb + g][2 * t4 + 9]);
-            const uint32_t a3 = pack2(sA[rb + g + 8][2 * t4 + 8], sA[rb + g + 8][2 * t4 + 9]);
+        const uint32_t base = sm + buf * STAGE;
+#pragma unroll 2
+        for (int k = 0; k < 4 * WG_TZ; ++k) {  // 16 voxels: rows 2 (k & 3) and the next of layer k >> 2
+            uint32_t B[NT / 2][4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (8 * j >= nt) break;
-                const uint32_t b0 = pack2(sB[2 * t4][8 * j + g], sB[2 * t4 + 1][8 * j + g]);
-                const uint32_t b1 = pack2(sB[2 * t4 + 8][8 * j + g], sB[2 * t4 + 9][8 * j + g]);
-                mma16816(acc[j], a0, a1, a2, a3, b0, b1);
+            for (int j = 0; j < NT / 2; ++j) ldsm4t(B[j], base + bLane + k * 16 * GROW + 32 * j);
+            const uint32_t ak = base + aLane + (uint32_t)(((k >> 2) * HALO + 2 * (k & 3)) * HALO * ROW);
+#pragma unroll
+            for (int t = 0; t < 3; ++t)
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    uint32_t A[4];
+                    ldsm4t(A, ak + t * ROW + 32 * m);
+#pragma unroll
+                    for (int j = 0; j < NT; ++j)
+                        mma16816(acc[t][m][j], A[0], A[1], A[2], A[3], B[j >> 1][2 * (j & 1)], B[j >> 1][2 * (j & 1) + 1]);
+                }
+            if (bias) {
+                constexpr uint32_t one = 0x3f803f80u;
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+                    mma16816(accB[j], one, one, one, one, B[j >> 1][2 * (j & 1)], B[j >> 1][2 * (j & 1) + 1]);
             }
         }
         __syncthreads();
     }
-    const int rb = warp * 16;
-    if (rb >= mt) return;
+    const int64_t per = 27LL * Cin * Cout + Cout;
+    float* d = part + blockIdx.x * per;
+    const int r = lane >> 2, t4 = lane & 3;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        if (8 * j >= nt) break;
+    for (int j = 0; j < NT; ++j) {
+        const int co = co0 + 8 * j + 2 * t4;
 #pragma unroll
-        for (int hrow = 0; hrow < 2; ++hrow) {
-            const int ci = ci0 + rb + g + 8 * hrow;
-            const int co = co0 + 8 * j + 2 * t4;
-            float* d = part + (int64_t)blockIdx.x * 27 * Cin * Cout + ((int64_t)tap * Cin + ci) * Cout + co;
-            d[0] = acc[j][2 * hrow];
-            d[1] = acc[j][2 * hrow + 1];
-        }
+        for (int t = 0; t < 3; ++t)
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    *reinterpret_cast<float2*>(d + ((int64_t)(3 * warp + t) * Cin + ci0 + 16 * m + r + 8 * h) * Cout + co) =
+                        make_float2(acc[t][m][j][2 * h], acc[t][m][j][2 * h + 1]);
+        if (bias && r == 0) *reinterpret_cast<float2*>(d + 27LL * Cin * Cout + co) = make_float2(accB[j][0], accB[j][1]);
     }
 }
 
-// dW[e] += sum over chunks c (in order) of part[c][e], e < per (= 27 Cin Cout).
-__global__ void kWGradSum(const float* __restrict__ part, float* __restrict__ dW, int64_t per, int chunks) {
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < per; e += (int64_t)gridDim.x * blockDim.x) {
-        float sum = 0.f;
-        for (int c = 0; c < chunks; ++c) sum += part[(int64_t)c * per + e];
-        dW[e] += sum;
+// dW[e] += sum over the slices of part, eight interleaved partial sums in a fixed order.
+__global__ void __launch_bounds__(256) kGradSum(const float* __restrict__ part, float* __restrict__ dW, int64_t per,
+                                                int slices) {
+    __shared__ float red[8][32];
+    const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+    const int64_t e = blockIdx.x * 32LL + lane;
+    float sum = 0.f;
+    if (e < per) {
+#pragma unroll 4
+        for (int c = grp; c < slices; c += 8) sum += part[(int64_t)c * per + e];
+    }
+    red[grp][lane] = sum;
+    __syncthreads();
+    if (grp == 0 && e < per) {
+        float t = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) t += red[q][lane];
+        dW[e] += t;
     }
 }
 
@@ -353,24 +395,7 @@ __global__ void kPoolBwd(const float* __restrict__ gout, float* __restrict__ gin
     }
 }
 
-// Decoder input: channels [0, Ca) = nearest upsampling of a (at n/2), [Ca, Ca+Cb) = skip b.
-__global__ void kUpConcat(const bf16* __restrict__ a, const bf16* __restrict__ b, bf16* __restrict__ out, int nf,
-                          int Ca, int Cb) {
-    const int C = Ca + Cb, nc = nf / 2;
-    const int64_t total = (int64_t)nf * nf * nf * C;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
-        const int64_t v = i / C;
-        if (c < Ca) {
-            const int x = (int)(v % nf) / 2, y = (int)((v / nf) % nf) / 2, z = (int)(v / ((int64_t)nf * nf)) / 2;
-            out[i] = a[(((int64_t)z * nc + y) * nc + x) * Ca + c];
-        } else {
-            out[i] = b[v * Cb + (c - Ca)];
-        }
-    }
-}
-
-// Backward of kUpConcat: ga (at n/2) = sum of the 8 children's first Ca channels,
+// Backward of the decoder's concatenated input: ga (at n/2) = sum of the 8 children's first Ca channels,
 // gb (skip) = the remaining channels (added to an existing gradient).
 __global__ void kUpConcatBwd(const float* __restrict__ g, float* __restrict__ ga, float* __restrict__ gb, int nf,
                              int Ca, int Cb) {
@@ -404,21 +429,6 @@ __global__ void kReluMask(const float* __restrict__ g, const bf16* __restrict__ 
                           int relu) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = __float2bfloat16((!relu || __bfloat162float(y[i]) > 0.f) ? g[i] : 0.f);
-}
-
-__global__ void kBiasGrad(const bf16* __restrict__ g, float* __restrict__ db, int64_t V, int C) {
-    // One block per channel group of 32 channels; threads stride over voxels.
-    __shared__ float s[256];
-    const int c = blockIdx.x;
-    float acc = 0.f;
-    for (int64_t v = threadIdx.x; v < V; v += blockDim.x) acc += __bfloat162float(g[v * C + c]);
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) db[c] += s[0];
 }
 
 // Masked MSE on channels 0..2 of y (C channels): loss = sum m (y - t)^2 / count;
@@ -498,13 +508,12 @@ struct vfem_net {
     bf16 *wb[kLayers] = {}, *wt[kLayers] = {};
     int64_t step = 0;
     // activations (bf16) and gradients (f32)
-    bf16 *x = nullptr, *e[4] = {}, *p[4] = {}, *c[3] = {}, *d[3] = {};
+    bf16 *x = nullptr, *e[4] = {}, *p[4] = {}, *d[3] = {};
     float* y = nullptr;
     float *t = nullptr, *mask = nullptr, *gy = nullptr;
     float *ge[4] = {}, *gp[4] = {}, *gc[3] = {}, *gd[3] = {};
     bf16* gmask = nullptr;  // masked gradient scratch (largest layer)
-    bf16* gbf = nullptr;    // bf16 copy of an input gradient (largest)
-    float* wgPart = nullptr;  // per-chunk weight-gradient tiles (largest layer)
+    float* wgPart = nullptr;  // per-block weight and bias gradients (largest layer)
     double* part = nullptr;
     float* hostStage = nullptr;
 };
@@ -617,49 +626,67 @@ void forward(vfem_net* N) {
     conv<true>(N, layerInput(N, 7), N->wb[7], N->w + N->boff[7], N->y, 0, 16, 0);
 }
 
-// Backward of one convolution: given dL/d(out) in gout (f32, [V][Cout]) and the
-// layer's output (for the relu mask), accumulate dW, db, and write dL/d(in) (f32)
-// into gin (overwrite).
-void convBwd(vfem_net* N, int l, const bf16* in, const bf16* out, const float* gout, float* gin, bool wantIn) {
+// Spatial blocks of layer l's weight gradient: one block per SM over its (ci, co) parts, at most one a tile.
+constexpr int wgM(int cin) { return cin == 48 ? 3 : cin >= 32 ? 2 : 1; }   // 16-channel ci tiles of a block
+constexpr int wgN(int cout) { return cout >= 32 ? 4 : 2; }                 // 8-channel co tiles
+int wgSlices(int n, int cin, int cout) {
+    const int tx = (n + 7) / 8, tiles = tx * tx * ((n + WG_TZ - 1) / WG_TZ);
+    const int parts = cin / (16 * wgM(cin)) * (cout / (8 * wgN(cout)));
+    const int perSm = wgM(cin) * wgN(cout) <= 4 ? 2 : 1;  // by registers: 24 to 96 accumulators a thread
+    return std::max(1, std::min(tiles, 152 * perSm / parts));
+}
+
+template <int MT, int NT>
+void launchWGrad(vfem_net* N, const Input& in, const bf16* g, int n, int Cout, int slices) {
+    constexpr size_t smem = 2 * (size_t)wgStageBytes<MT, NT>();
+    static const cudaError_t attr = cudaFuncSetAttribute(kWGrad<MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)smem);
+    (void)attr;
+    const dim3 grid((unsigned)slices, (unsigned)((in.Ca + in.Cb) / (16 * MT) * (Cout / (8 * NT))));
+    kWGrad<MT, NT><<<grid, WG_THREADS, smem, N->stream>>>(in, g, N->wgPart, n, Cout);
+}
+
+// Backward of convolution l: given dL/d(out) in gout (f32, [V][Cout]) and the
+// layer's output (for the relu mask), accumulate dW and db, and write dL/d(in)
+// (f32) into gin if wanted (overwrite).
+void convBwd(vfem_net* N, int l, const bf16* out, const float* gout, float* gin) {
     const int lvl = kLevel[l], Cin = kCin[l], Cout = kCout[l];
     const int n = N->n >> lvl;
-    const int64_t V = N->V[lvl];
+    const int64_t V = N->V[lvl], per = 27LL * Cin * Cout + Cout;
     kReluMask<<<blocks(V * Cout), 256, 0, N->stream>>>(gout, out, N->gmask, V * Cout, kRelu[l]);
-    kBiasGrad<<<Cout, 256, 0, N->stream>>>(N->gmask, N->gw + N->boff[l], V, Cout);
-    const int chunks = (int)((V + WG_CHUNK - 1) / WG_CHUNK);
-    dim3 gw((unsigned)chunks, 27, (unsigned)(((Cin + 63) / 64) * ((Cout + 63) / 64)));
-    kConvWGrad<<<gw, 128, 0, N->stream>>>(in, N->gmask, N->wgPart, n, Cin, Cout);
-    const int64_t per = 27LL * Cin * Cout;
-    kWGradSum<<<blocks(per), 256, 0, N->stream>>>(N->wgPart, N->gw + N->woff[l], per, chunks);
-    if (wantIn) conv<true>(N, Input{nullptr, N->gmask, 0, Cout}, N->wt[l], nullptr, gin, lvl, Cin, 0);
+    const Input in = layerInput(N, l);
+    const int slices = wgSlices(n, Cin, Cout);
+    if (Cin == 48) launchWGrad<3, 2>(N, in, N->gmask, n, Cout, slices);
+    else if (Cin == 16 && Cout == 16) launchWGrad<1, 2>(N, in, N->gmask, n, Cout, slices);
+    else if (Cin == 16) launchWGrad<1, 4>(N, in, N->gmask, n, Cout, slices);
+    else launchWGrad<2, 4>(N, in, N->gmask, n, Cout, slices);
+    kGradSum<<<(unsigned)((per + 31) / 32), 256, 0, N->stream>>>(N->wgPart, N->gw + N->woff[l], per, slices);
+    if (gin) conv<true>(N, Input{nullptr, N->gmask, 0, Cout}, N->wt[l], nullptr, gin, lvl, Cin, 0);
 }
 
 void backward(vfem_net* N) {
     const int64_t* V = N->V;
-    kUpConcat<<<blocks(V[2] * 192), 256, 0, N->stream>>>(N->e[3], N->e[2], N->c[2], N->n / 4, 128, 64);
-    kUpConcat<<<blocks(V[1] * 96), 256, 0, N->stream>>>(N->d[2], N->e[1], N->c[1], N->n / 2, 64, 32);
-    kUpConcat<<<blocks(V[0] * 48), 256, 0, N->stream>>>(N->d[1], N->e[0], N->c[0], N->n, 32, 16);
     // y = conv7(d0)
-    convBwd(N, 7, N->d[0], nullptr, N->gy, N->gd[0], true);
+    convBwd(N, 7, nullptr, N->gy, N->gd[0]);
     // d0 = relu(conv6(c0))
-    convBwd(N, 6, N->c[0], N->d[0], N->gd[0], N->gc[0], true);
+    convBwd(N, 6, N->d[0], N->gd[0], N->gc[0]);
     // c0 = [up(d1), e0]
     cudaMemsetAsync(N->ge[0], 0, sizeof(float) * V[0] * 16, N->stream);
     kUpConcatBwd<<<blocks(V[1] * 32 + V[0] * 16), 256, 0, N->stream>>>(N->gc[0], N->gd[1], N->ge[0], N->n, 32, 16);
-    convBwd(N, 5, N->c[1], N->d[1], N->gd[1], N->gc[1], true);
+    convBwd(N, 5, N->d[1], N->gd[1], N->gc[1]);
     cudaMemsetAsync(N->ge[1], 0, sizeof(float) * V[1] * 32, N->stream);
     kUpConcatBwd<<<blocks(V[2] * 64 + V[1] * 32), 256, 0, N->stream>>>(N->gc[1], N->gd[2], N->ge[1], N->n / 2, 64, 32);
-    convBwd(N, 4, N->c[2], N->d[2], N->gd[2], N->gc[2], true);
+    convBwd(N, 4, N->d[2], N->gd[2], N->gc[2]);
     cudaMemsetAsync(N->ge[2], 0, sizeof(float) * V[2] * 64, N->stream);
     kUpConcatBwd<<<blocks(V[3] * 128 + V[2] * 64), 256, 0, N->stream>>>(N->gc[2], N->ge[3], N->ge[2], N->n / 4, 128, 64);
     // e3 = relu(conv3(p3)); p3 = pool(e2)
-    convBwd(N, 3, N->p[3], N->e[3], N->ge[3], N->gp[3], true);
+    convBwd(N, 3, N->e[3], N->ge[3], N->gp[3]);
     kPoolBwd<<<blocks(V[2] * 64), 256, 0, N->stream>>>(N->gp[3], N->ge[2], N->n / 8, 64, 1);
-    convBwd(N, 2, N->p[2], N->e[2], N->ge[2], N->gp[2], true);
+    convBwd(N, 2, N->e[2], N->ge[2], N->gp[2]);
     kPoolBwd<<<blocks(V[1] * 32), 256, 0, N->stream>>>(N->gp[2], N->ge[1], N->n / 4, 32, 1);
-    convBwd(N, 1, N->p[1], N->e[1], N->ge[1], N->gp[1], true);
+    convBwd(N, 1, N->e[1], N->ge[1], N->gp[1]);
     kPoolBwd<<<blocks(V[0] * 16), 256, 0, N->stream>>>(N->gp[1], N->ge[0], N->n / 2, 16, 1);
-    convBwd(N, 0, N->x, N->e[0], N->ge[0], nullptr, false);
+    convBwd(N, 0, N->e[0], N->ge[0], nullptr);
 }
 
 }  // namespace
@@ -711,7 +738,6 @@ vfem_status vfem_net_create(int32_t n, vfem_net** out) {
     }
     const int cc[3] = {48, 96, 192}, dc[3] = {16, 32, 64};
     for (int l = 0; l < 3; ++l) {
-        NA(nalloc(&N->c[l], V[l] * cc[l]));
         NA(nalloc(&N->gc[l], V[l] * cc[l]));
         NA(nalloc(&N->d[l], V[l] * dc[l]));
         NA(nalloc(&N->gd[l], V[l] * dc[l]));
@@ -723,10 +749,9 @@ vfem_status vfem_net_create(int32_t n, vfem_net** out) {
     int64_t gmax = 0;
     for (int l = 0; l < kLayers; ++l) gmax = std::max<int64_t>(gmax, V[kLevel[l]] * std::max(kCin[l], kCout[l]));
     NA(nalloc(&N->gmask, gmax));
-    NA(nalloc(&N->gbf, gmax));
     int64_t wmax = 0;
     for (int l = 0; l < kLayers; ++l)
-        wmax = std::max<int64_t>(wmax, (V[kLevel[l]] + WG_CHUNK - 1) / WG_CHUNK * 27 * kCin[l] * kCout[l]);
+        wmax = std::max<int64_t>(wmax, wgSlices(n >> kLevel[l], kCin[l], kCout[l]) * (27LL * kCin[l] * kCout[l] + kCout[l]));
     NA(nalloc(&N->wgPart, wmax));
     NA(nalloc(&N->part, 4096));
     NA(cudaMallocHost((void**)&N->hostStage, sizeof(float) * V[0] * 16));
@@ -741,8 +766,8 @@ void vfem_net_destroy(vfem_net* N) {
     for (int l = 0; l < kLayers; ++l) { cudaFree(N->wb[l]); cudaFree(N->wt[l]); }
     cudaFree(N->x);
     for (int l = 0; l < 4; ++l) { cudaFree(N->e[l]); cudaFree(N->ge[l]); cudaFree(N->p[l]); cudaFree(N->gp[l]); }
-    for (int l = 0; l < 3; ++l) { cudaFree(N->c[l]); cudaFree(N->gc[l]); cudaFree(N->d[l]); cudaFree(N->gd[l]); }
-    cudaFree(N->y); cudaFree(N->gy); cudaFree(N->t); cudaFree(N->mask); cudaFree(N->gmask); cudaFree(N->gbf);
+    for (int l = 0; l < 3; ++l) { cudaFree(N->gc[l]); cudaFree(N->d[l]); cudaFree(N->gd[l]); }
+    cudaFree(N->y); cudaFree(N->gy); cudaFree(N->t); cudaFree(N->mask); cudaFree(N->gmask);
     cudaFree(N->part); cudaFree(N->wgPart);
     if (N->hostStage) cudaFreeHost(N->hostStage);
     if (N->stream) cudaStreamDestroy(N->stream);
