@@ -28,6 +28,7 @@
 #include <cstdint>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "vfem_net.h"
@@ -106,10 +107,9 @@ constexpr int HALO = 10;  // tile edge 8 and one voxel on each side
 template <int CK>
 __host__ __device__ constexpr int rowBytes() { return 32 * CK + 16; }
 
-// Copies 16 CK channels from c0 of the halo of the tile at (x0, y0, z0), TZ + 2 layers of 10 x 10
-// voxels, zeros outside the grid.
+// Copies the halo of the tile at (x0, y0, z0), TZ + 2 layers of 10 x 10 voxels, zeros outside the grid.
 template <int CK, int TZ, int NTH>
-__device__ __forceinline__ void stageHalo(uint32_t dst, const Input& in, int c0, int n, int x0, int y0, int z0) {
+__device__ __forceinline__ void stageHalo(uint32_t dst, const Input& in, int n, int x0, int y0, int z0) {
     constexpr int Q = 2 * CK, TOT = HALO * HALO * (TZ + 2) * Q;
     const int nh = n >> 1;
     for (int i = threadIdx.x; i < TOT; i += NTH) {
@@ -119,7 +119,7 @@ __device__ __forceinline__ void stageHalo(uint32_t dst, const Input& in, int c0,
         const bool ok = x >= 0 && x < n && y >= 0 && y < n && z >= 0 && z < n;
         const bf16* src = in.b;
         if (ok) {
-            const int c = c0 + 8 * q;
+            const int c = 8 * q;
             if (c < in.Ca) src = in.a + ((((int64_t)(z >> 1) * nh + (y >> 1)) * nh + (x >> 1)) * in.Ca + c);
             else src = in.b + ((((int64_t)z * n + y) * n + x) * in.Cb + c - in.Ca);
         }
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(64 * TZ) kConv(const Input in, const bf16* __r
     if (NS == 1) stageW(0, 0);
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int x0 = (tile % tx) * 8, y0 = (tile / tx) % tx * 8, z0 = tile / (tx * tx) * TZ;
-        stageHalo<CK, TZ, NTH>(sA, in, 0, n, x0, y0, z0);
+        stageHalo<CK, TZ, NTH>(sA, in, n, x0, y0, z0);
         if (NS > 1) stageW(0, 0);
         cpCommit();
         float acc[2][NT][4];
@@ -232,44 +232,95 @@ __global__ void __launch_bounds__(64 * TZ) kConv(const Input in, const bf16* __r
 
 // Weight and bias gradient: dW[tap][ci][co] = sum_v in[v + off(tap)][ci] g[v][co], db[co] = sum_v g[v][co].
 //
-// A block owns 16 MT x 8 NT (ci, co) of all 27 taps and walks 8 x 8 x 2 tiles
-// (blockIdx.x, + gridDim.x, ...): halo of the input and the tile of g, double-
-// buffered in shared memory.  Warp w = 3 dz + dy holds the three dx taps in
-// registers; a step is 16 voxels (two x rows) as the MMA's K, both operands by
-// transposing ldmatrix.  The bias is one more MMA against ones, in warp 4 of the
-// first ci block.  Each block writes its sums to a slice of part ([block][27 Cin
-// Cout weights, Cout biases], the parameters' layout); kGradSum adds the slices
-// in a fixed order, so the gradient is bit-reproducible.
+// A warp owns 16 MT x 8 NT (ci, co) of the three dx taps of one (dy, dz) over
+// WG_CHUNK consecutive voxels, WG_SUB at a time; a block is the three dy of one dz
+// (blockIdx.z).  With voxels in storage order a tap is a shift by dx + n dy +
+// n^2 dz, so a warp stages a run of WG_SUB + 2 input voxels and WG_SUB of g for
+// itself, in a ring of WG_BUFS buffers, and needs no block barrier.  A step is 16 voxels as the MMA's
+// K, both operands by transposing ldmatrix, whose per-row addresses send a voxel
+// without that neighbour to a row of zeros.  The bias is one more MMA against
+// ones, in the (0, 0) warp of the first ci block.  The chunk's sums go to its
+// slice of part ([chunk][27 Cin Cout weights, Cout biases], the parameters'
+// layout) and kGradSum adds the slices in order: the order of the sums depends
+// on the voxel numbering alone, so the gradient is bit-reproducible.
 //
-// The earlier kernel (a block per 2,048 voxels, tap and 64 x 64 channels) staged
-// both operands for every tap, element by element for the transpose, and the
-// bias ran in one block per channel.  Measured on GB300 at 72^3, weights and
-// bias: 16 x 16 channels 855 -> 40 us, 48 x 16 1,024 -> 106 us, 96 x 32 (36^3) 297 -> 58 us.
-constexpr int WG_TZ = 2, WG_THREADS = 288;
+// The earlier kernel staged both operands for every tap, element by element for
+// the transpose, and the bias ran in one block per channel.  Measured on GB300 at
+// 72^3, weights and bias: 16 x 16 channels 855 -> 64 us, 48 x 16 1,024 -> 104 us,
+// 96 x 32 (36^3) 297 -> 75 us; the weights with the same bits.  8 x 8 x 2 tiles
+// with a halo instead of runs (40, 106 and 58 us) change the order of the sums: a
+// weight whose gradient nearly cancels then takes another first Adam step.
+// Bound: the serial chain of 128 steps of a warp, few warps where a level is small.
+constexpr int WG_CHUNK = 2048, WG_SUB = 32, WG_BUFS = 3, WG_THREADS = 96;  // 2 buffers: 5% slower, 4: 48 x 16 60%
+
+// v / n for 0 <= v < 2^31 and n <= 512: mul = ceil(2^40 / n)
+__device__ __forceinline__ int divBy(int v, unsigned long long mul) {
+    return (int)(((unsigned long long)(unsigned)v * mul) >> 40);
+}
 
 template <int MT, int NT>
-__host__ __device__ constexpr int wgStageBytes() { return HALO * HALO * (WG_TZ + 2) * rowBytes<MT>() + 64 * WG_TZ * (16 * NT + 16); }
+__host__ __device__ constexpr int wgBufBytes() { return (WG_SUB + 2) * rowBytes<MT>() + WG_SUB * (16 * NT + 16); }
+template <int MT, int NT>
+__host__ __device__ constexpr int wgSmem() { return rowBytes<MT>() + 3 * WG_BUFS * wgBufBytes<MT, NT>(); }
 
 template <int MT, int NT>
 __global__ void __launch_bounds__(WG_THREADS) kWGrad(const Input in, const bf16* __restrict__ g,
-                                                     float* __restrict__ part, int n, int Cout) {
-    constexpr int ROW = rowBytes<MT>(), GROW = 16 * NT + 16, STAGE = wgStageBytes<MT, NT>();
-    constexpr uint32_t haloBytes = HALO * HALO * (WG_TZ + 2) * ROW;
+                                                     float* __restrict__ part, int n, unsigned long long mul, int Cout) {
+    constexpr int ROW = rowBytes<MT>(), GROW = 16 * NT + 16, Q = 2 * MT, BUF = wgBufBytes<MT, NT>();
+    constexpr uint32_t gOff = (WG_SUB + 2) * ROW;
     extern __shared__ __align__(16) unsigned char wgSm[];
     const uint32_t sm = (uint32_t)__cvta_generic_to_shared(wgSm);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31, dy = tid >> 5, dz = blockIdx.z, warp = 3 * dz + dy;
     const int Cin = in.Ca + in.Cb, coParts = Cout / (8 * NT);
     const int ci0 = (int)(blockIdx.y / coParts) * 16 * MT, co0 = (int)(blockIdx.y % coParts) * 8 * NT;
-    const int tx = (n + 7) >> 3, tiles = tx * tx * ((n + WG_TZ - 1) / WG_TZ);
-    auto stage = [&](int tile, int buf) {
-        const int x0 = (tile % tx) * 8, y0 = (tile / tx) % tx * 8, z0 = tile / (tx * tx) * WG_TZ;
-        stageHalo<MT, WG_TZ, WG_THREADS>(sm + buf * STAGE, in, ci0, n, x0, y0, z0);
-        for (int i = tid; i < 64 * WG_TZ * NT; i += WG_THREADS) {
-            const int q = i % NT, v = i / NT;
-            const int x = x0 + (v & 7), y = y0 + ((v >> 3) & 7), z = z0 + (v >> 6);
-            const bool ok = x < n && y < n && z < n;
-            cpAsync16(sm + buf * STAGE + haloBytes + v * GROW + 16 * q,
-                      ok ? g + (((int64_t)z * n + y) * n + x) * Cout + co0 + 8 * q : g, ok);
+    const int V = n * n * n, vb = blockIdx.x * WG_CHUNK, ve = min(V, vb + WG_CHUNK), nh = n >> 1;
+    for (int i = tid; i < ROW / 4; i += WG_THREADS) reinterpret_cast<uint32_t*>(wgSm)[i] = 0u;
+    __syncthreads();
+    const uint32_t mine = sm + ROW + dy * WG_BUFS * BUF;
+    const int shift = n * (dy - 1) + n * n * (dz - 1) - 1;  // first voxel of the staged run, from the first of g
+    // Pieces of 8 channels: `count` of them a voxel from channel c of a tensor with C channels, to
+    // byte `at` of each row.  row(r, src): the tensor's row of run voxel r (src = its number on the grid).
+    auto stagePieces = [&](auto count, uint32_t to, int first, const bf16* t, int C, int c, int at, auto row) {
+        constexpr int P = decltype(count)::value, PER = 32 / P;
+        const int r0 = lane / P, q = lane % P;
+#pragma unroll
+        for (int j = 0; j < (WG_SUB + 2 + PER - 1) / PER; ++j) {
+            const int r = r0 + j * PER, src = first + r, tr = row(r, src);  // row() shuffles: all lanes
+            if (r < WG_SUB + 2) {
+                const bool ok = (unsigned)src < (unsigned)V;
+                cpAsync16(to + r * ROW + at + 16 * q, ok ? t + (tr * (int64_t)C + c + 8 * q) : t, ok);
+            }
+        }
+    };
+    auto same = [](int, int src) { return src; };
+    auto stage = [&](int v0, uint32_t to) {
+        const int first = v0 + shift;
+        if (ci0 < in.Ca) {
+            // rows of the half-resolution tensor: one lane a voxel, two for lanes 0 and 1
+            auto half = [&](int src) {
+                const int yz = divBy(max(src, 0), mul), z = divBy(yz, mul), x = src - yz * n, y = yz - z * n;
+                return ((z >> 1) * nh + (y >> 1)) * nh + (x >> 1);
+            };
+            const int h0 = half(first + lane), h1 = half(first + 32 + (lane & 1));
+            auto up = [&](int r, int) {
+                const int a0 = __shfl_sync(0xffffffffu, h0, r & 31), a1 = __shfl_sync(0xffffffffu, h1, r & 1);
+                return r < 32 ? a0 : a1;
+            };
+            if constexpr (MT == 3) {
+                stagePieces(std::integral_constant<int, 4>(), to, first, in.a, in.Ca, ci0, 0, up);
+                stagePieces(std::integral_constant<int, 2>(), to, first, in.b, in.Cb, 0, 64, same);
+            } else {
+                stagePieces(std::integral_constant<int, Q == 6 ? 2 : Q>(), to, first, in.a, in.Ca, ci0, 0, up);
+            }
+        } else {
+            stagePieces(std::integral_constant<int, Q == 6 ? 2 : Q>(), to, first, in.b, in.Cb, ci0 - in.Ca, 0, same);
+        }
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            const int r = lane / NT + j * (32 / NT), v = v0 + r;
+            const bool ok = v < ve;
+            cpAsync16(to + gOff + r * GROW + 16 * (lane % NT),
+                      ok ? g + (v * (int64_t)Cout + co0 + 8 * (lane % NT)) : g, ok);
         }
         cpCommit();
     };
@@ -285,44 +336,63 @@ __global__ void __launch_bounds__(WG_THREADS) kWGrad(const Input in, const bf16*
                 for (int m = 0; m < MT; ++m) acc[t][m][j][e] = 0.f;
         }
     const bool bias = warp == 4 && ci0 == 0;
-    const uint32_t aLane =
-        (uint32_t)((((warp / 3) * HALO + warp % 3 + (lane >> 4)) * HALO + (lane & 7)) * ROW + 16 * ((lane >> 3) & 1));
-    const uint32_t bLane = haloBytes + (uint32_t)(((lane & 7) + 8 * ((lane >> 3) & 1)) * GROW + 16 * (lane >> 4));
-    int buf = 0;
-    if ((int)blockIdx.x < tiles) stage(blockIdx.x, 0);
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, buf ^= 1) {
-        if (tile + (int)gridDim.x < tiles) {
-            stage(tile + gridDim.x, buf ^ 1);
-            cpWait<1>();
-        } else {
-            cpWait<0>();
-        }
-        __syncthreads();
-        const uint32_t base = sm + buf * STAGE;
-#pragma unroll 2
-        for (int k = 0; k < 4 * WG_TZ; ++k) {  // 16 voxels: rows 2 (k & 3) and the next of layer k >> 2
+    const int lv = (lane & 7) + 8 * (lane >> 4);  // this lane's voxel row of A in a step
+    const uint32_t aHalf = 16 * ((lane >> 3) & 1), aZero = sm + aHalf;
+    const uint32_t bLane = gOff + (uint32_t)(((lane & 7) + 8 * ((lane >> 3) & 1)) * GROW + 16 * (lane >> 4));
+    // runs past the chunk's end are staged too (g as zeros, never used): a group per run keeps the count
+#pragma unroll
+    for (int i = 0; i < WG_BUFS - 1; ++i) stage(vb + i * WG_SUB, mine + i * BUF);
+    uint32_t cur = 0, put = (WG_BUFS - 1) * BUF;
+    int x, y, z;  // of this lane's voxel in the step
+    {
+        const int yz = divBy(vb + lv, mul);
+        z = divBy(yz, mul);
+        x = vb + lv - yz * n;
+        y = yz - z * n;
+    }
+    for (int v0 = vb; v0 < ve; v0 += WG_SUB) {
+        stage(v0 + (WG_BUFS - 1) * WG_SUB, mine + put);
+        cpWait<WG_BUFS - 1>();
+        __syncwarp();
+        const uint32_t base = mine + cur;
+        const int steps = (min(WG_SUB, ve - v0) + 15) >> 4;
+#pragma unroll
+        for (int k = 0; k < WG_SUB / 16; ++k) {
+            if (k >= steps) break;
             uint32_t B[NT / 2][4];
 #pragma unroll
             for (int j = 0; j < NT / 2; ++j) ldsm4t(B[j], base + bLane + k * 16 * GROW + 32 * j);
-            const uint32_t ak = base + aLane + (uint32_t)(((k >> 2) * HALO + 2 * (k & 3)) * HALO * ROW);
+            const bool row = v0 + 16 * k + lv < ve && (unsigned)(y + dy - 1) < (unsigned)n && (unsigned)(z + dz - 1) < (unsigned)n;
+            const uint32_t ak = base + (uint32_t)((16 * k + lv) * ROW) + aHalf;
 #pragma unroll
-            for (int t = 0; t < 3; ++t)
+            for (int t = 0; t < 3; ++t) {
+                const uint32_t at = row && (unsigned)(x + t - 1) < (unsigned)n ? ak + t * ROW : aZero;
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
                     uint32_t A[4];
-                    ldsm4t(A, ak + t * ROW + 32 * m);
+                    ldsm4t(A, at + 32 * m);
 #pragma unroll
                     for (int j = 0; j < NT; ++j)
                         mma16816(acc[t][m][j], A[0], A[1], A[2], A[3], B[j >> 1][2 * (j & 1)], B[j >> 1][2 * (j & 1) + 1]);
                 }
+            }
             if (bias) {
                 constexpr uint32_t one = 0x3f803f80u;
 #pragma unroll
                 for (int j = 0; j < NT; ++j)
                     mma16816(accB[j], one, one, one, one, B[j >> 1][2 * (j & 1)], B[j >> 1][2 * (j & 1) + 1]);
             }
+            for (x += 16; x >= n;) {
+                x -= n;
+                if (++y == n) {
+                    y = 0;
+                    ++z;
+                }
+            }
         }
-        __syncthreads();
+        __syncwarp();  // every lane has read this buffer before a later stage fills it
+        cur = cur + BUF == WG_BUFS * BUF ? 0 : cur + BUF;
+        put = put + BUF == WG_BUFS * BUF ? 0 : put + BUF;
     }
     const int64_t per = 27LL * Cin * Cout + Cout;
     float* d = part + blockIdx.x * per;
@@ -342,25 +412,22 @@ __global__ void __launch_bounds__(WG_THREADS) kWGrad(const Input in, const bf16*
     }
 }
 
-// dW[e] += sum over the slices of part, eight interleaved partial sums in a fixed order.
-__global__ void __launch_bounds__(256) kGradSum(const float* __restrict__ part, float* __restrict__ dW, int64_t per,
-                                                int slices) {
-    __shared__ float red[8][32];
-    const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
-    const int64_t e = blockIdx.x * 32LL + lane;
+// dW[e] += sum over the slices of part, in order (16 loads in flight, then their additions).
+__global__ void __launch_bounds__(64) kGradSum(const float* __restrict__ part, float* __restrict__ dW, int64_t per,
+                                               int slices) {
+    const int64_t e = blockIdx.x * 64LL + threadIdx.x;
+    if (e >= per) return;
     float sum = 0.f;
-    if (e < per) {
-#pragma unroll 4
-        for (int c = grp; c < slices; c += 8) sum += part[(int64_t)c * per + e];
-    }
-    red[grp][lane] = sum;
-    __syncthreads();
-    if (grp == 0 && e < per) {
-        float t = 0.f;
+    int c = 0;
+    for (; c + 16 <= slices; c += 16) {
+        float v[16];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) t += red[q][lane];
-        dW[e] += t;
+        for (int q = 0; q < 16; ++q) v[q] = part[(int64_t)(c + q) * per + e];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) sum += v[q];
     }
+    for (; c < slices; ++c) sum += part[(int64_t)c * per + e];
+    dW[e] += sum;
 }
 
 // ----------------------------------------------------------------------------- elementwise
@@ -626,24 +693,16 @@ void forward(vfem_net* N) {
     conv<true>(N, layerInput(N, 7), N->wb[7], N->w + N->boff[7], N->y, 0, 16, 0);
 }
 
-// Spatial blocks of layer l's weight gradient: one block per SM over its (ci, co) parts, at most one a tile.
-constexpr int wgM(int cin) { return cin == 48 ? 3 : cin >= 32 ? 2 : 1; }   // 16-channel ci tiles of a block
-constexpr int wgN(int cout) { return cout >= 32 ? 4 : 2; }                 // 8-channel co tiles
-int wgSlices(int n, int cin, int cout) {
-    const int tx = (n + 7) / 8, tiles = tx * tx * ((n + WG_TZ - 1) / WG_TZ);
-    const int parts = cin / (16 * wgM(cin)) * (cout / (8 * wgN(cout)));
-    const int perSm = wgM(cin) * wgN(cout) <= 4 ? 2 : 1;  // by registers: 24 to 96 accumulators a thread
-    return std::max(1, std::min(tiles, 152 * perSm / parts));
-}
+int wgChunks(int64_t V) { return (int)((V + WG_CHUNK - 1) / WG_CHUNK); }
 
 template <int MT, int NT>
-void launchWGrad(vfem_net* N, const Input& in, const bf16* g, int n, int Cout, int slices) {
-    constexpr size_t smem = 2 * (size_t)wgStageBytes<MT, NT>();
+void launchWGrad(vfem_net* N, const Input& in, const bf16* g, int n, int Cout, int chunks) {
     static const cudaError_t attr = cudaFuncSetAttribute(kWGrad<MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)smem);
+                                                         wgSmem<MT, NT>());
     (void)attr;
-    const dim3 grid((unsigned)slices, (unsigned)((in.Ca + in.Cb) / (16 * MT) * (Cout / (8 * NT))));
-    kWGrad<MT, NT><<<grid, WG_THREADS, smem, N->stream>>>(in, g, N->wgPart, n, Cout);
+    const dim3 grid((unsigned)chunks, (unsigned)((in.Ca + in.Cb) / (16 * MT) * (Cout / (8 * NT))), 3);
+    const unsigned long long mul = ((1ull << 40) + n - 1) / n;
+    kWGrad<MT, NT><<<grid, WG_THREADS, wgSmem<MT, NT>(), N->stream>>>(in, g, N->wgPart, n, mul, Cout);
 }
 
 // Backward of convolution l: given dL/d(out) in gout (f32, [V][Cout]) and the
@@ -654,13 +713,15 @@ void convBwd(vfem_net* N, int l, const bf16* out, const float* gout, float* gin)
     const int n = N->n >> lvl;
     const int64_t V = N->V[lvl], per = 27LL * Cin * Cout + Cout;
     kReluMask<<<blocks(V * Cout), 256, 0, N->stream>>>(gout, out, N->gmask, V * Cout, kRelu[l]);
+    // (ci, co) of a block: large ones read each operand least often; few chunks (V below
+    // 16 x 2,048 at the coarse levels) take small ones, to have blocks for the 152 SMs
+    const int chunks = wgChunks(V);
     const Input in = layerInput(N, l);
-    const int slices = wgSlices(n, Cin, Cout);
-    if (Cin == 48) launchWGrad<3, 2>(N, in, N->gmask, n, Cout, slices);
-    else if (Cin == 16 && Cout == 16) launchWGrad<1, 2>(N, in, N->gmask, n, Cout, slices);
-    else if (Cin == 16) launchWGrad<1, 4>(N, in, N->gmask, n, Cout, slices);
-    else launchWGrad<2, 4>(N, in, N->gmask, n, Cout, slices);
-    kGradSum<<<(unsigned)((per + 31) / 32), 256, 0, N->stream>>>(N->wgPart, N->gw + N->woff[l], per, slices);
+    if (Cin == 48) launchWGrad<3, 2>(N, in, N->gmask, n, Cout, chunks);
+    else if (Cout == 16) launchWGrad<1, 2>(N, in, N->gmask, n, Cout, chunks);
+    else if (Cin == 16 || chunks < 16) launchWGrad<1, 4>(N, in, N->gmask, n, Cout, chunks);
+    else launchWGrad<2, 4>(N, in, N->gmask, n, Cout, chunks);
+    kGradSum<<<(unsigned)((per + 63) / 64), 64, 0, N->stream>>>(N->wgPart, N->gw + N->woff[l], per, chunks);
     if (gin) conv<true>(N, Input{nullptr, N->gmask, 0, Cout}, N->wt[l], nullptr, gin, lvl, Cin, 0);
 }
 
@@ -751,7 +812,7 @@ vfem_status vfem_net_create(int32_t n, vfem_net** out) {
     NA(nalloc(&N->gmask, gmax));
     int64_t wmax = 0;
     for (int l = 0; l < kLayers; ++l)
-        wmax = std::max<int64_t>(wmax, wgSlices(n >> kLevel[l], kCin[l], kCout[l]) * (27LL * kCin[l] * kCout[l] + kCout[l]));
+        wmax = std::max<int64_t>(wmax, wgChunks(V[kLevel[l]]) * (27LL * kCin[l] * kCout[l] + kCout[l]));
     NA(nalloc(&N->wgPart, wmax));
     NA(nalloc(&N->part, 4096));
     NA(cudaMallocHost((void**)&N->hostStage, sizeof(float) * V[0] * 16));
