@@ -23,10 +23,10 @@
 #include <map>
 #include <string>
 #include <tuple>
-#include <thread>
 #include <type_traits>
 #include <vector>
 
+#include "host_copy.h"
 #include "kernels.h"
 #include "setup_gpu.h"
 
@@ -134,12 +134,11 @@ struct vfem_problem {
     Scalars* S = nullptr;
     Scalars* hS = nullptr;
     RedBuf rb{};
-    // compressed staging (measured on GB300: kernels reading and writing the
-    // caller's pageable host arrays directly were slower than these copies)
+    // a host vector in the compressed numbering, on the device (measured on GB300: kernels reading
+    // and writing the caller's host arrays directly were slower than these copies)
     unsigned* dFlag = nullptr;  // non-finite input flag of the scatter
     double* dComp = nullptr;  // 3 * nused(level 0) (largest level)
-    double* hIn = nullptr;    // pinned
-    double* hOut = nullptr;   // pinned
+    PinnedRing ring;          // for host vectors above kDirectMax
     // constants for the kernels
     double op64[45 + 576];
     float op32[45 + 576];
@@ -222,8 +221,6 @@ void freeProblem(vfem_problem* p) {
     cudaFree(p->dFlag); cudaFree(p->V64); cudaFree(p->V32); cudaFree(p->KV64); cudaFree(p->KV32);
     cudaFree(p->S); cudaFree(p->rb.partials); cudaFree(p->rb.ticket); cudaFree(p->dComp);
     if (p->hS) cudaFreeHost(p->hS);
-    if (p->hIn) cudaFreeHost(p->hIn);
-    if (p->hOut) cudaFreeHost(p->hOut);
     if (p->stream) cudaStreamDestroy(p->stream);
     delete p;
 }
@@ -750,8 +747,6 @@ vfem_status createImpl(const uint8_t* vox, int nx, int ny, int nz, const double*
     CKP(dalloc(&p->dComp, 3 * p->L[0].nused));
     CKP(dalloc(&p->dFlag, 1));
     CKP(cudaMallocHost((void**)&p->hS, sizeof(Scalars)));
-    CKP(cudaMallocHost((void**)&p->hIn, sizeof(double) * 3 * (size_t)std::max<int64_t>(1, p->L[0].nused)));
-    CKP(cudaMallocHost((void**)&p->hOut, sizeof(double) * 3 * (size_t)std::max<int64_t>(1, p->L[0].nused)));
     st = buildCoarse(p);
     if (st == VFEM_OK) st = ensureCoarse<float>(p, false);  // the mixed solver's, and a check that Kc is SPD
     if (st != VFEM_OK) return bail(st);
@@ -1222,35 +1217,11 @@ vfem_status solveImpl(vfem_problem* p, const vfem_options* optIn, bool haveX0, v
     return s;
 }
 
-// memcpy split over host threads for large host <-> pinned copies (one thread
-// copies ~10 GB/s on the Grace host; the staging copies are 8 bytes per DOF).
-void hostCopy(void* dst, const void* src, size_t bytes) {
-    const size_t kSlice = (size_t)32 << 20;
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    static const size_t cap = (size_t)std::max<long long>(1, envInt("VFEM_HOST_COPY_THREADS", 8));
-    const size_t nt = std::min<size_t>({cap, (size_t)hw, (bytes + kSlice - 1) / kSlice});
-    if (nt <= 1) {
-        std::memcpy(dst, src, bytes);
-        return;
-    }
-    const size_t chunk = (bytes / nt + 63) & ~(size_t)63;
-    std::vector<std::thread> th;
-    for (size_t t = 1; t < nt; ++t) {
-        const size_t off = t * chunk;
-        if (off >= bytes) break;
-        const size_t len = std::min(chunk, bytes - off);
-        th.emplace_back([=] { std::memcpy((char*)dst + off, (const char*)src + off, len); });
-    }
-    std::memcpy(dst, src, std::min(chunk, bytes));
-    for (auto& t : th) t.join();
-}
-
 // Host compressed vector -> dense device vector of level lv.  checkFinite: the
 // scatter flags non-finite input (read back by the caller after a sync).
 vfem_status toDenseHost(vfem_problem* p, int lv, const double* host, double* dense, bool checkFinite) {
     DevLevel& l = p->L[lv];
-    hostCopy(p->hIn, host, sizeof(double) * 3 * (size_t)l.nused);
-    CK(cudaMemcpyAsync(p->dComp, p->hIn, sizeof(double) * 3 * (size_t)l.nused, cudaMemcpyHostToDevice, p->stream));
+    CK(copyToDevice(p->ring, p->dComp, host, sizeof(double) * 3 * (size_t)l.nused, p->stream));
     CK(cudaMemsetAsync(dense, 0, sizeof(double) * (size_t)l.nvec(), p->stream));
     if (checkFinite) CK(cudaMemsetAsync(p->dFlag, 0, sizeof(unsigned), p->stream));
     p->launches += launchScatterCompressed<double>(p->stream, l.nused, l.nodeStore, p->dComp, dense,
@@ -1263,9 +1234,7 @@ vfem_status fromDenseHost(vfem_problem* p, int lv, const double* dense, double* 
     DevLevel& l = p->L[lv];
     p->launches += launchGatherCompressed<double>(p->stream, l.nused, l.nodeStore, dense, p->dComp);
     g_launches += 1;
-    CK(cudaMemcpyAsync(p->hOut, p->dComp, sizeof(double) * 3 * (size_t)l.nused, cudaMemcpyDeviceToHost, p->stream));
-    CK(cudaStreamSynchronize(p->stream));
-    hostCopy(host, p->hOut, sizeof(double) * 3 * (size_t)l.nused);
+    CK(copyToHost(p->ring, host, p->dComp, sizeof(double) * 3 * (size_t)l.nused, p->stream));
     return VFEM_OK;
 }
 
@@ -1389,7 +1358,9 @@ vfem_status vfem_solve(vfem_problem* p, const vfem_options* opt, const double* u
         vfem_status s0 = toDenseHost(p, 0, u0, p->x64, false);
         if (s0 != VFEM_OK) return s0;
     }
+    PopulateTask pages(u_out, sizeof(double) * 3 * (size_t)p->L[0].nused);  // while the solve runs
     vfem_status s = solveImpl(p, opt, u0 != nullptr, st);
+    pages.wait();
     if (s == VFEM_OK || s == VFEM_ERR_NOT_CONVERGED) {
         vfem_status s2 = fromDenseHost(p, 0, p->x64, u_out);
         if (s2 != VFEM_OK) return s2;

@@ -26,11 +26,11 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <cstring>
 #include <string>
 #include <type_traits>
 #include <vector>
 
+#include "host_copy.h"
 #include "vfem_net.h"
 
 namespace {
@@ -128,19 +128,24 @@ __device__ __forceinline__ void stageHalo(uint32_t dst, const Input& in, int n, 
     }
 }
 
+// a weight row: 8 NT channels, any 8 rows in different banks
+template <int NT>
+__host__ __device__ constexpr int wRowBytes() { return NT == 1 ? 48 : 16 * NT + 16; }
+
 template <int CK, int NT, int TG, int TZ>
 constexpr size_t convSmem() {
     return (size_t)HALO * HALO * (TZ + 2) * rowBytes<CK>() +
-           (size_t)(TG == 27 ? 1 : 2) * TG * 16 * CK * (16 * NT + 16);
+           (size_t)(TG == 27 ? 1 : 2) * TG * 16 * CK * wRowBytes<NT>();
 }
 
+// OUT_PRED: the network's 3 output channels, FP32 [V][3] (NT = 1: their 8-channel tile alone).
 // OUT_MASKED: the data gradient through the relu of `act` (the tensor it is the gradient of), BF16.
-enum ConvOut { OUT_BF16, OUT_F32, OUT_MASKED };
+enum ConvOut { OUT_BF16, OUT_F32, OUT_MASKED, OUT_PRED };
 template <int CK, int NT, int TG, int TZ, ConvOut OUT>
 __global__ void __launch_bounds__(64 * TZ) kConv(const Input in, const bf16* __restrict__ W,
                                                  const float* __restrict__ bias, const bf16* __restrict__ act,
                                                  void* __restrict__ out, int n, int Cout, int relu) {
-    constexpr int NTH = 64 * TZ, NS = 27 / TG, ROW = rowBytes<CK>(), WROW = 16 * NT + 16;
+    constexpr int NTH = 64 * TZ, NS = 27 / TG, ROW = rowBytes<CK>(), WROW = wRowBytes<NT>();
     constexpr uint32_t haloBytes = HALO * HALO * (TZ + 2) * ROW, stageBytes = TG * 16 * CK * WROW;
     extern __shared__ __align__(16) unsigned char convSm[];
     const uint32_t sA = (uint32_t)__cvta_generic_to_shared(convSm), sB = sA + haloBytes;
@@ -194,12 +199,13 @@ __global__ void __launch_bounds__(64 * TZ) kConv(const Input in, const bf16* __r
                     ldsm4(A[1], aTap + 32 * c + 2 * HALO * ROW);
 #pragma unroll
                     for (int j = 0; j < NT; j += 2) {
-                        uint32_t B[4];
+                        uint32_t B[4];  // (NT = 1: the upper half is the row's padding, unused)
                         ldsm4t(B, b0 + (uint32_t)((t * CK + c) * 16 * WROW + 16 * j));
 #pragma unroll
                         for (int m = 0; m < 2; ++m) {
                             mma16816(acc[m][j], A[m][0], A[m][1], A[m][2], A[m][3], B[0], B[1]);
-                            mma16816(acc[m][j + 1], A[m][0], A[m][1], A[m][2], A[m][3], B[2], B[3]);
+                            if constexpr (NT > 1)
+                                mma16816(acc[m][j + 1], A[m][0], A[m][1], A[m][2], A[m][3], B[2], B[3]);
                         }
                     }
                 }
@@ -227,7 +233,11 @@ __global__ void __launch_bounds__(64 * TZ) kConv(const Input in, const bf16* __r
                         if (!(__uint_as_float(y << 16) > 0.f)) r0 = 0.f;
                         if (!(__uint_as_float(y & 0xffff0000u) > 0.f)) r1 = 0.f;
                     }
-                    if (OUT == OUT_F32)
+                    if (OUT == OUT_PRED) {
+                        float* o = static_cast<float*>(out) + v * 3 + co;
+                        if (co < 3) o[0] = r0;
+                        if (co + 1 < 3) o[1] = r1;
+                    } else if (OUT == OUT_F32)
                         *reinterpret_cast<float2*>(static_cast<float*>(out) + v * Cout + co) = make_float2(r0, r1);
                     else
                         *reinterpret_cast<__nv_bfloat162*>(static_cast<bf16*>(out) + v * Cout + co) =
@@ -522,21 +532,39 @@ __global__ void kSkipGrad(const float* __restrict__ g, const float* __restrict__
     }
 }
 
-// Masked MSE on channels 0..2 of y (16 channels): loss = sum m (y - t)^2 / count;
-// its gradient as the BF16 operand g (16 channels, 0 beyond 2).  Partial sums in part[blockIdx].
+// The loss's factor 1 / (3 sum of the mask) (one block, beside the previous sample's kernels).
+__global__ void __launch_bounds__(1024) kMaskCount(const float* __restrict__ m, int64_t V, float* __restrict__ invCount) {
+    __shared__ double s[1024];
+    double acc = 0.0;
+    for (int64_t v = 4 * (int64_t)threadIdx.x; v < V; v += 4096) {  // V is a multiple of 512
+        const float4 q = *reinterpret_cast<const float4*>(m + v);
+        acc += ((double)q.x + q.y) + ((double)q.z + q.w);
+    }
+    s[threadIdx.x] = acc;
+    __syncthreads();
+    for (int o = 512; o > 0; o >>= 1) {
+        if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *invCount = s[0] > 0.0 ? (float)(1.0 / (3.0 * s[0])) : 0.f;
+}
+
+// Masked MSE of the prediction y: loss = sum m (y - t)^2 / count; its gradient as the BF16
+// operand g (16 channels, 0 beyond 2).  Partial sums in part[blockIdx], invCount behind them.
+constexpr int kLossBlocks = 1024;
 __global__ void kMse(const float* __restrict__ y, const float* __restrict__ t, const float* __restrict__ m,
-                     bf16* __restrict__ g, double* __restrict__ part, int64_t V, float invCount) {
+                     bf16* __restrict__ g, double* __restrict__ part, int64_t V, const float* __restrict__ inv) {
     __shared__ double s[256];
+    const float invCount = *inv;
     double acc = 0.0;
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
         const float mv = m[v];
-        const float4 yv = *reinterpret_cast<const float4*>(y + v * 16);
-        const float d[3] = {yv.x - t[v * 3], yv.y - t[v * 3 + 1], yv.z - t[v * 3 + 2]};
         float gr[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            acc += (double)(mv * d[c] * d[c]);
-            gr[c] = 2.f * mv * d[c] * invCount;
+            const float d = y[v * 3 + c] - t[v * 3 + c];
+            acc += (double)(mv * d * d);
+            gr[c] = 2.f * mv * d * invCount;
         }
         uint4* o = reinterpret_cast<uint4*>(g + v * 16);
         o[0] = make_uint4(bf16x2(gr[0], gr[1]), bf16x2(gr[2], 0.f), 0u, 0u);
@@ -548,7 +576,16 @@ __global__ void kMse(const float* __restrict__ y, const float* __restrict__ t, c
         if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = s[0];
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = s[0];
+        if (blockIdx.x == 0) part[kLossBlocks] = invCount;
+    }
+}
+
+// y = x / by
+__global__ void kDivide(const float* __restrict__ x, float* __restrict__ y, int64_t n, float by) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        y[i] = x[i] / by;
 }
 
 __global__ void kAdam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
@@ -596,6 +633,8 @@ inline int blocks(int64_t n) {
 }  // namespace
 
 // ----------------------------------------------------------------------------- network object
+constexpr int kLossRing = 64;  // samples between two reads of their losses
+
 struct vfem_net {
     int n = 0;  // finest grid size (multiple of 8)
     int64_t V[4] = {};
@@ -607,13 +646,16 @@ struct vfem_net {
     int64_t step = 0;
     // activations (bf16) and gradients (f32)
     bf16 *x = nullptr, *e[4] = {}, *p[4] = {}, *d[3] = {};
-    float* y = nullptr;
-    float *t = nullptr, *mask = nullptr, *xin = nullptr;
+    float* y = nullptr;  // prediction [V][3]
+    // a sample's host inputs on the device, twice: one is copied in while the other is trained on
+    float *xin[2] = {}, *t[2] = {}, *mask[2] = {}, *inv = nullptr;
+    cudaStream_t copyStream = nullptr;
+    cudaEvent_t copied[2] = {}, consumed[2] = {};
     float *gp[4] = {}, *gc[3] = {};  // gradients of the pooled and the decoder inputs
     bf16* gm[2] = {};                // gradient operands: of the last layer, of the others (largest layer)
     float* wgPart = nullptr;  // per-block weight and bias gradients (largest layer)
-    double* part = nullptr;
-    float* hostStage = nullptr;
+    vfem::PinnedRing ring;  // for samples above kDirectMax
+    double *part = nullptr, *hostPart = nullptr;  // loss sums of kLossRing samples; pinned copy
 };
 
 namespace {
@@ -655,7 +697,7 @@ void launchConv(vfem_net* N, const Input& in, const bf16* W, const float* b, con
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, 64 * TZ, smem);
         return std::max(1, k);
     }();
-    const int tx = (n + 7) / 8, tiles = tx * tx * ((n + TZ - 1) / TZ), parts = Cout / (8 * NT);
+    const int tx = (n + 7) / 8, tiles = tx * tx * ((n + TZ - 1) / TZ), parts = std::max(1, Cout / (8 * NT) / (OUT == OUT_PRED ? 2 : 1));
     const dim3 grid((unsigned)std::min(tiles, std::max(1, 152 * perSm / parts)), (unsigned)parts);
     kern<<<grid, 64 * TZ, smem, N->stream>>>(in, W, b, act, out, n, Cout, relu);
 }
@@ -685,7 +727,11 @@ void conv(vfem_net* N, const Input& in, const bf16* W, const float* b, const bf1
         CONV_CASE(64, 32, 4, 1, 4)
         CONV_CASE(32, 16, 2, 27, 4)
     }
-    CONV_CASE(16, 16, 2, 27, 4)
+    if constexpr (OUT == OUT_PRED) {
+        CONV_CASE(16, 16, 1, 27, 4)
+    } else {
+        CONV_CASE(16, 16, 2, 27, 4)
+    }
 #undef CONV_CASE
 }
 
@@ -727,7 +773,7 @@ void forward(vfem_net* N) {
     layer(4, N->d[2]);
     layer(5, N->d[1]);
     layer(6, N->d[0]);
-    conv<OUT_F32>(N, layerInput(N, 7), N->wb[7], N->w + N->boff[7], nullptr, N->y, 0, 16, 0);
+    conv<OUT_PRED>(N, layerInput(N, 7), N->wb[7], N->w + N->boff[7], nullptr, N->y, 0, 16, 0);
 }
 
 int wgChunks(int64_t V) { return (int)((V + WG_CHUNK - 1) / WG_CHUNK); }
@@ -838,10 +884,16 @@ vfem_status vfem_net_create(int32_t n, vfem_net** out) {
         NA(nalloc(&N->gc[l], V[l] * cc[l]));
         NA(nalloc(&N->d[l], V[l] * dc[l]));
     }
-    NA(nalloc(&N->y, V[0] * 16));
-    NA(nalloc(&N->xin, V[0] * 16));
-    NA(nalloc(&N->t, V[0] * 3));
-    NA(nalloc(&N->mask, V[0]));
+    NA(nalloc(&N->y, V[0] * 3));
+    for (int i = 0; i < 2; ++i) {
+        NA(nalloc(&N->xin[i], V[0] * 16));
+        NA(nalloc(&N->t[i], V[0] * 3));
+        NA(nalloc(&N->mask[i], V[0]));
+        NA(cudaEventCreateWithFlags(&N->copied[i], cudaEventDisableTiming));
+        NA(cudaEventCreateWithFlags(&N->consumed[i], cudaEventDisableTiming));
+    }
+    NA(nalloc(&N->inv, 2));
+    NA(cudaStreamCreateWithFlags(&N->copyStream, cudaStreamNonBlocking));
     int64_t gmax = 0;
     for (int l = 0; l < kLayers; ++l) gmax = std::max<int64_t>(gmax, V[kLevel[l]] * kCout[l]);
     NA(nalloc(&N->gm[0], V[0] * 16));
@@ -849,9 +901,9 @@ vfem_status vfem_net_create(int32_t n, vfem_net** out) {
     int64_t wmax = 0;
     for (int l = 0; l < kLayers; ++l)
         wmax = std::max<int64_t>(wmax, wgChunks(V[kLevel[l]]) * (27LL * kCin[l] * kCout[l] + kCout[l]));
-    NA(nalloc(&N->wgPart, wmax));
-    NA(nalloc(&N->part, 4096));
-    NA(cudaMallocHost((void**)&N->hostStage, sizeof(float) * V[0] * 16));
+    NA(nalloc(&N->wgPart, std::max(wmax, off)));  // also the batch mean on its way to the caller
+    NA(nalloc(&N->part, kLossRing * (kLossBlocks + 1)));
+    NA(cudaMallocHost((void**)&N->hostPart, sizeof(double) * kLossRing * (kLossBlocks + 1)));
 #undef NA
     *out = N;
     return VFEM_OK;
@@ -864,9 +916,15 @@ void vfem_net_destroy(vfem_net* N) {
     cudaFree(N->x);
     for (int l = 0; l < 4; ++l) { cudaFree(N->e[l]); cudaFree(N->p[l]); cudaFree(N->gp[l]); }
     for (int l = 0; l < 3; ++l) { cudaFree(N->gc[l]); cudaFree(N->d[l]); }
-    cudaFree(N->y); cudaFree(N->xin); cudaFree(N->t); cudaFree(N->mask); cudaFree(N->gm[0]); cudaFree(N->gm[1]);
+    cudaFree(N->y); cudaFree(N->inv); cudaFree(N->gm[0]); cudaFree(N->gm[1]);
+    for (int i = 0; i < 2; ++i) {
+        cudaFree(N->xin[i]); cudaFree(N->t[i]); cudaFree(N->mask[i]);
+        if (N->copied[i]) cudaEventDestroy(N->copied[i]);
+        if (N->consumed[i]) cudaEventDestroy(N->consumed[i]);
+    }
     cudaFree(N->part); cudaFree(N->wgPart);
-    if (N->hostStage) cudaFreeHost(N->hostStage);
+    if (N->hostPart) cudaFreeHost(N->hostPart);
+    if (N->copyStream) cudaStreamDestroy(N->copyStream);
     if (N->stream) cudaStreamDestroy(N->stream);
     delete N;
 }
@@ -886,8 +944,7 @@ vfem_status vfem_net_set_params(vfem_net* N, const float* params) {
 
 vfem_status vfem_net_get_params(vfem_net* N, float* params) {
     if (!N || !params) return netFail(VFEM_ERR_INVALID_ARGUMENT, "null argument");
-    NCK(cudaMemcpyAsync(params, N->w, sizeof(float) * N->nparam, cudaMemcpyDeviceToHost, N->stream));
-    NCK(cudaStreamSynchronize(N->stream));
+    NCK(vfem::copyToHost(N->ring, params, N->w, sizeof(float) * N->nparam, N->stream));
     return VFEM_OK;
 }
 
@@ -895,52 +952,63 @@ vfem_status vfem_net_get_params(vfem_net* N, float* params) {
 vfem_status vfem_net_forward(vfem_net* N, const float* input, float* output) {
     if (!N || !input || !output) return netFail(VFEM_ERR_INVALID_ARGUMENT, "null argument");
     const int64_t V = N->V[0];
-    std::memcpy(N->hostStage, input, sizeof(float) * V * 16);
-    NCK(cudaMemcpyAsync(N->xin, N->hostStage, sizeof(float) * V * 16, cudaMemcpyHostToDevice, N->stream));
-    kF32ToBf16<<<blocks(V * 2), 256, 0, N->stream>>>(N->xin, N->x, V * 16);
+    NCK(vfem::copyToDevice(N->ring, N->xin[0], input, sizeof(float) * V * 16, N->stream));
+    kF32ToBf16<<<blocks(V * 2), 256, 0, N->stream>>>(N->xin[0], N->x, V * 16);
     forward(N);
     NCK(cudaGetLastError());
-    NCK(cudaMemcpyAsync(N->hostStage, N->y, sizeof(float) * V * 16, cudaMemcpyDeviceToHost, N->stream));
-    NCK(cudaStreamSynchronize(N->stream));
-    for (int64_t v = 0; v < V; ++v)
-        for (int c = 0; c < 3; ++c) output[v * 3 + c] = N->hostStage[v * 16 + c];
+    NCK(vfem::copyToHost(N->ring, output, N->y, sizeof(float) * V * 3, N->stream));
     return VFEM_OK;
 }
 
 // Forward + backward of a batch of `batch` samples; gradients (summed over the
 // batch, divided by it) to grads (host, nparam) if given, Adam step with lr if
-// lr > 0.  loss_out: mean masked MSE.
+// lr > 0.  loss_out: mean masked MSE.  Sample b + 1 is copied to the device while
+// sample b is trained on; nothing waits for the host until the batch is through.
 vfem_status vfem_net_train_batch(vfem_net* N, const float* inputs, const float* targets, const float* masks,
                                  int32_t batch, float lr, float* grads, float* loss_out) {
     if (!N || !inputs || !targets || !masks || batch < 1) return netFail(VFEM_ERR_INVALID_ARGUMENT, "bad argument");
     const int64_t V = N->V[0];
     NCK(cudaMemsetAsync(N->gw, 0, sizeof(float) * N->nparam, N->stream));
     double lossSum = 0.0;
-    std::vector<double> part(1024);
+    auto copyIn = [&](int b) -> cudaError_t {
+        const int i = b & 1;
+        cudaError_t e;
+        if (b >= 2 && (e = cudaStreamWaitEvent(N->copyStream, N->consumed[i], 0)) != cudaSuccess) return e;
+        auto in = [&](float* dst, const float* src, int64_t per) {
+            return vfem::copyToDevice(N->ring, dst, src + b * V * per, sizeof(float) * V * per, N->copyStream);
+        };
+        if ((e = in(N->xin[i], inputs, 16)) || (e = in(N->t[i], targets, 3)) || (e = in(N->mask[i], masks, 1))) return e;
+        kMaskCount<<<1, 1024, 0, N->copyStream>>>(N->mask[i], V, N->inv + i);
+        return cudaEventRecord(N->copied[i], N->copyStream);
+    };
+    NCK(copyIn(0));
     for (int b = 0; b < batch; ++b) {
-        std::memcpy(N->hostStage, inputs + (int64_t)b * V * 16, sizeof(float) * V * 16);
-        NCK(cudaMemcpyAsync(N->xin, N->hostStage, sizeof(float) * V * 16, cudaMemcpyHostToDevice, N->stream));
-        kF32ToBf16<<<blocks(V * 2), 256, 0, N->stream>>>(N->xin, N->x, V * 16);
-        NCK(cudaMemcpyAsync(N->t, targets + (int64_t)b * V * 3, sizeof(float) * V * 3, cudaMemcpyHostToDevice, N->stream));
-        NCK(cudaMemcpyAsync(N->mask, masks + (int64_t)b * V, sizeof(float) * V, cudaMemcpyHostToDevice, N->stream));
+        const int i = b & 1, slot = b % kLossRing;
+        double* part = N->part + slot * (kLossBlocks + 1);
+        NCK(cudaStreamWaitEvent(N->stream, N->copied[i], 0));
+        kF32ToBf16<<<blocks(V * 2), 256, 0, N->stream>>>(N->xin[i], N->x, V * 16);
         forward(N);
-        double cnt = 0.0;
-        for (int64_t v = 0; v < V; ++v) cnt += masks[(int64_t)b * V + v];
-        const float invCount = cnt > 0 ? (float)(1.0 / (3.0 * cnt)) : 0.f;
-        kMse<<<1024, 256, 0, N->stream>>>(N->y, N->t, N->mask, N->gm[0], N->part, V, invCount);
+        kMse<<<kLossBlocks, 256, 0, N->stream>>>(N->y, N->t[i], N->mask[i], N->gm[0], part, V, N->inv + i);
+        NCK(cudaEventRecord(N->consumed[i], N->stream));
         backward(N);
-        NCK(cudaMemcpyAsync(part.data(), N->part, sizeof(double) * 1024, cudaMemcpyDeviceToHost, N->stream));
-        NCK(cudaStreamSynchronize(N->stream));
-        double s = 0.0;
-        for (double p : part) s += p;
-        lossSum += s * invCount;
+        if (b + 1 < batch) NCK(copyIn(b + 1));
+        if (b + 1 == batch || slot + 1 == kLossRing) {
+            NCK(cudaMemcpyAsync(N->hostPart, N->part, sizeof(double) * (slot + 1) * (kLossBlocks + 1),
+                                cudaMemcpyDeviceToHost, N->stream));
+            NCK(cudaStreamSynchronize(N->stream));
+            for (int q = 0; q <= slot; ++q) {
+                const double* h = N->hostPart + q * (kLossBlocks + 1);
+                double s = 0.0;
+                for (int k = 0; k < kLossBlocks; ++k) s += h[k];
+                lossSum += s * (float)h[kLossBlocks];
+            }
+        }
     }
     NCK(cudaGetLastError());
     if (loss_out) *loss_out = (float)(lossSum / batch);
     if (grads) {
-        NCK(cudaMemcpyAsync(grads, N->gw, sizeof(float) * N->nparam, cudaMemcpyDeviceToHost, N->stream));
-        NCK(cudaStreamSynchronize(N->stream));
-        for (int64_t i = 0; i < N->nparam; ++i) grads[i] /= (float)batch;
+        kDivide<<<blocks(N->nparam), 256, 0, N->stream>>>(N->gw, N->wgPart, N->nparam, (float)batch);
+        NCK(vfem::copyToHost(N->ring, grads, N->wgPart, sizeof(float) * N->nparam, N->stream));
     }
     if (lr > 0.f) {
         N->step++;
