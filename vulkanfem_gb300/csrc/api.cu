@@ -142,6 +142,8 @@ struct vfem_problem {
     // constants for the kernels
     double op64[45 + 576];
     float op32[45 + 576];
+    float cube32[8];     // a cube's constants for the FP32 products (Kc in matvec_march.cuh)
+    bool isCube = false;
     FxOperand fx;  // the structured FP64 product in block fixed point (matvec_fx.cu)
     // the tensor-core FP32 CG product (matvec_tc.cu), opt-in, when Ke admits an exact BF16 scaling
     TcOperand tc;
@@ -704,6 +706,12 @@ vfem_status createImpl(const uint8_t* vox, int nx, int ny, int nz, const double*
         p->op32[45 + i] = (float)p->ke.Ke[i];
     }
     fxPrepare(p->ke, p->fx);
+    {
+        double k[8] = {}, sum = 0.0;
+        p->isCube = cubeConstants(p->ke, k, sum);
+        const double v[8] = {k[0], k[1], k[2], k[3], k[4] + k[5], k[4] - k[5], k[6], k[7]};
+        for (int i = 0; p->isCube && i < 8; ++i) p->cube32[i] = (float)v[i];
+    }
     auto bail = [&](vfem_status s) {
         freeProblem(p);
         return s;
@@ -839,7 +847,7 @@ int matvec(vfem_problem* p, const MatvecArgs<T>& a, bool allowTc = true) {
             return 1;
         }
     }
-    return launchMatvec<T>(ctx(p), a, p->ke.structured, opc<T>(p));
+    return launchMatvec<T>(ctx(p), a, p->ke.structured, opc<T>(p), p->isCube ? p->cube32 : nullptr);
 }
 
 // z = M^-1 r on level `lv` (r, z given); returns kernels; on level 0 the final
@@ -984,7 +992,7 @@ int iteration(vfem_problem* p, const vfem_options& o, double** zOut64, float** z
             a.zin = *zOut32;
             a.pAlt = p->p32b;
             a.xacc = p->x32;
-            k += launchMatvecPX(c, a, static_cast<const float*>(opc<float>(p)));
+            k += launchMatvecPX(c, a, static_cast<const float*>(opc<float>(p)), p->isCube ? p->cube32 : nullptr);
         } else {
             k += matvec<float>(p, a);
         }
@@ -1635,7 +1643,7 @@ vfem_status vfem_profile_kernels(vfem_problem* p, int32_t reps, double* ms) {
                     a.zin = l0.z32;
                     a.pAlt = p->p32b;
                     a.xacc = p->x32;
-                    return launchMatvecPX(c, a, static_cast<const float*>(opc<float>(p)));
+                    return launchMatvecPX(c, a, static_cast<const float*>(opc<float>(p)), p->isCube ? p->cube32 : nullptr);
                 }
                 case VFEM_K_MATVEC_FP64: {
                     MatvecArgs<double> a = mvArgs<double>(p, 0, p->p64, p->Ap64, MV_AX);

@@ -20,7 +20,9 @@
 //                    deferred x update).
 // Reductions are deterministic: block partials in a fixed grid, summed in a
 // fixed order by the last block to finish (no floating-point atomics).
+#include <algorithm>
 #include <cfloat>
+#include <cmath>
 #include <cstdio>
 #include <mutex>
 #include <type_traits>
@@ -54,14 +56,15 @@ __global__ void __launch_bounds__(MV_TX* MV_TY, 1)
 
 // The structured (isotropic cube) product: walshMarch (matvec_march.cuh) and the
 // grid reduction of its dots.
-template <typename T, typename TC, int OUT = OUT_ANY>
+// KP: Ks<TC>, or the cube's Kc<TC>.
+template <typename T, typename TC, int OUT = OUT_ANY, typename KP = Ks<TC>>
 __global__ void __launch_bounds__(MV_TX* MV_TY, sizeof(TC) == 4 ? 3 : 2)
-    kMatvecH(MatvecArgs<T> a, const Ks<TC> kp, Scalars* S, RedBuf rb) {
+    kMatvecH(MatvecArgs<T> a, const KP kp, int layers, Scalars* S, RedBuf rb) {
     if (a.checkDone && S->done) return;
     if (a.condTrue && !trueResidualDue(S)) return;
     extern __shared__ __align__(16) unsigned char smemRaw[];
     DotAcc<TC> d0, d1;
-    [[maybe_unused]] const int sel = walshMarch<T, TC, OUT>(a, kp, S, smemRaw, d0, d1);
+    [[maybe_unused]] const int sel = walshMarch<T, TC, OUT, KP>(a, kp, S, smemRaw, d0, d1, layers);
     if (a.epi != EPI_NONE) {
         double v[2] = {d0.get(), d1.get()}, t[2];
         if (gridReduce<MV_TX * MV_TY, 2>(v, rb, t)) {
@@ -1177,25 +1180,65 @@ cudaError_t setKernelAttributes() {
     if ((e = cudaFuncSetAttribute(kMatvecH<float, float>, A, s32))) return e;
     if ((e = cudaFuncSetAttribute(kMatvecH<float, float, OUT_CG>, A, s32))) return e;
     if ((e = cudaFuncSetAttribute(kMatvecH<float, float, OUT_CG_PX>, A, s32))) return e;
+    if ((e = cudaFuncSetAttribute(kMatvecH<float, float, OUT_ANY, Kc<float>>, A, s32))) return e;
+    if ((e = cudaFuncSetAttribute(kMatvecH<float, float, OUT_CG, Kc<float>>, A, s32))) return e;
+    if ((e = cudaFuncSetAttribute(kMatvecH<float, float, OUT_CG_PX, Kc<float>>, A, s32))) return e;
     if ((e = cudaFuncSetAttribute(kMatvecH<double, double, OUT_CG>, A, s64))) return e;
     if ((e = cudaFuncSetAttribute(kMatvec<double>, A, s64))) return e;
     return cudaFuncSetAttribute(kMatvec<float>, A, s32);
 }
 
+// Node layers of a product block.  About 32, in equal parts, where that gives two
+// blocks an SM (128^3: 33 instead of 32, which left a fifth part of one layer; FP32
+// with the direction update 72 -> 70 us; 16 to 64 layers measure within 3% on
+// larger grids).  Smaller grids take the part count with the least (layers +
+// repeated layer and prologue) x (blocks an SM holds, at least `sat`: that many
+// share an SM without slowing each other): 33 x 17 x 17 nodes 24.6 -> 12.3 us, 65^3
+// 39 -> 21 us.
+int productLayers(const Grid& g, int sat) {
+    const int64_t tiles = (int64_t)((g.nx + MV_TX - 2) / (MV_TX - 1)) * ((g.ny + MV_TY - 2) / (MV_TY - 1));
+    int parts = std::max(1, (g.nz + MV_ZC / 2) / MV_ZC);
+    if (tiles * parts >= 2 * 152) return (g.nz + parts - 1) / parts;
+    int best = g.nz;
+    double least = 1e300;
+    for (parts = 1; 2 * parts <= g.nz + 1; ++parts) {
+        const int zc = (g.nz + parts - 1) / parts;
+        const double perSm = std::ceil((double)(tiles * ((g.nz + zc - 1) / zc)) / 152.0);
+        const double cost = (zc + 1.5) * std::max((double)sat, perSm);
+        if (cost < least) {
+            least = cost;
+            best = zc;
+        }
+        if (perSm > 8.0) break;
+    }
+    return best;
+}
+
+// FP32 products with a structured Ke take the cube's constants where it is one.
 template <typename T>
-int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, const void* opconst) {
+int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, const void* opconst, const float* cube) {
     const Grid& g = a.g;
-    dim3 grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + MV_TY - 2) / (MV_TY - 1), (g.nz + MV_ZC - 1) / MV_ZC);
+    const int zc = structured ? productLayers(g, 2) : MV_ZC;
+    dim3 grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + MV_TY - 2) / (MV_TY - 1), (g.nz + zc - 1) / zc);
     dim3 block(MV_TX, MV_TY);
     size_t smem = (size_t)(kSuElems + kSyElems) * sizeof(T);
+    const bool cg = a.mode == MV_AX && a.dot0 == DOT_X_OUT && !a.dot1 && !a.y32;
+    auto go = [&](auto kern, const auto& k) { kern<<<grid, block, smem, c.stream>>>(a, k, zc, c.S, c.rb); };
     if (structured) {
+        if constexpr (std::is_same<T, float>::value) {
+            if (cube) {
+                Kc<T> k;
+                for (int i = 0; i < 8; ++i) k.v[i] = cube[i];
+                if (cg) go(kMatvecH<T, T, OUT_CG, Kc<T>>, k);
+                else go(kMatvecH<T, T, OUT_ANY, Kc<T>>, k);
+                return 1;
+            }
+        }
         Ks<T> k;
         const T* src = static_cast<const T*>(opconst);
         for (int i = 0; i < 45; ++i) k.v[i] = src[i];
-        if (a.mode == MV_AX && a.dot0 == DOT_X_OUT && !a.dot1 && !a.y32)
-            kMatvecH<T, T, OUT_CG><<<grid, block, smem, c.stream>>>(a, k, c.S, c.rb);
-        else
-            kMatvecH<T, T><<<grid, block, smem, c.stream>>>(a, k, c.S, c.rb);
+        if (cg) go(kMatvecH<T, T, OUT_CG>, k);
+        else go(kMatvecH<T, T>, k);
     } else {
         Kd<T> k;
         const T* src = static_cast<const T*>(opconst) + 45;
@@ -1205,14 +1248,21 @@ int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, co
     return 1;
 }
 
-int launchMatvecPX(const LaunchCtx& c, const MatvecArgs<float>& a, const float* opconst) {
+int launchMatvecPX(const LaunchCtx& c, const MatvecArgs<float>& a, const float* opconst, const float* cube) {
     const Grid& g = a.g;
-    dim3 grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + MV_TY - 2) / (MV_TY - 1), (g.nz + MV_ZC - 1) / MV_ZC);
+    const int zc = productLayers(g, 2);
+    dim3 grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + MV_TY - 2) / (MV_TY - 1), (g.nz + zc - 1) / zc);
     dim3 block(MV_TX, MV_TY);
     size_t smem = (size_t)(kSuElems + kSyElems) * sizeof(float);
-    Ks<float> k;
-    for (int i = 0; i < 45; ++i) k.v[i] = opconst[i];
-    kMatvecH<float, float, OUT_CG_PX><<<grid, block, smem, c.stream>>>(a, k, c.S, c.rb);
+    if (cube) {
+        Kc<float> k;
+        for (int i = 0; i < 8; ++i) k.v[i] = cube[i];
+        kMatvecH<float, float, OUT_CG_PX, Kc<float>><<<grid, block, smem, c.stream>>>(a, k, zc, c.S, c.rb);
+    } else {
+        Ks<float> k;
+        for (int i = 0; i < 45; ++i) k.v[i] = opconst[i];
+        kMatvecH<float, float, OUT_CG_PX><<<grid, block, smem, c.stream>>>(a, k, zc, c.S, c.rb);
+    }
     return 1;
 }
 
@@ -1514,7 +1564,7 @@ cudaError_t launchMatvecNoAlloc(cudaStream_t s, const MatvecArgs<double>& a, boo
     } else if (structured) {
         Ks<double> k;
         for (int i = 0; i < 45; ++i) k.v[i] = static_cast<const double*>(opconst)[i];
-        kMatvecH<double, double><<<grid, block, smem, s>>>(b, k, S, rb);
+        kMatvecH<double, double><<<grid, block, smem, s>>>(b, k, MV_ZC, S, rb);
     } else {
         Kd<double> k;
         for (int i = 0; i < 576; ++i) k.v[i] = static_cast<const double*>(opconst)[45 + i];
@@ -1526,7 +1576,7 @@ cudaError_t launchMatvecNoAlloc(cudaStream_t s, const MatvecArgs<double>& a, boo
 
 // ------------------------------------------------------------------ instantiations
 #define INST_T(T)                                                                                                     \
-    template int launchMatvec<T>(const LaunchCtx&, const MatvecArgs<T>&, bool, const void*);                         \
+    template int launchMatvec<T>(const LaunchCtx&, const MatvecArgs<T>&, bool, const void*, const float*);                            \
     template int launchRestrict<T>(const LaunchCtx&, const Grid&, const Grid&, int, const T*, T*, int);               \
     template int launchProlongSmooth<T>(const LaunchCtx&, const Grid&, const Grid&, int, const T*, const T*,          \
                                         const T*, const uint8_t*, T*, double, int, const T*, int, int, HalfDiag);    \

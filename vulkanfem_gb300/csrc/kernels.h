@@ -120,8 +120,16 @@ struct LaunchCtx {
 cudaError_t setKernelAttributes();
 
 // ---- launchers (return the number of kernels launched) ----
+// cube: FP32 products, the constants of a cube's Ke (Kc in matvec_march.cuh) or null.
 template <typename T>
-int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, const void* opconst);
+int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, const void* opconst,
+                 const float* cube);
+int productLayers(const Grid& g, int sat);  // node layers a product block marches
+
+// The 8 constants of a cube's Khat (k: a - b, b of the normal strains; the shears; the mode-7
+// terms; (a + b) / 2 and (a - b) / 2 of the bending pairs; a - b, b of the (1,1,1) triple) and C, the
+// largest sum of |k| over what a component collects.  False when Ke is not a cube's.
+bool cubeConstants(const KeData& ke, double (&k)[8], double& C);
 
 // The FP64 product in block fixed point (matvec_fx.cu): the 8 constants of a
 // cube's Ke, or the 576 entries of any other, as 62-bit integers.  fxEligible:
@@ -135,7 +143,6 @@ struct FxOperand {
 bool fxPrepare(const KeData& ke, FxOperand& op);
 cudaError_t fxSetAttributes();
 bool fxEligible(const FxOperand& op, double scale);
-int fxLayers(const Grid& g);  // node layers a block marches
 void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOperand& op, const double* opconst,
                     Scalars* S, const RedBuf& rb);
 
@@ -207,7 +214,7 @@ int launchFlushX(const LaunchCtx& c, int64_t n, double* x64, float* x32, const f
 // FP32 CG product with the direction update fused into its input stage
 // (structured Ke): p = z + beta p_old, x32 += alpha p_old (unless folded),
 // y = K p (fixed rows 0), p.(Kp) -> EPI_ALPHA; flips Scalars::pSel.
-int launchMatvecPX(const LaunchCtx& c, const MatvecArgs<float>& a, const float* opconst);
+int launchMatvecPX(const LaunchCtx& c, const MatvecArgs<float>& a, const float* opconst, const float* cube);
 // Mixed precision: r -= alpha Ap with r.r (x += alpha p deferred); p = z + beta p
 // with the deferred x += alpha p.
 int launchUpdateR(const LaunchCtx& c, int64_t n, float* r, const float* Ap);

@@ -8,7 +8,7 @@
 // the dot of a node to the FP64 pipe.
 //
 // Measured: 191^3 with voids and log-normal moduli 3.72 -> 0.49 ms; 33 x 17 x 17
-// nodes 262 -> 20 us (shorter marches by fxLayers among it); a Ke in another
+// nodes 262 -> 20 us (shorter marches by productLayers among it); a Ke in another
 // corner order, as the dense 24 x 24 product, 96 x 80 x 72 half full, 1.56 ->
 // 0.26 ms.  Bound now: instruction issue (1,100 warp instructions per element
 // row, 59% of the issue slots, ALU 56%, wide multiply-adds 54% of their pipe)
@@ -457,7 +457,7 @@ template <int OUT>
 __device__ __noinline__ void fp64March(const MatvecArgs<double>* a, const Ks<double>* kp, int zc, Scalars* S,
                                        unsigned char* smem, DotAcc<double>* d) {
     d[0] = d[1] = DotAcc<double>();
-    walshMarch<double, double, OUT>(*a, *kp, S, smem, d[0], d[1], zc);
+    walshMarch<double, double, OUT, Ks<double>>(*a, *kp, S, smem, d[0], d[1], zc);
 }
 template <int OUT>
 __device__ __noinline__ void fp64March(const MatvecArgs<double>* a, const Kd<double>* kp, int zc, Scalars*,
@@ -505,6 +505,7 @@ bool fxDigits(const double* k, int n, double C, int low, int32_t* k1, int32_t* k
     outExp = 9 - f - 1023 - 127;
     return true;
 }
+}  // namespace
 
 // Khat of a cube, whose axes are interchangeable, has one constant per kind of
 // entry (a: diagonal, b: off-diagonal): normal strains (a, b), in-plane shears
@@ -532,7 +533,6 @@ bool cubeConstants(const KeData& ke, double (&k)[8], double& C) {
         2 * (std::fabs(k[4]) + std::fabs(k[5])) + std::fabs(k[6]) + std::fabs(k[7]);
     return true;
 }
-}  // namespace
 
 bool fxPrepare(const KeData& ke, FxOperand& op) {
     double k[8], C = 0.0;
@@ -567,7 +567,7 @@ bool fxEligible(const FxOperand& op, double scale) {
 
 void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOperand& op, const double* opconst,
                     Scalars* S, const RedBuf& rb) {
-    const int zc = fxLayers(a.g);
+    const int zc = productLayers(a.g, op.cube ? 2 : 1);
     const Grid& g = a.g;
     const dim3 block(MV_TX, FX_TY),
         grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + FX_TY - 2) / (FX_TY - 1), (g.nz + zc - 1) / zc);
@@ -596,15 +596,6 @@ void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOp
     else
         go(FxDenseArgs(), 24, 24, Kd<double>(), opconst + 45,
            cg ? kMatvecFx<OUT_CG, FxDenseArgs, Kd<double>> : kMatvecFx<OUT_ANY, FxDenseArgs, Kd<double>>);
-}
-
-int fxLayers(const Grid& g) {
-    // Few blocks: shorter marches (each repeats one element layer) until every SM has two blocks.
-    // 33 x 17 x 17 nodes: 6 blocks of 17 layers take 60 us, 54 blocks of 2 layers 20 us.
-    const int64_t tiles = (int64_t)((g.nx + MV_TX - 2) / (MV_TX - 1)) * ((g.ny + FX_TY - 2) / (FX_TY - 1));
-    int zc = MV_ZC;
-    while (zc > 2 && tiles * ((g.nz + zc - 1) / zc) < 2 * 152) zc /= 2;
-    return zc;
 }
 
 }  // namespace vfem

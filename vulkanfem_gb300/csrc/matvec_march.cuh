@@ -33,6 +33,13 @@ template <typename T>
 struct Ks {
     T v[45];
 };
+// The same for a cube, whose axes are interchangeable: one constant per kind of
+// entry (cubeConstants): a - b and b of the normal strains, the shears, the
+// mode-7 terms, a and b of the bending pairs, a - b and b of the (1,1,1) triple.
+template <typename T>
+struct Kc {
+    T v[8];
+};
 template <typename T>
 struct Kd {
     T v[576];
@@ -56,6 +63,37 @@ __device__ __forceinline__ void applyKhat(const T (&u)[24], T (&y)[24], const Ks
     KS_(36, 18, 18) KS_(37, 18, 16) KS_(38, 18, 11) KS_(39, 16, 18) KS_(40, 16, 16) KS_(41, 16, 11)
     KS_(42, 11, 18) KS_(43, 11, 16) KS_(44, 11, 11)
 #undef KS_
+}
+
+// y = e Khat u in the modes 1..7.
+template <typename T>
+__device__ __forceinline__ void scaledKhat(T (&u)[24], T (&y)[24], const Ks<T>& k, T e);
+// The cube's: 8 scaled constants and 33 operations instead of 21 and 45.
+template <typename T>
+__device__ __forceinline__ void scaledKhat(T (&u)[24], T (&y)[24], const Kc<T>& k, T e) {
+    T c[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) c[i] = e * k.v[i];
+    y[0] = y[1] = y[2] = T(0);
+    const T n = c[1] * (u[3] + u[7] + u[14]), t = c[7] * (u[18] + u[16] + u[11]);
+    y[3] = fma(c[0], u[3], n);
+    y[7] = fma(c[0], u[7], n);
+    y[14] = fma(c[0], u[14], n);
+    y[6] = y[4] = c[2] * (u[6] + u[4]);
+    y[12] = y[5] = c[2] * (u[12] + u[5]);
+    y[13] = y[8] = c[2] * (u[13] + u[8]);
+    y[23] = c[3] * u[23];
+    y[22] = c[3] * u[22];
+    y[21] = c[3] * u[21];
+    y[10] = fma(c[4], u[10], c[5] * u[17]);
+    y[17] = fma(c[4], u[17], c[5] * u[10]);
+    y[9] = fma(c[4], u[9], c[5] * u[20]);
+    y[20] = fma(c[4], u[20], c[5] * u[9]);
+    y[15] = fma(c[4], u[15], c[5] * u[19]);
+    y[19] = fma(c[4], u[19], c[5] * u[15]);
+    y[18] = fma(c[6], u[18], t);
+    y[16] = fma(c[6], u[16], t);
+    y[11] = fma(c[6], u[11], t);
 }
 
 // y = e * Ke u, general symmetric Ke.
@@ -369,6 +407,11 @@ __device__ __forceinline__ void scaleModes<float>(float (&u)[24], float e) {
         u[3 * m + 2] *= e;
     }
 }
+template <typename T>
+__device__ __forceinline__ void scaledKhat(T (&u)[24], T (&y)[24], const Ks<T>& k, T e) {
+    scaleModes<T>(u, e);
+    applyKhat<T>(u, y, k);
+}
 // nb = carry + (y_bottom + y_top); carry = y_bottom - y_top.
 template <typename T>
 __device__ __forceinline__ void foldCarry(const T (&y)[24], T (&carry)[12], T (&nb)[12]) {
@@ -427,15 +470,15 @@ enum MvOut : int { OUT_ANY = 0, OUT_CG = 1, OUT_TRUE = 2, OUT_CG_PX = 3 };
 // The march of one block of 32 x 8 threads over its node layers (MV_ZC;
 // `layers` in FP64, where the fixed-point product's blocks share the march): fills d0 and d1 (this
 // thread's dots) and returns the p buffer read (OUT_CG_PX).
-template <typename T, typename TC, int OUT>
-__device__ __forceinline__ int walshMarch(const MatvecArgs<T>& a, const Ks<TC>& kp, Scalars* S,
+template <typename T, typename TC, int OUT, typename KP>
+__device__ __forceinline__ int walshMarch(const MatvecArgs<T>& a, const KP& kp, Scalars* S,
                                            unsigned char* smemRaw, DotAcc<TC>& d0, DotAcc<TC>& d1,
                                           [[maybe_unused]] int layers = MV_ZC) {
     typedef Cvt<T, TC> C;
     TC* su = reinterpret_cast<TC*>(smemRaw);
     TC* sy = su + kSuElems;
     const Grid g = a.g;
-    const int zc = std::is_same<TC, double>::value ? layers : MV_ZC;
+    const int zc = layers;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int x0 = blockIdx.x * (MV_TX - 1), y0 = blockIdx.y * (MV_TY - 1), z0 = blockIdx.z * zc;
     const int zend = min(z0 + zc, g.nz);
@@ -580,8 +623,7 @@ __device__ __forceinline__ int walshMarch(const MatvecArgs<T>& a, const Ks<TC>& 
             TC uh[24], yh[24];
             const TC e = sc * TC(Ee);
             sumDiff12<TC>(qb, qt, uh);
-            scaleModes<TC>(uh, e);
-            applyKhat<TC>(uh, yh, kp);
+            scaledKhat<TC>(uh, yh, kp, e);
             foldCarry<TC>(yh, carry, nb);
         } else {
 #pragma unroll
