@@ -135,7 +135,8 @@ constexpr int PZR = 4;
 // (row 2cy-1, the block's first plane, the left x neighbour of lane 0) are
 // recomputed from rf and Ap.  checkDone = 2: run only in an iteration that
 // replaced the residual by the true one (restricting the replacement).
-template <typename T, bool UPD>
+// PZ: coarse layers a thread marches (1 on small grids: more blocks, shorter chains).
+template <typename T, bool UPD, int PZ = PZR>
 __global__ void __launch_bounds__(256) kRestrict2(Grid gf, Grid gc, const T* __restrict__ rf, const T* __restrict__ Ap,
                                                   T* __restrict__ rOut, T* __restrict__ rc, Scalars* S, RedBuf rb,
                                                   int checkDone) {
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(256) kRestrict2(Grid gf, Grid gc, const T* __r
 #pragma unroll
         for (int c = 0; c < 3; ++c) P[c] = row[1][c] + half * (row[0][c] + row[2][c]);
     };
-    const int cz0 = blockIdx.z * PZR, cz1 = min(gc.nz, cz0 + PZR);
+    const int cz0 = blockIdx.z * PZ, cz1 = min(gc.nz, cz0 + PZ);
     T Pm[3];
     planeSum(2 * cz0 - 1, false, Pm);
     for (int cz = cz0; cz < cz1; ++cz) {
@@ -225,6 +226,57 @@ __global__ void __launch_bounds__(256) kRestrict2(Grid gf, Grid gc, const T* __r
     if (UPD) {
         double v[1] = {acc.get()}, t[1];
         if (gridReduce<256, 1>(v, rb, t)) applyEpi(EPI_CONV, S, t[0], 0.0);
+    }
+}
+
+// The same restriction for FP64, whose operations bound it: y, then z, then x
+// (42 operations a coarse node instead of 54, and three shuffles a layer instead
+// of eighteen a plane).  A warp's first lane only supplies its right column to
+// the next one, so a warp restricts 31 coarse columns.
+__global__ void __launch_bounds__(256) kRestrict64(Grid gf, Grid gc, const double* __restrict__ rf,
+                                                   double* __restrict__ rc, const Scalars* S, int checkDone) {
+    if (checkDone && S->done) return;
+    const int lane = threadIdx.x, cx = (int)blockIdx.x * 31 + lane - 1, cy = blockIdx.y * 8 + threadIdx.y;
+    const bool out = lane > 0 && cx < gc.nx && cy < gc.ny;
+    const int fx0 = 2 * cx;
+    const bool ok0 = fx0 >= 0 && fx0 < gf.nx, ok1 = fx0 + 1 >= 0 && fx0 + 1 < gf.nx;
+    // y-weighted columns 2cx and 2cx + 1 of fine layer fz
+    auto plane = [&](int fz, double (&Y)[6]) {
+        double v[3][6];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            const int fy = 2 * cy - 1 + r;
+            const bool row = fy >= 0 && fy < gf.ny && fz >= 0 && fz < gf.nz;
+            const double* p = rf + 3 * (row ? gf.store(0, fy, fz) : 0) + 3 * fx0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                v[r][c] = row && ok0 ? p[c] : 0.0;
+                v[r][3 + c] = row && ok1 ? p[3 + c] : 0.0;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 6; ++c) Y[c] = fma(0.5, v[0][c] + v[2][c], v[1][c]);
+    };
+    const int cz0 = blockIdx.z * PZR, cz1 = min(gc.nz, cz0 + PZR);
+    double Ym[6];
+    plane(2 * cz0 - 1, Ym);
+    for (int cz = cz0; cz < cz1; ++cz) {
+        double Y0[6], Yp[6], Z[6];
+        plane(2 * cz, Y0);
+        plane(2 * cz + 1, Yp);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            Z[c] = fma(0.5, Ym[c] + Yp[c], Y0[c]);
+            Ym[c] = Yp[c];
+        }
+        double q[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) q[c] = fma(0.5, __shfl_up_sync(0xffffffffu, Z[3 + c], 1) + Z[3 + c], Z[c]);
+        if (out) {
+            double* o = rc + 3 * gc.store(cx, cy, cz);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) o[c] = q[c];
+        }
     }
 }
 
@@ -526,6 +578,92 @@ __device__ __forceinline__ void ldDiag12(const __half* p, float (&v)[12]) {
     }
 }
 
+// The 2x transfers of small grids, one thread per value (coarse value of the
+// restriction, fine value of the up-leg): every load of a thread is in flight at
+// once, where the marching kernels above wait for one plane after the other.
+// Same operations in the same order as kRestrict2 and kProlongFlat (FP32).  Measured,
+// FP64 / FP32 us, marching -> this: restriction from 33 x 17 x 17 nodes 18.4 / 6.7 ->
+// 6.2 / 4.2, from 65^3 18.5 / 8.2 -> 10.3 / 4.2, from 97^3 30.8 / 9.8 -> 22.6 / 6.2;
+// up-leg to 33 x 17 x 17 16.4 / 10.3 -> 9.2 / 8.3, to 49^3 24.3 / 12.3 -> 22.5 /
+// 12.4, to 65^3 35.0 / 14.4 -> 36.9 / 16.3: hence the limits, in fine nodes.
+constexpr int64_t kSmallRestrict = 1000000, kSmallProlong = 100000;
+
+template <typename T>
+__global__ void __launch_bounds__(256) kRestrictSmall(Grid gf, Grid gc, const T* __restrict__ rf, T* __restrict__ rc,
+                                                      const Scalars* S, int checkDone) {
+    if (checkDone && S->done) return;
+    if (checkDone == 2 && S->replStamp != S->matvecs) return;
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= 3 * (int)gc.nnode) return;
+    const int s = i / 3, c = i - 3 * s, cyz = s / gc.nx, cx = s - cyz * gc.nx, cz = cyz / gc.ny, cy = cyz - cz * gc.ny;
+    const T half = T(0.5);
+    T v[3][3][3];
+#pragma unroll
+    for (int dz = 0; dz < 3; ++dz)
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+                const int fx = 2 * cx - 1 + dx, fy = 2 * cy - 1 + dy, fz = 2 * cz - 1 + dz;
+                const bool ok = (unsigned)fx < (unsigned)gf.nx && (unsigned)fy < (unsigned)gf.ny && (unsigned)fz < (unsigned)gf.nz;
+                v[dz][dy][dx] = ok ? rf[3 * ((fz * gf.ny + fy) * gf.nx + fx) + c] : T(0);
+            }
+    T P[3];
+#pragma unroll
+    for (int dz = 0; dz < 3; ++dz) {
+        T row[3];
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy) row[dy] = v[dz][dy][1] + half * (v[dz][dy][0] + v[dz][dy][2]);
+        P[dz] = row[1] + half * (row[0] + row[2]);
+    }
+    rc[i] = P[1] + half * (P[0] + P[2]);
+}
+
+template <typename T, typename DT>
+__global__ void __launch_bounds__(256)
+    kProlongSmall(Grid gf, Grid gc, const T* __restrict__ zc, const T* __restrict__ rf, const DT* __restrict__ dinv,
+                  const uint8_t* __restrict__ flags, T* __restrict__ zf, double coef, int maskFixed,
+                  const T* __restrict__ aux, int epi, Scalars* S, RedBuf rb, int checkDone) {
+    if (checkDone && S->done) return;
+    DotAcc<T> d0, d1;
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < 3 * (int)gf.nnode; i += gridDim.x * 256) {
+        const int s = i / 3, c = i - 3 * s, fyz = s / gf.nx, fx = s - fyz * gf.nx, fz = fyz / gf.ny, fy = fyz - fz * gf.ny;
+        const T half = T(0.5);
+        const uint32_t fl = flags[s];
+        const T rv = rf[i], dv = (T)diagVal(dinv[i]);
+        // coarse corners; an odd position has a neighbour one up on its axis
+        const int px = 3 * (fx & 1), py = (fy & 1) ? 3 * gc.nx : 0, pz = (fz & 1) ? 3 * gc.nx * gc.ny : 0;
+        const T* b = zc + 3 * (((fz >> 1) * gc.ny + (fy >> 1)) * gc.nx + (fx >> 1)) + c;
+        T q[2][2][2];
+#pragma unroll
+        for (int z = 0; z < 2; ++z)
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) q[z][y][x] = b[(z ? pz : 0) + (y ? py : 0) + (x ? px : 0)];
+        const bool used = (fl & FLAG_USED) != 0;
+        const bool zero = !used || (maskFixed && (fl & FLAG_FIXED));
+        const T r = used ? rv : T(0);
+        T w[2][2];
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) w[y][x] = (fz & 1) ? half * (q[0][y][x] + q[1][y][x]) : q[0][y][x];
+        const T r0 = (fx & 1) ? half * (w[0][0] + w[0][1]) : w[0][0], r1 = (fx & 1) ? half * (w[1][0] + w[1][1]) : w[1][0];
+        const T pv = (fy & 1) ? half * (r0 + r1) : r0;
+        const T out = zero ? T(0) : pv + (T)coef * dv * r;
+        zf[i] = out;
+        if (epi != EPI_NONE) {
+            d0.add(r * out);
+            if (aux) d1.add(out * aux[i]);
+        }
+    }
+    if (epi != EPI_NONE) {
+        double v[2] = {d0.get(), d1.get()}, t[2];
+        if (gridReduce<256, 2>(v, rb, t)) applyEpi(epi, S, t[0], t[1]);
+    }
+}
+
 // DT: the type the inverse diagonal is stored in (T, or FP16 scaled so that
 // coef already carries the scale).
 template <typename T, typename DT>
@@ -578,14 +716,29 @@ __global__ void __launch_bounds__(256)
                 const bool zero = !used || (maskFixed && (fl & FLAG_FIXED));
                 const T* b = C + (ly >> 1) * cw + 3 * (fx >> 1);
                 T pv[3];
-                if (fx & 1) {
+                if constexpr (std::is_same<T, double>::value) {
+                    // FP64 operations bound this kernel: plain corner sums here, one power-of-two
+                    // weight in the multiply-add below (C holds the sum of two layers when fz is odd)
+                    const bool ox = fx & 1, oy = ly & 1;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) pv[c] = b[c];
+                    if (ox) {
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) pv[c] += b[c + 3];
+                    }
+                    if (oy) {
+                        const T* b1 = b + cw;
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) pv[c] += ox ? b1[c] + b1[c + 3] : b1[c];
+                    }
+                } else if (fx & 1) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) pv[c] = half * (b[c] + b[c + 3]);
                 } else {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) pv[c] = b[c];
                 }
-                if (ly & 1) {
+                if (std::is_same<T, float>::value && (ly & 1)) {
                     const T* b1 = b + cw;
                     if (fx & 1) {
 #pragma unroll
@@ -598,7 +751,13 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     const T r = used ? rv[3 * t + c] : T(0);
-                    const T out = zero ? T(0) : pv[c] + cf * dv[3 * t + c] * r;
+                    T out;
+                    if constexpr (std::is_same<T, double>::value) {
+                        const double wt = __hiloint2double((1023 - (int)zodd - (fx & 1) - (ly & 1)) << 20, 0);
+                        out = zero ? 0.0 : fma(wt, pv[c], cf * dv[3 * t + c] * r);
+                    } else {
+                        out = zero ? T(0) : pv[c] + cf * dv[3 * t + c] * r;
+                    }
                     if (epi != EPI_NONE) {
                         d0.add(r * out);
                         if (aux) d1.add(out * aux[3 * (n0 + t) + c]);
@@ -651,7 +810,8 @@ __global__ void __launch_bounds__(256)
             asm volatile("cp.async.wait_all;\n" ::: "memory");
             __syncthreads();
             if (zodd) {
-                for (int q = threadIdx.x; q < nstage; q += blockDim.x) C[q] = half * (C[q] + C[nstage + q]);
+                for (int q = threadIdx.x; q < nstage; q += blockDim.x)
+                    C[q] = std::is_same<T, double>::value ? C[q] + C[nstage + q] : half * (C[q] + C[nstage + q]);
                 __syncthreads();
             }
             staged = true;
@@ -1275,8 +1435,17 @@ int launchRestrict(const LaunchCtx& c, const Grid& gf, const Grid& gc, int div, 
         if constexpr (std::is_same<T, float>::value) {
             if ((c.tma & 1) && launchRestrictTma(c, gf, gc, rf, nullptr, nullptr, rc, checkDone)) return 1;
         }
-        dim3 grid((gc.nx + 31) / 32, (gc.ny + 7) / 8, (gc.nz + PZR - 1) / PZR);
-        kRestrict2<T, false><<<grid, block, 0, c.stream>>>(gf, gc, rf, nullptr, nullptr, rc, c.S, c.rb, checkDone);
+        if (gf.nnode <= kSmallRestrict) {
+            kRestrictSmall<T><<<(unsigned)((3 * gc.nnode + 255) / 256), 256, 0, c.stream>>>(gf, gc, rf, rc, c.S, checkDone);
+            return 1;
+        }
+        if constexpr (std::is_same<T, double>::value) {
+            dim3 grid((gc.nx + 30) / 31, (gc.ny + 7) / 8, (gc.nz + PZR - 1) / PZR);
+            kRestrict64<<<grid, block, 0, c.stream>>>(gf, gc, rf, rc, c.S, checkDone);
+        } else {
+            dim3 grid((gc.nx + 31) / 32, (gc.ny + 7) / 8, (gc.nz + PZR - 1) / PZR);
+            kRestrict2<T, false><<<grid, block, 0, c.stream>>>(gf, gc, rf, nullptr, nullptr, rc, c.S, c.rb, checkDone);
+        }
     }
     return 1;
 }
@@ -1284,8 +1453,11 @@ int launchRestrict(const LaunchCtx& c, const Grid& gf, const Grid& gc, int div, 
 int launchUpdateRestrict(const LaunchCtx& c, const Grid& gf, const Grid& gc, const float* rIn, const float* Ap,
                          float* rOut, float* rc) {
     if ((c.tma & 1) && launchRestrictTma(c, gf, gc, rIn, Ap, rOut, rc, 1)) return 1;
-    dim3 block(32, 8), grid((gc.nx + 31) / 32, (gc.ny + 7) / 8, (gc.nz + PZR - 1) / PZR);
-    kRestrict2<float, true><<<grid, block, 0, c.stream>>>(gf, gc, rIn, Ap, rOut, rc, c.S, c.rb, 1);
+    const bool small = gf.nnode <= kSmallRestrict;
+    const int pz = small ? 1 : PZR;
+    dim3 block(32, 8), grid((gc.nx + 31) / 32, (gc.ny + 7) / 8, (gc.nz + pz - 1) / pz);
+    auto kern = small ? kRestrict2<float, true, 1> : kRestrict2<float, true>;
+    kern<<<grid, block, 0, c.stream>>>(gf, gc, rIn, Ap, rOut, rc, c.S, c.rb, 1);
     return 1;
 }
 
@@ -1302,6 +1474,14 @@ int launchProlongSmooth(const LaunchCtx& c, const Grid& gf, const Grid& gc, int 
         const int vec = al(rf) && al(zf) && ((uintptr_t)flags & 3u) == 0 &&
                         (half ? ((uintptr_t)hd.d & 7u) == 0 : al(dinv));
         auto go = [&](auto kern, const auto* dptr, double cf) {
+            typedef typename std::remove_const<typename std::remove_pointer<decltype(dptr)>::type>::type DT;
+            if (gf.nnode <= kSmallProlong) {
+                // (few enough blocks for a cheap grid reduction)
+                const int64_t blocks = std::min<int64_t>((3 * gf.nnode + 255) / 256, 152 * 2);
+                kProlongSmall<T, DT><<<(unsigned)blocks, 256, 0, c.stream>>>(
+                    gf, gc, zc, rf, dptr, flags, zf, cf, maskFixed, aux, epi, c.S, c.rb, checkDone);
+                return;
+            }
             if (flatSmem > 48 * 1024)
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProlongFlatMaxSmem);
             kern<<<(unsigned)flatBlocksN, 256, flatSmem, c.stream>>>(gf, gc, zc, rf, dptr, flags, zf, cf, maskFixed, aux,
