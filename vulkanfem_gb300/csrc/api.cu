@@ -489,7 +489,7 @@ vfem_status ensureCoarse<float>(vfem_problem* p, bool vcycle) {
     const int64_t n = p->nc;
     __half* out = nullptr;
     float* full = nullptr;
-    CK(dalloc(&out, coarseTiles(n) * CT * CT));
+    CK(dalloc(&out, coarseHalfValues(n)));
     if (dalloc(&full, n * n + 1) != cudaSuccess) {
         cudaFree(out);
         return fail(VFEM_ERR_OUT_OF_MEMORY, "coarse inverse workspace");

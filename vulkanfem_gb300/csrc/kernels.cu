@@ -844,6 +844,66 @@ __global__ void __launch_bounds__(256) kGemv64(const double* __restrict__ K, int
     if (lane == 0) zc[freeDof[row]] = acc;
 }
 
+// Small coarsest systems in one kernel: the block gathers the right-hand side into
+// shared memory, a warp takes a row of the full inverse (FP64, or FP16 with rows
+// padded to 8 values) with independent partial sums.  Gathering, streaming and
+// reducing took two kernels in FP64 and three in mixed precision, each mostly
+// latency.  Measured, FP64 / mixed us, before -> this: n = 600 11.3 / 15.3 -> 6.3 /
+// 5.5, n = 1,944 18.5 / 17.5 -> 14.5 / 8.2 (FP64 FMAs alone 8), n = 2,700 25.7 / 19.6
+// -> 24.7 / 8.3, n = 3,993 44.2 / 18.0 -> 47.2 / 12.3, where FP64 is better off with
+// kGemv64 and the mixed form, at twice the bytes of the packed half, would soon be
+// with that: hence kSmallCoarse.
+__device__ __forceinline__ void smallRow(const __half* k, const float* b, int n, int lane, float (&acc)[4]) {
+    for (int j = 8 * lane; j < n; j += 256) {
+        const uint4 q = *reinterpret_cast<const uint4*>(k + j);
+        const float4 b0 = *reinterpret_cast<const float4*>(b + j), b1 = *reinterpret_cast<const float4*>(b + j + 4);
+        const float2 k0 = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
+        const float2 k1 = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
+        const float2 k2 = __half22float2(*reinterpret_cast<const __half2*>(&q.z));
+        const float2 k3 = __half22float2(*reinterpret_cast<const __half2*>(&q.w));
+        acc[0] = fmaf(k0.x, b0.x, fmaf(k2.x, b1.x, acc[0]));
+        acc[1] = fmaf(k0.y, b0.y, fmaf(k2.y, b1.y, acc[1]));
+        acc[2] = fmaf(k1.x, b0.z, fmaf(k3.x, b1.z, acc[2]));
+        acc[3] = fmaf(k1.y, b0.w, fmaf(k3.y, b1.w, acc[3]));
+    }
+}
+__device__ __forceinline__ void smallRow(const double* k, const double* b, int n, int lane, double (&acc)[4]) {
+    int j = lane;
+    for (; j + 96 < n; j += 128) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = fma(k[j + 32 * q], b[j + 32 * q], acc[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+        if (j + 32 * q < n) acc[q] = fma(k[j + 32 * q], b[j + 32 * q], acc[q]);
+}
+template <typename T, typename KT>
+__global__ void __launch_bounds__(256) kCoarseSmall(const KT* __restrict__ K, int n, int ld, T scale,
+                                                    const int32_t* __restrict__ freeDof, const T* __restrict__ rc,
+                                                    T* __restrict__ zc, const Scalars* S, int checkDone) {
+    if (checkDone && S->done) return;
+    __shared__ __align__(16) T b[kSmallCoarse<T> + 8];
+    for (int j = threadIdx.x; j < ((n + 7) & ~7); j += 256) b[j] = j < n ? rc[freeDof[j]] : T(0);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= n) return;
+    T acc[4] = {T(0), T(0), T(0), T(0)};
+    smallRow(K + (int64_t)row * ld, b, n, lane, acc);
+    T sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) zc[freeDof[row]] = sum * scale;
+}
+
+// FP16 rows of the full inverse for kCoarseSmall.
+__global__ void __launch_bounds__(256) kPackRowsHalf(const float* __restrict__ K, int n, int ld, float invScale,
+                                                     __half* __restrict__ rows) {
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n * ld; i += gridDim.x * 256) {
+        const int r = i / ld, c = i - r * ld;
+        rows[i] = __float2half_rn(c < n ? K[(int64_t)r * n + c] * invScale : 0.0f);
+    }
+}
+
 // ---- coarsest solve of the mixed-precision cycle: y = Kinv b with the
 // symmetric inverse stored once, in FP16.  Kinv is kept as the lower block
 // triangle of 64 x 64 tiles (tile (I, J <= I) at index I (I + 1) / 2 + J,
@@ -1531,6 +1591,16 @@ template <typename T>
 int launchCoarseSolve(const LaunchCtx& c, CoarseInv<T> Kinv, int64_t n, const int32_t* freeDof, const T* rc, T* tmp,
                       T* part, T* zc, int checkDone) {
     if (n <= 0) return 0;
+    if (n <= kSmallCoarse<T>) {
+        const unsigned blocks = (unsigned)((n + 7) / 8);
+        if constexpr (std::is_same<T, double>::value)
+            kCoarseSmall<double, double><<<blocks, 256, 0, c.stream>>>(Kinv.K, (int)n, (int)n, 1.0, freeDof, rc, zc, c.S,
+                                                                       checkDone);
+        else
+            kCoarseSmall<float, __half><<<blocks, 256, 0, c.stream>>>(Kinv.K, (int)n, (int)coarseLd(n), Kinv.scale,
+                                                                      freeDof, rc, zc, c.S, checkDone);
+        return 1;
+    }
     kCoarseGather<T><<<(int)((n + 255) / 256), 256, 0, c.stream>>>(n, freeDof, rc, tmp, c.S, checkDone);
     if constexpr (std::is_same<T, double>::value) {
         kGemv64<<<(int)((n * 32 + 255) / 256), 256, 0, c.stream>>>(Kinv.K, n, tmp, freeDof, zc, c.S, checkDone);
@@ -1559,6 +1629,10 @@ int launchMaxDiag(cudaStream_t s, const float* K, int64_t n, float* out) {
 }
 
 int launchPackSymHalf(cudaStream_t s, const float* K, int64_t n, float invScale, __half* tiles) {
+    if (n <= kSmallCoarse<float>) {
+        kPackRowsHalf<<<flatBlocks(n * coarseLd(n)), NT, 0, s>>>(K, (int)n, (int)coarseLd(n), invScale, tiles);
+        return 1;
+    }
     const int64_t nb = coarseBlocks(n);
     kPackSymHalf<<<flatBlocks(symTileCount(nb) * CT * CT), NT, 0, s>>>(K, n, nb, invScale, tiles);
     return 1;

@@ -10,6 +10,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "vfem_internal.h"
 
 namespace vfem {
@@ -180,6 +182,12 @@ int launchProlongAdd(const LaunchCtx& c, const Grid& gf, const Grid& gc, int div
 constexpr int CT = 64;
 inline int64_t coarseBlocks(int64_t n) { return (n + CT - 1) / CT; }
 inline int64_t coarseTiles(int64_t n) { return coarseBlocks(n) * (coarseBlocks(n) + 1) / 2; }
+// Up to kSmallCoarse free DOFs one kernel does it all (kCoarseSmall) and the mixed
+// inverse is n FP16 rows of coarseLd(n) values instead.
+template <typename T>
+constexpr int kSmallCoarse = std::is_same<T, double>::value ? 3000 : 4096;
+inline int64_t coarseLd(int64_t n) { return (n + 7) & ~(int64_t)7; }
+inline int64_t coarseHalfValues(int64_t n) { return n <= kSmallCoarse<float> ? n * coarseLd(n) : coarseTiles(n) * CT * CT; }
 template <typename T>
 struct CoarseInv;
 template <>
@@ -200,7 +208,7 @@ int launchToHalf(cudaStream_t s, const float* x, int64_t n, float invScale, __ha
 // *out = the largest diagonal entry of a row-major n x n matrix.
 int launchMaxDiag(cudaStream_t s, const float* K, int64_t n, float* out);
 // Pack a full symmetric row-major n x n matrix, times invScale, into
-// coarseTiles(n) FP16 tiles.
+// coarseTiles(n) FP16 tiles (coarseHalfValues(n) values).
 int launchPackSymHalf(cudaStream_t s, const float* K, int64_t n, float invScale, __half* tiles);
 
 // CG vector updates on flat arrays of length n.
