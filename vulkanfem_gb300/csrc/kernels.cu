@@ -559,7 +559,6 @@ __device__ __forceinline__ void cpAsync(T* dst, const T* src) {
 // Inverse-diagonal values of a chunk: T, or FP16 (scaled; 8-byte loads).
 __device__ __forceinline__ float diagVal(__half h) { return __half2float(h); }
 __device__ __forceinline__ float diagVal(float v) { return v; }
-__device__ __forceinline__ double diagVal(double v) { return v; }
 template <typename T>
 __device__ __forceinline__ void ldDiag12(const T* p, T (&v)[12]) {
 #pragma unroll
@@ -579,13 +578,13 @@ __device__ __forceinline__ void ldDiag12(const __half* p, float (&v)[12]) {
 }
 
 // The 2x transfers of small grids, one thread per value (coarse value of the
-// restriction, fine value of the up-leg): every load of a thread is in flight at
+// restriction, fine value of the FP32 up-leg): every load of a thread is in flight at
 // once, where the marching kernels above wait for one plane after the other.
-// Same operations in the same order as kRestrict2 and kProlongFlat (FP32).  Measured,
+// Same operations in the same order as kRestrict2 and kProlongFlat.  Measured,
 // FP64 / FP32 us, marching -> this: restriction from 33 x 17 x 17 nodes 18.4 / 6.7 ->
 // 6.2 / 4.2, from 65^3 18.5 / 8.2 -> 10.3 / 4.2, from 97^3 30.8 / 9.8 -> 22.6 / 6.2;
-// up-leg to 33 x 17 x 17 16.4 / 10.3 -> 9.2 / 8.3, to 49^3 24.3 / 12.3 -> 22.5 /
-// 12.4, to 65^3 35.0 / 14.4 -> 36.9 / 16.3: hence the limits, in fine nodes.
+// FP32 up-leg to 33 x 17 x 17 10.3 -> 8.3, to 49^3 12.3 -> 12.4, to 65^3 14.4 -> 16.3:
+// hence the limits, in fine nodes.
 constexpr int64_t kSmallRestrict = 1000000, kSmallProlong = 100000;
 
 template <typename T>
@@ -716,29 +715,14 @@ __global__ void __launch_bounds__(256)
                 const bool zero = !used || (maskFixed && (fl & FLAG_FIXED));
                 const T* b = C + (ly >> 1) * cw + 3 * (fx >> 1);
                 T pv[3];
-                if constexpr (std::is_same<T, double>::value) {
-                    // FP64 operations bound this kernel: plain corner sums here, one power-of-two
-                    // weight in the multiply-add below (C holds the sum of two layers when fz is odd)
-                    const bool ox = fx & 1, oy = ly & 1;
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) pv[c] = b[c];
-                    if (ox) {
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) pv[c] += b[c + 3];
-                    }
-                    if (oy) {
-                        const T* b1 = b + cw;
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) pv[c] += ox ? b1[c] + b1[c + 3] : b1[c];
-                    }
-                } else if (fx & 1) {
+                if (fx & 1) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) pv[c] = half * (b[c] + b[c + 3]);
                 } else {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) pv[c] = b[c];
                 }
-                if (std::is_same<T, float>::value && (ly & 1)) {
+                if (ly & 1) {
                     const T* b1 = b + cw;
                     if (fx & 1) {
 #pragma unroll
@@ -751,13 +735,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     const T r = used ? rv[3 * t + c] : T(0);
-                    T out;
-                    if constexpr (std::is_same<T, double>::value) {
-                        const double wt = __hiloint2double((1023 - (int)zodd - (fx & 1) - (ly & 1)) << 20, 0);
-                        out = zero ? 0.0 : fma(wt, pv[c], cf * dv[3 * t + c] * r);
-                    } else {
-                        out = zero ? T(0) : pv[c] + cf * dv[3 * t + c] * r;
-                    }
+                    const T out = zero ? T(0) : pv[c] + cf * dv[3 * t + c] * r;
                     if (epi != EPI_NONE) {
                         d0.add(r * out);
                         if (aux) d1.add(out * aux[3 * (n0 + t) + c]);
@@ -811,7 +789,7 @@ __global__ void __launch_bounds__(256)
             __syncthreads();
             if (zodd) {
                 for (int q = threadIdx.x; q < nstage; q += blockDim.x)
-                    C[q] = std::is_same<T, double>::value ? C[q] + C[nstage + q] : half * (C[q] + C[nstage + q]);
+                    C[q] = half * (C[q] + C[nstage + q]);
                 __syncthreads();
             }
             staged = true;
@@ -823,6 +801,151 @@ __global__ void __launch_bounds__(256)
     if (epi != EPI_NONE) {
         double v[2] = {d0.get(), d1.get()}, t[2];
         if (gridReduce<256, 2>(v, rb, t)) applyEpi(epi, S, t[0], t[1]);
+    }
+}
+
+// x * 2^-k (k = 0 .. 3) without an FP64 operation.
+__device__ __forceinline__ double scaleDown(double x, int k) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
+    if (e - 4u < 0x7ffu - 4u) return __hiloint2double(hi - (k << 20), lo);
+    if (((hi & 0x7fffffff) | lo) == 0) return x;
+    return x * __hiloint2double((1023 - k) << 20, 0);  // subnormal result, infinity or NaN
+}
+
+// The 2x up-leg in FP64, flat like kProlongFlat.  FP64 operations (1.7 a clock and SM)
+// bound it, so a value takes about 4 of them: the sums over y are made once per coarse
+// column in shared memory (C: the rows summed over z; behind them, once the layer above
+// is summed in, the odd fine rows), a warp adds over x only where a lane needs it, the
+// weight 2^-k is an integer subtraction from the exponent, and dv * r takes one multiply
+// and one multiply-add.  (kProlongFlat's corner sums, up to 7 operations where a warp
+// spans two rows.)  A thread takes 2 nodes (4: 617 instead of 580 us to 257^3).
+// Measured, us, kProlongFlat in FP64 -> this: up-leg to 257^3 757 -> 580, 129^3 149 ->
+// 95, 97^3 70.5 -> 47, 65^3 35 -> 22.6, 34^3 14.5 -> 11.3; FP64 operations alone 405 and
+// bytes 193 to 257^3.  Rows and threads of a block: to 65^3 16 rows x 256 threads 26.8,
+// 8 x 128 22.6, 4 x 128 24.9; to 97^3 47, 51, 55; to 34^3 12.8, 12.5, 11.3.
+template <int ROWS, int NTH>
+__global__ void __launch_bounds__(NTH)
+    kProlong64(Grid gf, Grid gc, const double* __restrict__ zc, const double* __restrict__ rf,
+               const double* __restrict__ dinv, const uint8_t* __restrict__ flags, double* __restrict__ zf, double coef,
+               int maskFixed, const double* __restrict__ aux, int epi, int vec, float invNx, Scalars* S, RedBuf rb,
+               int checkDone) {
+    constexpr int CH = 2;  // nodes a thread takes at a time
+    if (checkDone && S->done) return;
+    extern __shared__ __align__(16) unsigned char prolongSmem[];
+    double* C = reinterpret_cast<double*>(prolongSmem);  // coarse rows; then the layer above, later the row sums
+    const int groups = (gf.ny + ROWS - 1) / ROWS;
+    const int fz = blockIdx.x / groups;
+    const int fy0 = (blockIdx.x - fz * groups) * ROWS, fy1 = min(gf.ny, fy0 + ROWS);
+    const int cw = 3 * gc.nx, cy0 = fy0 >> 1, cz = fz >> 1;
+    const int nstage = min(ROWS / 2 + 1, gc.ny - cy0) * cw;
+    const int nsum = ((fy1 - fy0) >> 1) * cw;  // odd fine rows
+    const bool zodd = fz & 1;
+    {
+        const double* src = zc + 3 * gc.store(0, cy0, cz);
+        const int64_t up = 3 * ((int64_t)gc.nx * gc.ny);
+        for (int j = threadIdx.x; j < nstage; j += NTH) {
+            cpAsync(C + j, src + j);
+            if (zodd) cpAsync(C + nstage + j, src + up + j);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    const int64_t nBeg = gf.store(0, fy0, fz);
+    const int nb = (fy1 - fy0) * gf.nx;
+    const int64_t j1 = (nBeg + nb + CH - 1) / CH;
+    double d0 = 0.0, d1 = 0.0;
+    bool staged = false;
+    for (int64_t j = nBeg / CH + threadIdx.x;; j += NTH) {
+        const bool have = j < j1;
+        const int64_t n0 = CH * j;
+        const int ln0 = (int)(n0 - nBeg);  // 1 - CH .. nb - 1
+        const bool full = vec && ln0 >= 0 && ln0 + CH <= nb;
+        double rv[3 * CH], dv[3 * CH];
+        uint32_t fl4 = 0;
+        if (have) {
+            if (full) {
+#pragma unroll
+                for (int q = 0; q < 3 * CH; q += 2) {
+                    const double2 a = *reinterpret_cast<const double2*>(rf + 3 * n0 + q);
+                    const double2 b = *reinterpret_cast<const double2*>(dinv + 3 * n0 + q);
+                    rv[q] = a.x; rv[q + 1] = a.y;
+                    dv[q] = b.x; dv[q + 1] = b.y;
+                }
+            } else {
+#pragma unroll
+                for (int t = 0; t < CH; ++t) {
+                    const bool in = ln0 + t >= 0 && ln0 + t < nb;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        rv[3 * t + c] = in ? rf[3 * (n0 + t) + c] : 0.0;
+                        dv[3 * t + c] = in ? dinv[3 * (n0 + t) + c] : 0.0;
+                    }
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < CH; ++t)
+                if (ln0 + t >= 0 && ln0 + t < nb) fl4 |= (uint32_t)flags[n0 + t] << (8 * t);
+        }
+        if (!staged) {
+            // every thread passes here once, after issuing its first chunk's loads
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+            __syncthreads();
+            if (zodd) {
+                for (int q = threadIdx.x; q < nstage; q += NTH) C[q] += C[nstage + q];
+                __syncthreads();
+            }
+            for (int q = threadIdx.x; q < nsum; q += NTH) C[nstage + q] = C[q] + C[q + cw];
+            __syncthreads();
+            staged = true;
+        }
+        if (!have) break;
+        // (ly, fx) of the chunk's first node; fx < 0 for nodes before the range
+        const int lnc = max(ln0, 0);
+        int ly = __float2int_rz(((float)lnc + 0.5f) * invNx);
+        int fx = lnc - ly * gf.nx;
+        if (fx < 0) { --ly; fx += gf.nx; }
+        if (fx >= gf.nx) { ++ly; fx -= gf.nx; }
+        fx -= lnc - ln0;
+#pragma unroll
+        for (int t = 0; t < CH; ++t) {
+            const bool in = full || (ln0 + t >= 0 && ln0 + t < nb);
+            if (in) {
+                const uint32_t fl = (fl4 >> (8 * t)) & 0xffu;
+                const bool used = (fl & FLAG_USED) != 0;
+                const bool zero = !used || (maskFixed && (fl & FLAG_FIXED));
+                const double* b = C + ((ly & 1) ? nstage : 0) + (ly >> 1) * cw + 3 * (fx >> 1);
+                const int k = (int)zodd + (ly & 1) + (fx & 1);
+                double pv[3] = {b[0], b[1], b[2]};
+                if (fx & 1) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) pv[c] += b[c + 3];
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const double r = used ? rv[3 * t + c] : 0.0;
+                    const double out = zero ? 0.0 : fma(coef, dv[3 * t + c] * r, scaleDown(pv[c], k));
+                    if (epi != EPI_NONE) {
+                        d0 = fma(r, out, d0);
+                        if (aux) d1 = fma(out, aux[3 * (n0 + t) + c], d1);
+                    }
+                    rv[3 * t + c] = out;
+                    if (!full) zf[3 * (n0 + t) + c] = out;
+                }
+            }
+            if (++fx == gf.nx) {
+                fx = 0;
+                ++ly;
+            }
+        }
+        if (full) {
+#pragma unroll
+            for (int q = 0; q < 3 * CH; q += 2)
+                *reinterpret_cast<double2*>(zf + 3 * n0 + q) = make_double2(rv[q], rv[q + 1]);
+        }
+    }
+    if (epi != EPI_NONE) {
+        double v[2] = {d0, d1}, t[2];
+        if (gridReduce<NTH, 2>(v, rb, t)) applyEpi(epi, S, t[0], t[1]);
     }
 }
 
@@ -1533,6 +1656,7 @@ int launchProlongSmooth(const LaunchCtx& c, const Grid& gf, const Grid& gc, int 
         const bool half = std::is_same<T, float>::value && hd.d != nullptr;
         const int vec = al(rf) && al(zf) && ((uintptr_t)flags & 3u) == 0 &&
                         (half ? ((uintptr_t)hd.d & 7u) == 0 : al(dinv));
+        // (FP32)
         auto go = [&](auto kern, const auto* dptr, double cf) {
             typedef typename std::remove_const<typename std::remove_pointer<decltype(dptr)>::type>::type DT;
             if (gf.nnode <= kSmallProlong) {
@@ -1556,7 +1680,26 @@ int launchProlongSmooth(const LaunchCtx& c, const Grid& gf, const Grid& gc, int 
                 return 1;
             }
         }
-        go(kProlongFlat<T, T>, dinv, coef);
+        if constexpr (std::is_same<T, double>::value) {
+            auto go64 = [&](auto rowsTag, auto nthTag) {
+                constexpr int ROWS = decltype(rowsTag)::value, NTH = decltype(nthTag)::value;
+                const int64_t blocks = (int64_t)((gf.ny + ROWS - 1) / ROWS) * gf.nz;
+                const size_t smem = 2 * sizeof(double) * (ROWS / 2 + 1) * 3 * (size_t)gc.nx;
+                if (smem > 48 * 1024)
+                    cudaFuncSetAttribute(kProlong64<ROWS, NTH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kProlongFlatMaxSmem);
+                kProlong64<ROWS, NTH><<<(unsigned)blocks, NTH, smem, c.stream>>>(
+                    gf, gc, zc, rf, dinv, flags, zf, coef, maskFixed, aux, epi, vec, 1.0f / gf.nx, c.S, c.rb, checkDone);
+            };
+            // 16 rows where that gives 4 blocks an SM, else 8 where those give 2, else 4
+            using std::integral_constant;
+            const auto blocksOf = [&](int rows) { return (int64_t)((gf.ny + rows - 1) / rows) * gf.nz; };
+            if (blocksOf(16) >= 4 * 152) go64(integral_constant<int, 16>(), integral_constant<int, 256>());
+            else if (blocksOf(8) >= 2 * 152) go64(integral_constant<int, 8>(), integral_constant<int, 128>());
+            else go64(integral_constant<int, 4>(), integral_constant<int, 128>());
+        } else {
+            go(kProlongFlat<float, float>, dinv, coef);
+        }
     } else if (div == 2) {
         // grids beyond the flat kernel's block or shared-memory limits (over ~1000^3 nodes)
         dim3 cgrid((gc.nx + 31) / 32, (gc.ny + 7) / 8, (gc.nz + PZC - 1) / PZC);
