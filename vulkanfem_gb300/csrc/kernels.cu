@@ -1507,6 +1507,13 @@ inline int flatBlocks(int64_t n) {
     return (int)b;
 }
 
+// Blocks of the vector updates that also reduce (4 values a thread and step): each block's
+// sum costs five FP64 additions a warp and a partial that the last block reads, so 3 an
+// SM (8 for kUpdateR on large grids: 103 us to 257^3 instead of 110) and none without work.  kUpdateXR in FP64 with 8 an SM (one thread a value) / 4 / 3 /
+// 2, us: 65^3 nodes 16.7 / 14.4 / 13.3 / 12.4, 129^3 61 / 56 / 54 / 58, 257^3 399 / 413 /
+// 369 / 385; kUpdateR to 65^3 14.4 -> 9.1.
+inline int reduceBlocks(int64_t n, int perSm) { return (int)std::min<int64_t>((n / 4 + NT) / NT, 152 * perSm); }
+
 inline dim3 nodeGrid(const Grid& g) {
     return dim3((g.nx + 31) / 32, (g.ny + 7) / 8, (g.nz + PZ - 1) / PZ);
 }
@@ -1783,7 +1790,7 @@ int launchPackSymHalf(cudaStream_t s, const float* K, int64_t n, float invScale,
 
 template <typename TX, typename TV>
 int launchUpdateXR(const LaunchCtx& c, int64_t n, TX* x, TV* r, const TV* p, const TV* Ap) {
-    kUpdateXR<TX, TV><<<flatBlocks(n), NT, 0, c.stream>>>(n, x, r, p, Ap, c.S, c.rb);
+    kUpdateXR<TX, TV><<<reduceBlocks(n, 3), NT, 0, c.stream>>>(n, x, r, p, Ap, c.S, c.rb);
     return 1;
 }
 
@@ -1794,7 +1801,7 @@ int launchFlushX(const LaunchCtx& c, int64_t n, double* x64, float* x32, const f
 }
 
 int launchUpdateR(const LaunchCtx& c, int64_t n, float* r, const float* Ap) {
-    kUpdateR<<<flatBlocks(n), NT, 0, c.stream>>>(n, r, Ap, c.S, c.rb);
+    kUpdateR<<<reduceBlocks(n, n > 4 * NT * 152 * 8 ? 8 : 3), NT, 0, c.stream>>>(n, r, Ap, c.S, c.rb);
     return 1;
 }
 
