@@ -34,3 +34,17 @@ def test_two_level_cycle(shape, n):
         tol = 8 * cond * eps + (4 * 2.0 ** -11 if precision == "mixed" else 0.0)
         assert np.linalg.norm(z - want) <= tol * scale
     A.close()
+
+
+def test_even_split_of_the_tiles():
+    """6,552 coarse free DOFs: 5,356 tiles of the packed FP16 inverse over 1,824 warps, ranges
+    that end within and across row blocks.  Mixed against FP64: 2^-11 of the FP16 inverse and
+    smoother and the FP32 inversion, whose condition number here is about 1e4."""
+    d = domains.cantilever(28, 24, 22, 2)
+    A = api.assembleSystemMatrix(d.voxels, domains.hex8_stiffness(), d.fixed, 2)
+    assert A.coarse_free_dofs == 6552
+    r = np.random.default_rng(0).random(A.rows())
+    z = api.MultigridPreconditioner(A).solve(r)
+    zm = api.MultigridPreconditioner(A, precision="mixed").solve(r)
+    assert np.linalg.norm(zm - z) <= 8 * 2.0 ** -11 * np.linalg.norm(z)
+    A.close()

@@ -1036,9 +1036,8 @@ __global__ void __launch_bounds__(256) kPackRowsHalf(const float* __restrict__ K
 // SPD inverse), so every entry above 2^-10 of that maximum keeps FP16's 11-bit
 // significand; the products accumulate in FP32.  The rounding is symmetric, so
 // the coarse operator stays symmetric.  kSymRuns streams runs of consecutive
-// tiles of one row block: it reads each tile once, accumulates K_IJ b_J for
-// y_I over the run and writes K_IJ^T b_I (for y_J, off-diagonal tiles) per
-// tile; kSymRunsReduce sums the partials per row block in a fixed order
+// tiles: it reads each tile once, accumulates K_IJ b_J for y_I over a row block
+// and writes K_IJ^T b_I (for y_J, off-diagonal tiles) per tile; kSymRunsReduce sums the partials per row block in a fixed order
 // (deterministic, no atomics) and applies the scale.
 __host__ __device__ inline int64_t symTileCount(int64_t nb) { return nb * (nb + 1) / 2; }
 // Tile index -> (I, J): FP32 square root, corrected exactly in integers (an FP64
@@ -1095,94 +1094,108 @@ __global__ void __launch_bounds__(1024) kMaxDiag(const float* __restrict__ K, in
     }
 }
 
-// Runs of tiles: row block I's tiles are contiguous in memory; a run is up to
-// SYM_RUN consecutive tiles (I, J0 .. J0 + SYM_RUN - 1) of one row, and one
-// block streams a run.  Runs of row I: ceil((I + 1) / SYM_RUN), numbered in row
-// order from symRunStart(I).
-constexpr int SYM_RUN = 16;
-__host__ __device__ inline int64_t symRunStart(int64_t I) {
-    const int64_t a = I / SYM_RUN, b = I % SYM_RUN;
-    return SYM_RUN * a * (a + 1) / 2 + b * (a + 1);
+// The tiles, numbered row block after row block, are split evenly over the warps that fit
+// on the chip: warp w of W takes tiles symStart(w) .. symStart(w + 1) - 1.  Where a row
+// block ends within its range, or the range ends, it writes that row block's sums.
+constexpr int SYM_WARPS = 4, SYM_PER_SM = 3, SYM_BLOCKS = SYM_PER_SM * 152;
+__host__ __device__ inline int64_t symWarps(int64_t tiles) {
+    return tiles < (int64_t)SYM_WARPS * SYM_BLOCKS ? tiles : (int64_t)SYM_WARPS * SYM_BLOCKS;
 }
+__host__ __device__ inline int64_t symStart(int64_t w, int64_t tiles, int64_t warps) { return w * tiles / warps; }
 
-// One run per block, 16 x 16 threads each holding a 4 x 4 sub-block of every
-// tile (four 8-byte row loads).  The row sums K_IJ b_J accumulate in registers across the
-// run and reduce once (partial of the run at part[run][0..63]); the column sums
-// K_IJ^T b_I of each off-diagonal tile reduce over the row groups through a
-// double-buffered shared array (one barrier per tile) into part[tile][64..127].
-// The next tile's values are loaded while the current one is used.
-__global__ void __launch_bounds__(256) kSymRuns(const __half* __restrict__ tiles, const float* __restrict__ b,
-                                                float* __restrict__ part, int64_t nb, const Scalars* S,
-                                                int checkDone) {
+// A lane holds 8 columns of every fourth row of a tile (16 loads of 16 bytes) and replaces
+// each by the next tile's as soon as it is used, so a whole tile per warp is in flight and
+// nothing waits on a barrier.  The row sums K_IJ b_J stay in registers until the row block
+// ends (part[its last tile][0..63]); the column sums K_IJ^T b_I of an off-diagonal tile
+// need two shuffles a value (part[tile][64..127]).  DRAM bound: 183 MB for n = 13,500 in
+// 32.6 us (5.6 TB/s); with gather and reduction 47.9 us, where blocks of 256 threads on
+// runs of 16 tiles with a barrier per tile took 55.3 and warps on runs of 8 (one wave and
+// a half of blocks) 47.5; for n = 4,752 18.1, 21.7 and 19.5.  Two blocks an SM 49.2.
+__global__ void __launch_bounds__(32 * SYM_WARPS, SYM_PER_SM)
+    kSymRuns(const __half* __restrict__ tiles, const float* __restrict__ b, float* __restrict__ part, int64_t nb,
+             const Scalars* S, int checkDone) {
     if (checkDone && S->done) return;
-    __shared__ float colp[2][8][CT];
-    const int64_t run = blockIdx.x;
-    int64_t lo = 0, hi = nb - 1;  // largest I with symRunStart(I) <= run
-    while (lo < hi) {
-        const int64_t mid = (lo + hi + 1) / 2;
-        if (symRunStart(mid) <= run) lo = mid;
-        else hi = mid - 1;
+    const int64_t T = nb * (nb + 1) / 2, W = symWarps(T), w = blockIdx.x * (int64_t)SYM_WARPS + (threadIdx.x >> 5);
+    if (w >= W) return;
+    int64_t t = symStart(w, T, W);
+    const int64_t tEnd = symStart(w + 1, T, W);
+    // row block of the first tile: the largest I with I (I + 1) / 2 <= t
+    int I = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while ((int64_t)I * (I + 1) / 2 > t) --I;
+    while ((int64_t)(I + 1) * (I + 2) / 2 <= t) ++I;
+    int J = (int)(t - (int64_t)I * (I + 1) / 2);
+    const int lane = threadIdx.x & 31, tc = lane & 7, tr = lane >> 3;
+    float bI[16], rs[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        bI[i] = b[I * CT + 4 * i + tr];
+        rs[i] = 0.f;
     }
-    const int64_t I = lo;
-    const int64_t J0 = (run - symRunStart(I)) * SYM_RUN, J1 = min(J0 + SYM_RUN, I + 1);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int tc = lane & 15, tr = warp * 2 + (lane >> 4);
-    const int64_t rowTile = I * (I + 1) / 2;
-    float bI[4];
+    const uint4* K = reinterpret_cast<const uint4*>(tiles + t * (CT * CT)) + lane;
+    uint4 k[16];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) bI[j] = b[I * CT + 4 * tr + j];
-    float rs[4] = {0.f, 0.f, 0.f, 0.f};
-    uint2 nxt[4];
-    auto loadTile = [&](int64_t J, uint2 (&raw)[4]) {
-        const __half* K = tiles + (rowTile + J) * (CT * CT);
+    for (int i = 0; i < 16; ++i) k[i] = K[32 * i];
+    const float4* bp = reinterpret_cast<const float4*>(b + J * CT + 8 * tc);
+    float4 q0 = bp[0], q1 = bp[1];
+    for (; t < tEnd; ++t) {
+        const float2 bj[4] = {make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y),
+                              make_float2(q1.z, q1.w)};
+        const bool more = t + 1 < tEnd, diagonal = J == I;
+        K += CT * CT / 8;
+        J = diagonal ? 0 : J + 1;
+        if (more) {
+            bp = reinterpret_cast<const float4*>(b + J * CT + 8 * tc);
+            q0 = bp[0];
+            q1 = bp[1];
+        }
+        float2 cs[4] = {};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) raw[i] = *reinterpret_cast<const uint2*>(K + (4 * tr + i) * CT + 4 * tc);
-    };
-    loadTile(J0, nxt);
-    int buf = 0;
-    for (int64_t J = J0; J < J1; ++J) {
-        uint2 cur[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) cur[i] = nxt[i];
-        if (J + 1 < J1) loadTile(J + 1, nxt);
-        const float2 bJ01 = make_float2(b[J * CT + 4 * tc], b[J * CT + 4 * tc + 1]);
-        const float2 bJ23 = make_float2(b[J * CT + 4 * tc + 2], b[J * CT + 4 * tc + 3]);
-        float2 cs01 = make_float2(0.f, 0.f), cs23 = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 k01 = __half22float2(*reinterpret_cast<const __half2*>(&cur[i].x));
-            const float2 k23 = __half22float2(*reinterpret_cast<const __half2*>(&cur[i].y));
-            const float2 r2 = __ffma2_rn(k23, bJ23, __fmul2_rn(k01, bJ01));
+        for (int i = 0; i < 16; ++i) {
+            const float2 k0 = __half22float2(*reinterpret_cast<const __half2*>(&k[i].x));
+            const float2 k1 = __half22float2(*reinterpret_cast<const __half2*>(&k[i].y));
+            const float2 k2 = __half22float2(*reinterpret_cast<const __half2*>(&k[i].z));
+            const float2 k3 = __half22float2(*reinterpret_cast<const __half2*>(&k[i].w));
+            if (more) k[i] = K[32 * i];
+            const float2 r2 = __ffma2_rn(k3, bj[3], __ffma2_rn(k2, bj[2], __ffma2_rn(k1, bj[1], __fmul2_rn(k0, bj[0]))));
             rs[i] += r2.x + r2.y;
             const float2 bi = make_float2(bI[i], bI[i]);
-            cs01 = __ffma2_rn(k01, bi, cs01);
-            cs23 = __ffma2_rn(k23, bi, cs23);
+            cs[0] = __ffma2_rn(k0, bi, cs[0]);
+            cs[1] = __ffma2_rn(k1, bi, cs[1]);
+            cs[2] = __ffma2_rn(k2, bi, cs[2]);
+            cs[3] = __ffma2_rn(k3, bi, cs[3]);
         }
-        if (J != I) {  // the same for the whole block
-            float cs[4] = {cs01.x, cs01.y, cs23.x, cs23.y};
+        if (!diagonal) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) cs[j] += __shfl_xor_sync(0xffffffffu, cs[j], 16);
-            if (lane < 16) {
+            for (int o = 8; o <= 16; o <<= 1)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) colp[buf][warp][4 * tc + j] = cs[j];
+                for (int j = 0; j < 4; ++j) {
+                    cs[j].x += __shfl_xor_sync(0xffffffffu, cs[j].x, o);
+                    cs[j].y += __shfl_xor_sync(0xffffffffu, cs[j].y, o);
+                }
+            if (tr == 0) {
+                float4* out = reinterpret_cast<float4*>(part + t * (2 * CT) + CT + 8 * tc);
+                out[0] = make_float4(cs[0].x, cs[0].y, cs[1].x, cs[1].y);
+                out[1] = make_float4(cs[2].x, cs[2].y, cs[3].x, cs[3].y);
             }
-            __syncthreads();
-            if (threadIdx.x < CT) {
-                float sum = 0.f;
-#pragma unroll
-                for (int w = 0; w < 8; ++w) sum += colp[buf][w][threadIdx.x];
-                part[(rowTile + J) * (2 * CT) + CT + threadIdx.x] = sum;
-            }
-            buf ^= 1;
         }
-    }
+        if (diagonal || !more) {
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1)
+            for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], o);
-    if (tc == 0) {
+                for (int i = 0; i < 16; ++i) rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], o);
+            if (tc == 0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) part[run * (2 * CT) + 4 * tr + i] = rs[i];
+                for (int i = 0; i < 16; ++i) part[t * (2 * CT) + 4 * i + tr] = rs[i];
+            }
+            ++I;
+            if (more) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    bI[i] = b[I * CT + 4 * i + tr];
+                    rs[i] = 0.f;
+                }
+            }
+        }
     }
 }
 
@@ -1196,7 +1209,15 @@ __global__ void __launch_bounds__(1024) kSymRunsReduce(const float* __restrict__
     const int64_t I = blockIdx.x;
     const int r = threadIdx.x & (CT - 1), grp = threadIdx.x >> 6;
     float s = 0.f;
-    for (int64_t q = symRunStart(I) + grp; q < symRunStart(I + 1); q += 16) s += part[q * (2 * CT) + r];
+    // row sums of row block I: at its last tile and at the last tile of every warp's range in it
+    const int64_t T = nb * (nb + 1) / 2, W = symWarps(T), t0 = I * (I + 1) / 2, t1 = t0 + I + 1;
+    if (grp == 0) s = part[(t1 - 1) * (2 * CT) + r];
+    for (int64_t w = ((t0 + 1) * W + T - 1) / T + grp;; w += 16) {  // the first w with symStart(w) > t0
+        const int64_t t = symStart(w, T, W);
+        if (t >= t1) break;
+        s += part[(t - 1) * (2 * CT) + r];
+    }
+#pragma unroll 8
     for (int64_t Ip = I + 1 + grp; Ip < nb; Ip += 16) s += part[(Ip * (Ip + 1) / 2 + I) * (2 * CT) + CT + r];
     red[grp][r] = s;
     __syncthreads();
@@ -1757,7 +1778,8 @@ int launchCoarseSolve(const LaunchCtx& c, CoarseInv<T> Kinv, int64_t n, const in
         return 2;
     } else {
         const int64_t nb = coarseBlocks(n);
-        kSymRuns<<<(unsigned)symRunStart(nb), 256, 0, c.stream>>>(Kinv.K, tmp, part, nb, c.S, checkDone);
+        kSymRuns<<<(unsigned)std::min<int64_t>((coarseTiles(n) + SYM_WARPS - 1) / SYM_WARPS, SYM_BLOCKS), 32 * SYM_WARPS, 0,
+                   c.stream>>>(Kinv.K, tmp, part, nb, c.S, checkDone);
         kSymRunsReduce<<<(unsigned)nb, 1024, 0, c.stream>>>(part, nb, n, freeDof, Kinv.scale, zc, c.S, checkDone);
         return 3;
     }
