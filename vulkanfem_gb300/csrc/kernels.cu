@@ -1559,37 +1559,43 @@ cudaError_t setKernelAttributes() {
     return cudaFuncSetAttribute(kMatvec<float>, A, s32);
 }
 
-// Node layers of a product block.  About 32, in equal parts, where that gives two
-// blocks an SM (128^3: 33 instead of 32, which left a fifth part of one layer; FP32
-// with the direction update 72 -> 70 us; 16 to 64 layers measure within 3% on
-// larger grids).  Smaller grids take the part count with the least (layers +
-// repeated layer and prologue) x (blocks an SM holds, at least `sat`: that many
-// share an SM without slowing each other): 33 x 17 x 17 nodes 24.6 -> 12.3 us, 65^3
-// 39 -> 21 us.
-int productLayers(const Grid& g, int sat) {
+// Node layers a product block marches: the part count with the least (layers + repeated
+// layer, prologue and epilogue) x (blocks an SM gets, at least `sat`: that many share an
+// SM without slowing each other).  FP64 at every size, about 32 layers before -> this, us:
+// 129^3 nodes 119 -> 88 (380 blocks left a fourth of them to a second wave; 285 don't),
+// 193^3 248 -> 242, 225^3 390 -> 377, 257^3 539 -> 527.
+int marchLayers(const Grid& g, int sat) {
     const int64_t tiles = (int64_t)((g.nx + MV_TX - 2) / (MV_TX - 1)) * ((g.ny + MV_TY - 2) / (MV_TY - 1));
-    int parts = std::max(1, (g.nz + MV_ZC / 2) / MV_ZC);
-    if (tiles * parts >= 2 * 152) return (g.nz + parts - 1) / parts;
     int best = g.nz;
     double least = 1e300;
-    for (parts = 1; 2 * parts <= g.nz + 1; ++parts) {
+    for (int parts = std::max(1, g.nz / 64); 2 * parts <= g.nz + 1; ++parts) {
         const int zc = (g.nz + parts - 1) / parts;
         const double perSm = std::ceil((double)(tiles * ((g.nz + zc - 1) / zc)) / 152.0);
-        const double cost = (zc + 1.5) * std::max((double)sat, perSm);
+        const double cost = (zc + 3.0) * std::max((double)sat, perSm);
         if (cost < least) {
             least = cost;
             best = zc;
         }
-        if (perSm > 8.0) break;
+        if ((perSm > 8.0 && zc < 16) || perSm > 32.0) break;
     }
     return best;
+}
+
+// FP32: about 32 layers, in equal parts, where that gives two blocks an SM; longer
+// marches wait on memory longer (with the direction update, 33 layers / marchLayers: 129^3
+// 69.5 / 74 us, 193^3 187 / 213).  Smaller grids take marchLayers: 33 x 17 x 17 nodes
+// 24.6 -> 12.3 us, 65^3 39 -> 21 us.
+inline int productLayers(const Grid& g) {
+    const int64_t tiles = (int64_t)((g.nx + MV_TX - 2) / (MV_TX - 1)) * ((g.ny + MV_TY - 2) / (MV_TY - 1));
+    const int parts = std::max(1, (g.nz + MV_ZC / 2) / MV_ZC);
+    return tiles * parts >= 2 * 152 ? (g.nz + parts - 1) / parts : marchLayers(g, 2);
 }
 
 // FP32 products with a structured Ke take the cube's constants where it is one.
 template <typename T>
 int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, const void* opconst, const float* cube) {
     const Grid& g = a.g;
-    const int zc = structured ? productLayers(g, 2) : MV_ZC;
+    const int zc = structured ? productLayers(g) : MV_ZC;
     dim3 grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + MV_TY - 2) / (MV_TY - 1), (g.nz + zc - 1) / zc);
     dim3 block(MV_TX, MV_TY);
     size_t smem = (size_t)(kSuElems + kSyElems) * sizeof(T);
@@ -1621,7 +1627,7 @@ int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, co
 
 int launchMatvecPX(const LaunchCtx& c, const MatvecArgs<float>& a, const float* opconst, const float* cube) {
     const Grid& g = a.g;
-    const int zc = productLayers(g, 2);
+    const int zc = productLayers(g);
     dim3 grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + MV_TY - 2) / (MV_TY - 1), (g.nz + zc - 1) / zc);
     dim3 block(MV_TX, MV_TY);
     size_t smem = (size_t)(kSuElems + kSyElems) * sizeof(float);

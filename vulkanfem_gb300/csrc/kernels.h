@@ -126,7 +126,7 @@ cudaError_t setKernelAttributes();
 template <typename T>
 int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, const void* opconst,
                  const float* cube);
-int productLayers(const Grid& g, int sat);  // node layers a product block marches
+int marchLayers(const Grid& g, int sat);  // node layers a product block marches
 
 // The 8 constants of a cube's Khat (k: a - b, b of the normal strains; the shears; the mode-7
 // terms; (a + b) / 2 and (a - b) / 2 of the bending pairs; a - b, b of the (1,1,1) triple) and C, the

@@ -8,7 +8,7 @@
 // the dot of a node to the FP64 pipe.
 //
 // Measured: 191^3 with voids and log-normal moduli 3.72 -> 0.49 ms; 33 x 17 x 17
-// nodes 262 -> 20 us (shorter marches by productLayers among it); a Ke in another
+// nodes 262 -> 20 us (shorter marches by marchLayers among it); a Ke in another
 // corner order, as the dense 24 x 24 product, 96 x 80 x 72 half full, 1.56 ->
 // 0.26 ms.  Bound now: instruction issue (1,100 warp instructions per element
 // row, 59% of the issue slots, ALU 56%, wide multiply-adds 54% of their pipe)
@@ -567,7 +567,7 @@ bool fxEligible(const FxOperand& op, double scale) {
 
 void launchMatvecFx(cudaStream_t stream, const MatvecArgs<double>& a, const FxOperand& op, const double* opconst,
                     Scalars* S, const RedBuf& rb) {
-    const int zc = productLayers(a.g, op.cube ? 2 : 1);
+    const int zc = marchLayers(a.g, op.cube ? 2 : 1);
     const Grid& g = a.g;
     const dim3 block(MV_TX, FX_TY),
         grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + FX_TY - 2) / (FX_TY - 1), (g.nz + zc - 1) / zc);
