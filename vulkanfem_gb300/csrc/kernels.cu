@@ -545,7 +545,10 @@ struct V4<double> {
 // 16 rows per block beat 32 (a partial last wave of blocks) and a persistent
 // grid taking units from a counter (its per-unit barriers and counter round
 // trips cost more than the wave tail).
-constexpr int PR = 16;
+// 160 threads in 6 blocks an SM against 256 in 4, us, FP32 up-leg to 65^3 nodes 12.7 / 14.4,
+// 97^3 18.5 / 22.2, 161^2 x 145 42.3 / 46.4, 193^3 65.8 / 70.9, 257^3 124.6 / 130.5 (bytes
+// alone 82); 128 threads in 8 63.5 to 193^3 but 144 to 257^3; 10 blocks spill registers.
+constexpr int PR = 16, kProlongThreads = 160;
 constexpr int kProlongCoarseRows = PR / 2 + 1;
 constexpr size_t kProlongFlatMaxSmem = 200 * 1024;
 __host__ __device__ inline int prolongFlatRowGroups(const Grid& gf) { return (gf.ny + PR - 1) / PR; }
@@ -666,7 +669,7 @@ __global__ void __launch_bounds__(256)
 // DT: the type the inverse diagonal is stored in (T, or FP16 scaled so that
 // coef already carries the scale).
 template <typename T, typename DT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kProlongThreads, 6)
     kProlongFlat(Grid gf, Grid gc, const T* __restrict__ zc, const T* __restrict__ rf, const DT* __restrict__ dinv,
                  const uint8_t* __restrict__ flags, T* __restrict__ zf, double coef, int maskFixed,
                  const T* __restrict__ aux, int epi, int vec, float invNx, Scalars* S, RedBuf rb, int checkDone) {
@@ -800,7 +803,7 @@ __global__ void __launch_bounds__(256)
     }
     if (epi != EPI_NONE) {
         double v[2] = {d0.get(), d1.get()}, t[2];
-        if (gridReduce<256, 2>(v, rb, t)) applyEpi(epi, S, t[0], t[1]);
+        if (gridReduce<kProlongThreads, 2>(v, rb, t)) applyEpi(epi, S, t[0], t[1]);
     }
 }
 
@@ -1702,7 +1705,7 @@ int launchProlongSmooth(const LaunchCtx& c, const Grid& gf, const Grid& gc, int 
             }
             if (flatSmem > 48 * 1024)
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProlongFlatMaxSmem);
-            kern<<<(unsigned)flatBlocksN, 256, flatSmem, c.stream>>>(gf, gc, zc, rf, dptr, flags, zf, cf, maskFixed, aux,
+            kern<<<(unsigned)flatBlocksN, kProlongThreads, flatSmem, c.stream>>>(gf, gc, zc, rf, dptr, flags, zf, cf, maskFixed, aux,
                                                                      epi, vec, 1.0f / gf.nx, c.S, c.rb, checkDone);
         };
         if constexpr (std::is_same<T, float>::value) {
