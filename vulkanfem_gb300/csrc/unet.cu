@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <string>
@@ -682,6 +683,20 @@ cudaError_t nalloc(T** p, int64_t n) {
     return cudaStreamSynchronize(cudaStreamLegacy);
 }
 
+// A kernel's set-up on each device it is launched on (a kernel's attributes belong to one
+// device): make() on the first launch there, its result (not 0) afterwards.
+struct PerDevice {
+    std::atomic<int> value[64] = {};
+    template <typename F>
+    int get(F make) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return make();
+        int v = value[dev].load(std::memory_order_acquire);
+        if (!v) value[dev].store(v = make(), std::memory_order_release);
+        return v;
+    }
+};
+
 // One convolution at level lvl: (Cin, Cout) as the network has them, forward and data gradient.
 // TZ: 8 x 8 x 4 tiles, or 8 x 8 x 2 where the halo is large (Cin >= 128) or the level
 // has too few voxels to fill the GPU's 152 SMs with the taller ones.
@@ -691,12 +706,13 @@ void launchConv(vfem_net* N, const Input& in, const bf16* W, const float* b, con
     constexpr size_t smem = convSmem<CK, NT, TG, TZ>();
     static_assert(smem <= 227 * 1024, "tile too large");
     auto kern = kConv<CK, NT, TG, TZ, OUT>;
-    static const int perSm = [&] {
+    static PerDevice blocksPerSm;
+    const int perSm = blocksPerSm.get([&] {
         int k = 0;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, 64 * TZ, smem);
         return std::max(1, k);
-    }();
+    });
     const int tx = (n + 7) / 8, tiles = tx * tx * ((n + TZ - 1) / TZ), parts = std::max(1, Cout / (8 * NT) / (OUT == OUT_PRED ? 2 : 1));
     const dim3 grid((unsigned)std::min(tiles, std::max(1, 152 * perSm / parts)), (unsigned)parts);
     kern<<<grid, 64 * TZ, smem, N->stream>>>(in, W, b, act, out, n, Cout, relu);
@@ -780,9 +796,11 @@ int wgChunks(int64_t V) { return (int)((V + WG_CHUNK - 1) / WG_CHUNK); }
 
 template <int MT, int NT>
 void launchWGrad(vfem_net* N, const Input& in, const bf16* g, int n, int Cout, int chunks) {
-    static const cudaError_t attr = cudaFuncSetAttribute(kWGrad<MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         wgSmem<MT, NT>());
-    (void)attr;
+    static PerDevice ready;
+    ready.get([] {
+        cudaFuncSetAttribute(kWGrad<MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgSmem<MT, NT>());
+        return 1;
+    });
     const dim3 grid((unsigned)chunks, (unsigned)((in.Ca + in.Cb) / (16 * MT) * (Cout / (8 * NT))), 3);
     const unsigned long long mul = ((1ull << 40) + n - 1) / n;
     kWGrad<MT, NT><<<grid, WG_THREADS, wgSmem<MT, NT>(), N->stream>>>(in, g, N->wgPart, n, mul, Cout);
