@@ -61,7 +61,7 @@ typedef enum vfem_mg_mode {
 typedef enum vfem_precision {
     VFEM_PREC_FP64 = 0,     /* plain FP64 MG-PCG */
     VFEM_PREC_MIXED = 1     /* FP32 CG + FP32 V-cycle, FP64 reductions, FP64 solution accumulation,
-                               true residual f - K x in double-float arithmetic substituted for the
+                               true residual f - K x, FP64-accurate, substituted for the
                                recursive one (reliable updates, `replace_delta`, `replace_every`)
                                and checked at exit */
 } vfem_precision;
@@ -265,7 +265,7 @@ typedef enum vfem_kernel_class {
     VFEM_K_UPDATE_P_FP32 = 9,     /* mixed: p = z + beta p with the deferred x += alpha p */
     VFEM_K_COARSE_FP64 = 10,
     VFEM_K_COARSE_FP32 = 11,
-    VFEM_K_TRUE_RESIDUAL_DF = 12, /* f - K x on FP64 vectors in double-float arithmetic */
+    VFEM_K_TRUE_RESIDUAL_DF = 12, /* f - K x on FP64 vectors (block fixed point for a cube's Ke) */
     VFEM_K_UPDATE_RESTRICT_MIXED = 13, /* mixed: r -= alpha Ap, r.r and the first restriction in one pass */
     VFEM_K_MATVEC_FP32_SIMT = 14, /* the FP32 CG product on the CUDA cores, whichever product the problem uses */
     VFEM_K_MATVEC_FP32_PX = 15,   /* the mixed solve's FP32 CG product with the direction update (p = z + beta p,

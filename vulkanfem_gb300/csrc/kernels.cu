@@ -5,14 +5,16 @@
 //   kMatvecH, kMatvec  MatxVec.comp + FixedNodes.comp + VecDotVec.comp
 //                    (MatrixFreeSparse.hpp:197-214): atomic-free element-by-element
 //                    product on a 2.5-D tile (kMatvecH: Walsh-factorised isotropic
-//                    cube Ke; kMatvec: general Ke), fixed rows zeroed, dots fused.
-//   kRestrict2, kRestrict  CWiseMult.comp + Restrict.comp (MultigridPreconditioner.hpp:67-108):
+//                    cube Ke; kMatvec: general Ke; FP64 mostly in matvec_fx.cu), fixed
+//                    rows zeroed, dots fused.
+//   kRestrict2, kRestrict64, kRestrictSmall, kRestrict  CWiseMult.comp + Restrict.comp (MultigridPreconditioner.hpp:67-108):
 //                    full weighting on the dense grid (kRestrict2<T, true> also
 //                    performs the mixed solve's residual update, ConjugateGradient_1.comp).
-//   kProlongFlat, kProlongSmooth2, kProlongSmooth  Interpolate.comp + PreSmoothAndAXPY.comp +
+//   kProlongFlat, kProlong64, kProlongSmall, kProlongSmooth2, kProlongSmooth
+//                    Interpolate.comp + PreSmoothAndAXPY.comp +
 //                    Smooth.comp (MultigridPreconditioner.hpp:110-155,176-181),
 //                    fixed mask and r.z fused.
-//   kCoarseGather/kSymRuns/kSymRunsReduce, kGemv64  the coarsest SimplicialLDLT solve
+//   kCoarseSmall, kCoarseGather/kSymRuns/kSymRunsReduce, kGemv64  the coarsest SimplicialLDLT solve
 //                    (MultigridPreconditioner.hpp:174-175) as a dense symmetric
 //                    inverse: FP16 packed half tiles (mixed) or the full FP64 matrix.
 //   kUpdateXR, kUpdateR  ConjugateGradient_1.comp + VecDotVec.comp (r.r).
@@ -979,21 +981,21 @@ __global__ void __launch_bounds__(256) kGemv64(const double* __restrict__ K, int
 // -> 24.7 / 8.3, n = 3,993 44.2 / 18.0 -> 47.2 / 12.3, where FP64 is better off with
 // kGemv64 and the mixed form, at twice the bytes of the packed half, would soon be
 // with that: hence kSmallCoarse.
-__device__ __forceinline__ void smallRow(const __half* k, const float* b, int n, int lane, float (&acc)[4]) {
+__device__ __forceinline__ float smallRow(const __half* k, const float* b, int n, int lane) {
+    float2 acc[4] = {};
     for (int j = 8 * lane; j < n; j += 256) {
         const uint4 q = *reinterpret_cast<const uint4*>(k + j);
         const float4 b0 = *reinterpret_cast<const float4*>(b + j), b1 = *reinterpret_cast<const float4*>(b + j + 4);
-        const float2 k0 = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
-        const float2 k1 = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
-        const float2 k2 = __half22float2(*reinterpret_cast<const __half2*>(&q.z));
-        const float2 k3 = __half22float2(*reinterpret_cast<const __half2*>(&q.w));
-        acc[0] = fmaf(k0.x, b0.x, fmaf(k2.x, b1.x, acc[0]));
-        acc[1] = fmaf(k0.y, b0.y, fmaf(k2.y, b1.y, acc[1]));
-        acc[2] = fmaf(k1.x, b0.z, fmaf(k3.x, b1.z, acc[2]));
-        acc[3] = fmaf(k1.y, b0.w, fmaf(k3.y, b1.w, acc[3]));
+        acc[0] = __ffma2_rn(__half22float2(*reinterpret_cast<const __half2*>(&q.x)), make_float2(b0.x, b0.y), acc[0]);
+        acc[1] = __ffma2_rn(__half22float2(*reinterpret_cast<const __half2*>(&q.y)), make_float2(b0.z, b0.w), acc[1]);
+        acc[2] = __ffma2_rn(__half22float2(*reinterpret_cast<const __half2*>(&q.z)), make_float2(b1.x, b1.y), acc[2]);
+        acc[3] = __ffma2_rn(__half22float2(*reinterpret_cast<const __half2*>(&q.w)), make_float2(b1.z, b1.w), acc[3]);
     }
+    const float2 s = __fadd2_rn(__fadd2_rn(acc[0], acc[1]), __fadd2_rn(acc[2], acc[3]));
+    return s.x + s.y;
 }
-__device__ __forceinline__ void smallRow(const double* k, const double* b, int n, int lane, double (&acc)[4]) {
+__device__ __forceinline__ double smallRow(const double* k, const double* b, int n, int lane) {
+    double acc[4] = {};
     int j = lane;
     for (; j + 96 < n; j += 128) {
 #pragma unroll
@@ -1002,6 +1004,7 @@ __device__ __forceinline__ void smallRow(const double* k, const double* b, int n
 #pragma unroll
     for (int q = 0; q < 3; ++q)
         if (j + 32 * q < n) acc[q] = fma(k[j + 32 * q], b[j + 32 * q], acc[q]);
+    return (acc[0] + acc[1]) + (acc[2] + acc[3]);
 }
 template <typename T, typename KT>
 __global__ void __launch_bounds__(256) kCoarseSmall(const KT* __restrict__ K, int n, int ld, T scale,
@@ -1013,9 +1016,7 @@ __global__ void __launch_bounds__(256) kCoarseSmall(const KT* __restrict__ K, in
     __syncthreads();
     const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= n) return;
-    T acc[4] = {T(0), T(0), T(0), T(0)};
-    smallRow(K + (int64_t)row * ld, b, n, lane, acc);
-    T sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    T sum = smallRow(K + (int64_t)row * ld, b, n, lane);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if (lane == 0) zc[freeDof[row]] = sum * scale;
