@@ -653,11 +653,14 @@ __device__ __forceinline__ int walshMarch(const MatvecArgs<T>& a, const KP& kp, 
             const int64_t s = (int64_t)oCol + (int64_t)k * plane;
             if constexpr (OUT == OUT_CG || OUT == OUT_CG_PX) {
                 const bool fixed = (fl & FLAG_FIXED) != 0;
+                // FP64: x is the caller's (vfem_apply_operator_device_noalloc) and may hold anything
+                // at unused nodes; the FP32 solver's own vectors hold 0 there and at fixed nodes
+                const bool live = std::is_same<T, float>::value || ((fl & FLAG_USED) && !fixed);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     const TC out = fixed ? TC(0) : sum[c];
                     a.y[3 * s + c] = C::out(out);
-                    dAx = fma(xo[c], out, dAx);
+                    if (live) dAx = fma(xo[c], out, dAx);
                 }
             } else if constexpr (OUT == OUT_TRUE) {
                 const bool fixed = (fl & FLAG_FIXED) != 0;
