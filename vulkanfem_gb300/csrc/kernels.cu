@@ -5,8 +5,8 @@
 //   kMatvecH, kMatvec  MatxVec.comp + FixedNodes.comp + VecDotVec.comp
 //                    (MatrixFreeSparse.hpp:197-214): atomic-free element-by-element
 //                    product on a 2.5-D tile (kMatvecH: Walsh-factorised isotropic
-//                    cube Ke; kMatvec: general Ke; FP64 mostly in matvec_fx.cu), fixed
-//                    rows zeroed, dots fused.
+//                    cube Ke; kMatvec: general Ke; FP64 in matvec_fx.cu where the Ke allows
+//                    it), fixed rows zeroed, dots fused.
 //   kRestrict2, kRestrict64, kRestrictSmall, kRestrict  CWiseMult.comp + Restrict.comp (MultigridPreconditioner.hpp:67-108):
 //                    full weighting on the dense grid (kRestrict2<T, true> also
 //                    performs the mixed solve's residual update, ConjugateGradient_1.comp).
@@ -44,12 +44,12 @@ constexpr int PZ = 8;  // z nodes per thread in the per-node kernels
 // and the grid reduction of its dots.
 template <typename T, typename TC = T>
 __global__ void __launch_bounds__(MV_TX* MV_TY, 1)
-    kMatvec(MatvecArgs<T> a, const Kd<TC> kp, Scalars* S, RedBuf rb) {
+    kMatvec(MatvecArgs<T> a, const Kd<TC> kp, int layers, Scalars* S, RedBuf rb) {
     if (a.checkDone && S->done) return;
     if (a.condTrue && !trueResidualDue(S)) return;
     extern __shared__ __align__(16) unsigned char smemRaw[];
     DotAcc<TC> d0, d1;
-    denseMarch<T, TC>(a, kp, smemRaw, d0, d1);
+    denseMarch<T, TC>(a, kp, smemRaw, d0, d1, layers);
     if (a.epi != EPI_NONE) {
         double v[2] = {d0.get(), d1.get()}, t[2];
         if (gridReduce<MV_TX * MV_TY, 2>(v, rb, t)) applyEpi(a.epi, S, t[0], t[1]);
@@ -1595,11 +1595,19 @@ inline int productLayers(const Grid& g) {
     return tiles * parts >= 2 * 152 ? (g.nz + parts - 1) / parts : marchLayers(g, 2);
 }
 
+// Layers of a march in the products of one type: the FP64 marches are bound by their
+// operations, so marchLayers on every grid, with the blocks that share an SM.
+template <typename T>
+inline int layersFor(const Grid& g, bool structured) {
+    if (std::is_same<T, double>::value) return marchLayers(g, structured ? 2 : 1);
+    return structured ? productLayers(g) : MV_ZC;
+}
+
 // FP32 products with a structured Ke take the cube's constants where it is one.
 template <typename T>
 int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, const void* opconst, const float* cube) {
     const Grid& g = a.g;
-    const int zc = structured ? productLayers(g) : MV_ZC;
+    const int zc = layersFor<T>(g, structured);
     dim3 grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + MV_TY - 2) / (MV_TY - 1), (g.nz + zc - 1) / zc);
     dim3 block(MV_TX, MV_TY);
     size_t smem = (size_t)(kSuElems + kSyElems) * sizeof(T);
@@ -1624,7 +1632,7 @@ int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, co
         Kd<T> k;
         const T* src = static_cast<const T*>(opconst) + 45;
         for (int i = 0; i < 576; ++i) k.v[i] = src[i];
-        kMatvec<T><<<grid, block, smem, c.stream>>>(a, k, c.S, c.rb);
+        kMatvec<T><<<grid, block, smem, c.stream>>>(a, k, zc, c.S, c.rb);
     }
     return 1;
 }
@@ -1995,16 +2003,18 @@ cudaError_t launchMatvecNoAlloc(cudaStream_t s, const MatvecArgs<double>& a, boo
     b.condTrue = 0;
     size_t smem = (size_t)(kSuElems + kSyElems) * sizeof(double);
     dim3 block(MV_TX, MV_TY);
+    const int zc = layersFor<double>(g, structured);
+    grid.z = (g.nz + zc - 1) / zc;
     if (fxEligible(fx, b.scale)) {
         launchMatvecFx(s, b, fx, static_cast<const double*>(opconst), S, rb);
     } else if (structured) {
         Ks<double> k;
         for (int i = 0; i < 45; ++i) k.v[i] = static_cast<const double*>(opconst)[i];
-        kMatvecH<double, double><<<grid, block, smem, s>>>(b, k, MV_ZC, S, rb);
+        kMatvecH<double, double><<<grid, block, smem, s>>>(b, k, zc, S, rb);
     } else {
         Kd<double> k;
         for (int i = 0; i < 576; ++i) k.v[i] = static_cast<const double*>(opconst)[45 + i];
-        kMatvec<double><<<grid, block, smem, s>>>(b, k, S, rb);
+        kMatvec<double><<<grid, block, smem, s>>>(b, k, zc, S, rb);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return cudaMemcpyAsync(xKx, &S->red0, sizeof(double), cudaMemcpyDeviceToDevice, s);

@@ -134,9 +134,10 @@ int marchLayers(const Grid& g, int sat);  // node layers a product block marches
 bool cubeConstants(const KeData& ke, double (&k)[8], double& C);
 
 // The FP64 product in block fixed point (matvec_fx.cu): the 8 constants of a
-// cube's Ke, or the 576 entries of any other, as 62-bit integers.  fxEligible:
-// the operand is ready and `scale` a power of two.  opconst: the problem's
-// 45 + 576 FP64 constants.
+// cube's Ke, or the 576 entries of another whose entries all couple at one scale
+// (fxPrepare), as 62-bit integers.  fxEligible: the operand is ready and `scale` a
+// power of two; other products run the FP64 marches (launchMatvec).  opconst: the
+// problem's 45 + 576 FP64 constants.
 struct FxOperand {
     int32_t k1[576], k0[576];
     int outExp;

@@ -1,5 +1,8 @@
 // matvec_fx.cu -- the FP64 product in block fixed point.
 //
+// Two forms: the cube's 8 constants in the Walsh basis, and the dense 24 x 24 matrix
+// for a Ke in another corner order (which matrices: fxPrepare).
+//
 // GB300 issues FP64 at 1/64 of its FP32 rate: measured 1.7 FP64 operations per
 // clock and SM against 58 64-bit integer additions and 29 multiply-adds 32 x 32
 // -> 64.  The FP64 marches (walshMarch and denseMarch, matvec_march.cuh) are
@@ -19,8 +22,8 @@
 //
 // Numbers.  A node's three components are staged as 58-bit integers under the
 // node's largest exponent.  An element reads its 24 values on a grid S with
-// S - 3 <= (exponent of its largest value) <= S and 2^-57 of 2^S as the unit;
-// the Walsh transforms are then exact.  The largest of the 20 combinations that
+// S - 3 <= (exponent of its largest value) <= S (dense: S) and 2^-57 of 2^S as the
+// unit; the Walsh transforms are then exact.  The largest of the 20 combinations that
 // Khat scales is shifted up to 2^61..2^62 (lz), multiplied by 62-bit constants
 // in two 32-bit digits, and by the modulus' 24-bit significand, with rounding;
 // what leaves the element has the unit 2^(O + 9 - f), O = S + exponent(E) - lz,
@@ -28,8 +31,8 @@
 // Outputs with different O are aligned to the larger one where they meet.
 // Against 113-bit arithmetic the result's relative error is 3e-16 to 6e-16
 // (random, smooth, graded and point vectors, moduli 1, log-normal or spread
-// over e^20), where the FP64 march has 5e-16 to 4e-15; the dense form's 5e-17 to
-// 8e-16, where the FP64 one has 1e-16 to 2.5e-15.
+// over e^20), where the FP64 march has 5e-16 to 4e-15; the dense form's, for the
+// matrices it takes, 5e-17 to 8e-16, where the FP64 one has 1e-16 to 2.5e-15.
 //
 // No sum can overflow: the combinations are below 2^62, so a component's corner
 // value is at most C 2^f 2^62 / 2^64 / 2 <= 2^59 per element, and a node sums 8
@@ -249,7 +252,7 @@ __device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const KA& K
         int nO = cO;
         if (__any_sync(0xffffffffu, act)) {
             if constexpr (DENSE) {
-                if (act && (el > S || S > el + FX_SLACK)) S = el + 1;
+                if (act) S = el;  // no quad is carried, so the finest grid each time
             } else if (act && (el > S || S > el + FX_SLACK || qS != S)) {
                 longlong2 vb[4];
                 quadB(k & 1, vb);
@@ -534,16 +537,33 @@ bool cubeConstants(const KeData& ke, double (&k)[8], double& C) {
     return true;
 }
 
+// The integer forms round every constant to one unit and every value of an element to
+// one grid.  For a cube that is what the FP64 march's Walsh transforms do as well, and
+// the constants themselves are sums rounded at 2^-53 of the largest entry.  The dense
+// FP64 march keeps each product Ke_rc u_c to its own 53 bits, so the dense integers take
+// only a Ke whose rows can't tell: every value reaches every row (no entry below the
+// largest row sum / 256).  An error of 2^-56 of C max|u| is then within 2^-48 of any
+// row's own sum |Ke_rc u_c|, the bound of the 26 roundings of an FP64 row.  Measured on
+// random, graded and point vectors with one value 1e9 times the others, largest error
+// over that sum, dense integers / FP64: ratio 126 2^-49.4 / 2^-49.4, 236 2^-48.6 /
+// 2^-49.6, 2,396 2^-45.2 / 2^-49.4.  Rows of another scale, uncoupled components or
+// corners and single zeros (the cube's at nu = 1/4) go to the FP64 marches, as does a Ke
+// with the 45-entry pattern that is not a cube's.
 bool fxPrepare(const KeData& ke, FxOperand& op) {
     double k[8], C = 0.0;
     op.cube = cubeConstants(ke, k, C);
     if (op.cube) return op.ready = fxDigits(k, 8, C, 0, op.k1, op.k0, op.outExp);
+    if (ke.structured) return op.ready = false;
+    double least = std::fabs(ke.Ke[0]);
     for (int r = 0; r < 24; ++r) {
         double row = 0.0;
-        for (int c = 0; c < 24; ++c) row += std::fabs(ke.Ke[24 * r + c]);
+        for (int c = 0; c < 24; ++c) {
+            row += std::fabs(ke.Ke[24 * r + c]);
+            least = std::fmin(least, std::fabs(ke.Ke[24 * r + c]));
+        }
         C = std::fmax(C, row);
     }
-    return op.ready = fxDigits(ke.Ke, 576, C, 3, op.k1, op.k0, op.outExp);
+    return op.ready = C <= 256.0 * least && fxDigits(ke.Ke, 576, C, 3, op.k1, op.k0, op.outExp);
 }
 
 cudaError_t fxSetAttributes() {

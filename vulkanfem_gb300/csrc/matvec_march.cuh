@@ -148,8 +148,7 @@ __device__ __forceinline__ void ldSlot<double>(const double* p, double& a, doubl
 // no element touches) cannot reach the dot.
 template <typename T, typename TC>
 __device__ __forceinline__ void mvOutput(const MatvecArgs<T>& a, int64_t s, const TC (&sum)[3], uint8_t fl,
-                                         const TC (&xo)[3], DotAcc<TC>& d0, DotAcc<TC>& d1,
-                                          [[maybe_unused]] int layers = MV_ZC) {
+                                         const TC (&xo)[3], DotAcc<TC>& d0, DotAcc<TC>& d1) {
     typedef Cvt<T, TC> C;
     const bool fixed = (fl & FLAG_FIXED) != 0;
     const bool live = (fl & FLAG_USED) && !fixed;
