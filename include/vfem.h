@@ -265,7 +265,7 @@ typedef enum vfem_kernel_class {
     VFEM_K_UPDATE_P_FP32 = 9,     /* mixed: p = z + beta p with the deferred x += alpha p */
     VFEM_K_COARSE_FP64 = 10,
     VFEM_K_COARSE_FP32 = 11,
-    VFEM_K_TRUE_RESIDUAL_DF = 12, /* f - K x on FP64 vectors (as the FP64 product computes it) */
+    VFEM_K_TRUE_RESIDUAL_DF = 12, /* the mixed solve's f - K x on FP64 vectors: fixed point, else double-float */
     VFEM_K_UPDATE_RESTRICT_MIXED = 13, /* mixed: r -= alpha Ap, r.r and the first restriction in one pass */
     VFEM_K_MATVEC_FP32_SIMT = 14, /* the FP32 CG product on the CUDA cores, whichever product the problem uses */
     VFEM_K_MATVEC_FP32_PX = 15,   /* the mixed solve's FP32 CG product with the direction update (p = z + beta p,

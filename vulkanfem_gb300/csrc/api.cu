@@ -144,7 +144,7 @@ struct vfem_problem {
     float op32[45 + 576];
     float cube32[8];     // a cube's constants for the FP32 products (Kc in matvec_march.cuh)
     bool isCube = false;
-    FxOperand fx;  // the structured FP64 product in block fixed point (matvec_fx.cu)
+    FxOperand fx;  // the FP64 product in block fixed point, where the Ke allows it (matvec_fx.cu)
     // the tensor-core FP32 CG product (matvec_tc.cu), opt-in, when Ke admits an exact BF16 scaling
     TcOperand tc;
     bool tcReady = false;
@@ -850,6 +850,13 @@ int matvec(vfem_problem* p, const MatvecArgs<T>& a, bool allowTc = true) {
     return launchMatvec<T>(ctx(p), a, p->ke.structured, opc<T>(p), p->isCube ? p->cube32 : nullptr);
 }
 
+// The mixed solve's residual on FP64 vectors: the FP64 product where that runs in fixed
+// point, else double-float (257^3 nodes: 1.2 ms, 2.7; the FP64 march 8.9).
+int matvecMixedResidual(vfem_problem* p, const MatvecArgs<double>& a) {
+    if (fxEligible(p->fx, a.scale)) return matvec<double>(p, a);
+    return launchMatvecDF(ctx(p), a, p->ke.structured, p->op64);
+}
+
 // z = M^-1 r on level `lv` (r, z given); returns kernels; on level 0 the final
 // pass produces r.z (and z.aux) with epilogue `epi`.  *outZ receives the buffer
 // holding the result (it differs from z in the multiplicative cycle when the
@@ -1015,7 +1022,7 @@ int iteration(vfem_problem* p, const vfem_options& o, double** zOut64, float** z
         t.dot0 = DOT_OUT_OUT;
         t.epi = EPI_TRUE;
         t.condTrue = 1;
-        k += matvec<double>(p, t);
+        k += matvecMixedResidual(p, t);
         // a replaced residual is restricted again
         if (fused) k += launchRestrict<float>(c, l0.g, p->L[1].g, 2, r, p->L[1].r32, 2);
         float* z = nullptr;
@@ -1061,7 +1068,7 @@ vfem_status solvePhase(vfem_problem* p, const vfem_options& o, bool haveX0, vfem
         a.f = p->f64;
         a.checkDone = 0;
         if (mixed) a.y32 = l0.r32;
-        launches += matvec<double>(p, a);
+        launches += mixed ? matvecMixedResidual(p, a) : matvec<double>(p, a);
     } else {
         launches += launchFill<double>(p->stream, n, p->x64, 0.0);
         launches += launchConvert<double, double>(p->stream, n, p->f64, l0.r64);
@@ -1697,7 +1704,7 @@ vfem_status vfem_profile_kernels(vfem_problem* p, int32_t reps, double* ms) {
                     a.y32 = l0.t32;
                     a.dot0 = DOT_OUT_OUT;
                     a.epi = EPI_STORE;
-                    return matvec<double>(p, a);
+                    return matvecMixedResidual(p, a);
                 }
             }
         };

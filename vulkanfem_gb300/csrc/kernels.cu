@@ -1560,6 +1560,10 @@ cudaError_t setKernelAttributes() {
     if ((e = cudaFuncSetAttribute(kMatvecH<float, float, OUT_CG_PX, Kc<float>>, A, s32))) return e;
     if ((e = cudaFuncSetAttribute(kMatvecH<double, double, OUT_CG>, A, s64))) return e;
     if ((e = cudaFuncSetAttribute(kMatvec<double>, A, s64))) return e;
+    static_assert(sizeof(df) == sizeof(double), "the same shared memory");
+    if ((e = cudaFuncSetAttribute(kMatvecH<double, df, OUT_TRUE>, A, s64))) return e;
+    if ((e = cudaFuncSetAttribute(kMatvecH<double, df>, A, s64))) return e;
+    if ((e = cudaFuncSetAttribute(kMatvec<double, df>, A, s64))) return e;
     return cudaFuncSetAttribute(kMatvec<float>, A, s32);
 }
 
@@ -1633,6 +1637,27 @@ int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, co
         const T* src = static_cast<const T*>(opconst) + 45;
         for (int i = 0; i < 576; ++i) k.v[i] = src[i];
         kMatvec<T><<<grid, block, smem, c.stream>>>(a, k, zc, c.S, c.rb);
+    }
+    return 1;
+}
+
+int launchMatvecDF(const LaunchCtx& c, const MatvecArgs<double>& a, bool structured, const double* opconst) {
+    const Grid& g = a.g;
+    const int zc = layersFor<float>(g, structured);  // its operations are FP32's
+    dim3 grid((g.nx + MV_TX - 2) / (MV_TX - 1), (g.ny + MV_TY - 2) / (MV_TY - 1), (g.nz + zc - 1) / zc);
+    dim3 block(MV_TX, MV_TY);
+    const size_t smem = (size_t)(kSuElems + kSyElems) * sizeof(df);
+    if (structured) {
+        Ks<df> k;
+        for (int i = 0; i < 45; ++i) k.v[i] = df(opconst[i]);
+        if (a.mode == MV_RESID && a.dot0 == DOT_OUT_OUT && !a.dot1 && a.y32)
+            kMatvecH<double, df, OUT_TRUE><<<grid, block, smem, c.stream>>>(a, k, zc, c.S, c.rb);
+        else
+            kMatvecH<double, df><<<grid, block, smem, c.stream>>>(a, k, zc, c.S, c.rb);
+    } else {
+        Kd<df> k;
+        for (int i = 0; i < 576; ++i) k.v[i] = df(opconst[45 + i]);
+        kMatvec<double, df><<<grid, block, smem, c.stream>>>(a, k, zc, c.S, c.rb);
     }
     return 1;
 }

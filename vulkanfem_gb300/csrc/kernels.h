@@ -126,6 +126,10 @@ cudaError_t setKernelAttributes();
 template <typename T>
 int launchMatvec(const LaunchCtx& c, const MatvecArgs<T>& a, bool structured, const void* opconst,
                  const float* cube);
+// The product on FP64 vectors in double-float arithmetic (FP32 instructions, ~48-bit
+// significands): the mixed solve's true residual where the FP64 product is not in
+// fixed point.  a.y may be null.
+int launchMatvecDF(const LaunchCtx& c, const MatvecArgs<double>& a, bool structured, const double* opconst);
 int marchLayers(const Grid& g, int sat);  // node layers a product block marches
 
 // The 8 constants of a cube's Khat (k: a - b, b of the normal strains; the shears; the mode-7

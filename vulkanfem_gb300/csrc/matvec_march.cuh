@@ -1,13 +1,14 @@
 // matvec_march.cuh -- the element-by-element product's building blocks shared by
 // its translation units: the Walsh-basis and dense element products, the output
-// stage and the march up a z range (kernels.cu: FP32 and FP64 kernels;
-// matvec_fx.cu: the fixed-point FP64 product, which hands blocks it cannot
-// represent to the FP64 march).  Everything here has
+// stage and the march up a z range (kernels.cu: FP32, FP64 and double-float
+// kernels; matvec_fx.cu: the fixed-point FP64 product, which hands blocks it
+// cannot represent to the FP64 march).  Everything here has
 // internal linkage (one copy per translation unit).
 #pragma once
 
 #include <type_traits>
 
+#include "double_float.cuh"
 #include "kernels.h"
 #include "reduce.cuh"
 
@@ -16,7 +17,7 @@ namespace {
 
 constexpr int MV_TX = 32, MV_TY = 8, MV_ZC = 32;  // z layers per product block (32: 5% faster than 16)
 
-// One name for both FP32 and FP64 multiply-adds in the templates below.
+// One name for FP32, FP64 and double-float multiply-adds in the templates below.
 __device__ __forceinline__ float fma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma(double a, double b, double c) { return ::fma(a, b, c); }
 
@@ -26,8 +27,24 @@ struct Cvt {
     static __device__ __forceinline__ TC in(T v) { return TC(v); }
     static __device__ __forceinline__ T out(TC v) { return T(v); }
 };
+template <>
+struct Cvt<double, df> {
+    static __device__ __forceinline__ df in(double v) {
+        const float h = __double2float_rn(v);
+        return df(h, __double2float_rn(v - (double)h));
+    }
+    static __device__ __forceinline__ double out(df v) { return (double)v.hi + (double)v.lo; }
+};
 __device__ __forceinline__ float toF(float v) { return v; }
 __device__ __forceinline__ float toF(double v) { return (float)v; }
+__device__ __forceinline__ float toF(df v) { return v.hi; }  // hi is v rounded to FP32
+
+template <>
+struct DotAcc<df> {
+    df s = df(0.f, 0.f);
+    __device__ __forceinline__ void add(df v) { s = s + v; }
+    __device__ __forceinline__ double get() const { return (double)s.hi + (double)s.lo; }
+};
 
 template <typename T>
 struct Ks {
@@ -124,8 +141,20 @@ __device__ __forceinline__ void stSlot<double>(double* p, double a, double b, do
     reinterpret_cast<double2*>(p)[0] = make_double2(a, b);
     reinterpret_cast<double2*>(p)[1] = make_double2(c, 0.0);
 }
+template <>
+__device__ __forceinline__ void stSlot<df>(df* p, df a, df b, df c) {
+    reinterpret_cast<float4*>(p)[0] = make_float4(a.hi, a.lo, b.hi, b.lo);
+    reinterpret_cast<float4*>(p)[1] = make_float4(c.hi, c.lo, 0.f, 0.f);
+}
 template <typename T>
 __device__ __forceinline__ void ldSlot(const T* p, T& a, T& b, T& c);
+template <>
+__device__ __forceinline__ void ldSlot<df>(const df* p, df& a, df& b, df& c) {
+    const float4 v0 = reinterpret_cast<const float4*>(p)[0], v1 = reinterpret_cast<const float4*>(p)[1];
+    a = df(v0.x, v0.y);
+    b = df(v0.z, v0.w);
+    c = df(v1.x, v1.y);
+}
 template <>
 __device__ __forceinline__ void ldSlot<float>(const float* p, float& a, float& b, float& c) {
     const float4 v = *reinterpret_cast<const float4*>(p);
@@ -190,7 +219,8 @@ __device__ __forceinline__ void mvOutput(const MatvecArgs<T>& a, int64_t s, cons
 // loaded without integer division: every thread loads its own slot, row 8
 // comes from the ty == 0 threads and column 32 from nine threads of row 1.
 //
-// T is the storage type of the vectors, TC the arithmetic type.
+// T is the storage type of the vectors, TC the arithmetic type (T, or df for the
+// true residual of the mixed-precision solve: FP64 vectors, df arithmetic).
 // One block's march: fills d0 and d1 (this thread's dots).
 template <typename T, typename TC>
 __device__ __forceinline__ void denseMarch(const MatvecArgs<T>& a, const Kd<TC>& kp, unsigned char* smemRaw,
@@ -446,7 +476,7 @@ __device__ __forceinline__ void foldCarry<float>(const float (&y)[24], float (&c
 // Same tile, pipelining and output stage as kMatvec.  The two Walsh-domain
 // carries stay in registers across the z march.  Launch bounds, measured on
 // the 256^3 workload: FP32 3 blocks per SM (80 registers, no spills; 4 blocks
-// spill and run 33% slower); FP64 2 blocks per SM (128 registers, a few
+// spill and run 33% slower); FP64 and df 2 blocks per SM (128 registers, a few
 // spilled values; 20% faster than 1 block without spills).
 //
 // OUT selects the output stage at compile time (runtime mode switches in the
