@@ -34,10 +34,21 @@
 // over e^20), where the FP64 march has 5e-16 to 4e-15; the dense form's, for the
 // matrices it takes, 5e-17 to 8e-16, where the FP64 one has 1e-16 to 2.5e-15.
 //
-// No sum can overflow: the combinations are below 2^62, so a component's corner
-// value is at most C 2^f 2^62 / 2^64 / 2 <= 2^59 per element, and a node sums 8
-// of them; sums in between are taken modulo 2^64.  A middle digit sum has at
-// most two (dense: 24, hence the coarser k0) products of 2^61 and 2^62 besides.  Values the grid cannot take
+// What the common grid does not keep: where one component's values are so equal, or have
+// so few bits, that FP64 sums them without rounding (a rigid translation), FP64 keeps the
+// other components' digits below it and the grid does not: x = 1e6 at every node beside
+// random y and z, 2e-12 relative against 1e-16.  With rounded values in the large
+// component FP64 loses them as well (1e6 + random: 2e-12 against 1.2e-11).  Taking such
+// elements' modes from exact differences, out of line, cost the march its registers
+// (191^3 0.49 -> 0.74 ms).
+//
+// No sum overflows.  Staged values are below 2^58 (S = the largest exponent), modes below
+// 2^61, sums of two below 2^62, of three below 3 x 2^61; where lz > 0 all are below 2^62.  A
+// component's corner value is then at most C 2^f (3 x 2^61) / 2^64 / 2 <= 3 x 2^58 per element,
+// a node's 8 of them 3 x 2^61; sums in between are taken modulo 2^64.  A middle digit
+// sum has one product with k0 (at most 2^30 2^31) and one with k1 (with its start in
+// kb at most 2^32 |k1|, |k1| <= 2^30); the threes' has two of each, fxPrepare checks
+// their constants; the dense form's 24, hence its coarser k0.  Values the grid cannot take
 // (non-finite ones or exponents beyond 2^+-575 next to a filled voxel, subnormal
 // moduli) make the block repeat its march in FP64, so that results for those
 // are what the FP64 march gives.
@@ -508,6 +519,15 @@ bool fxDigits(const double* k, int n, double C, int low, int32_t* k1, int32_t* k
     outExp = 9 - f - 1023 - 127;
     return true;
 }
+
+// The middle digit sum of `three` for constants j and j + 1: the common product with j + 1
+// of up to 3 x 2^61 beside an own one of 2^61, or both of 2^62 (digits of 2^32).
+bool threeFits(const FxOperand& op, int j) {
+    const double own = std::fabs((double)op.k0[j]), sum = std::fabs((double)op.k0[j + 1]);
+    const double lead = std::fabs((double)op.k1[j]) + std::fabs((double)op.k1[j + 1]);
+    const double w = 0x1p30 + 1.0;
+    return std::fmax(1.5 * w * sum + 0.5 * w * own, w * (sum + own)) + 0x1p32 * lead + 0x1p31 < 0x1p63;
+}
 }  // namespace
 
 // Khat of a cube, whose axes are interchangeable, has one constant per kind of
@@ -552,7 +572,8 @@ bool cubeConstants(const KeData& ke, double (&k)[8], double& C) {
 bool fxPrepare(const KeData& ke, FxOperand& op) {
     double k[8], C = 0.0;
     op.cube = cubeConstants(ke, k, C);
-    if (op.cube) return op.ready = fxDigits(k, 8, C, 0, op.k1, op.k0, op.outExp);
+    if (op.cube)
+        return op.ready = fxDigits(k, 8, C, 0, op.k1, op.k0, op.outExp) && threeFits(op, 0) && threeFits(op, 6);
     if (ke.structured) return op.ready = false;
     double least = std::fabs(ke.Ke[0]);
     for (int r = 0; r < 24; ++r) {
