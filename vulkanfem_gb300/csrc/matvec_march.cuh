@@ -482,8 +482,9 @@ __device__ __forceinline__ void foldCarry<float>(const float (&y)[24], float (&c
 // OUT selects the output stage at compile time (runtime mode switches in the
 // owner stage cost ~20% of this issue-bound kernel):
 //   OUT_ANY   mvOutput with the runtime mode and dots;
-//   OUT_CG    the CG product: y = Kx (fixed rows 0), dot x.(Kx); the per-thread
-//             dot sums at most 48 terms and accumulates with plain FMAs;
+//   OUT_CG    the CG product: y = Kx (fixed rows 0), dot x.(Kx); a thread adds its nodes'
+//             sums of three plainly, up to 47 layers in FP32 (productLayers): a chain of
+//             50 roundings, where a term at a time had 96 in marches of 32;
 //   OUT_TRUE  the true residual: r = f - Kx, its FP32 rounding to y32, y (FP64)
 //             only when given, dot r.r;
 //   OUT_CG_PX the CG product with the mixed solve's direction update fused into
@@ -496,9 +497,8 @@ __device__ __forceinline__ void foldCarry<float>(const float (&y)[24], float (&c
 //             p_old as their halo.
 enum MvOut : int { OUT_ANY = 0, OUT_CG = 1, OUT_TRUE = 2, OUT_CG_PX = 3 };
 
-// The march of one block of 32 x 8 threads over its node layers (MV_ZC;
-// `layers` in FP64, where the fixed-point product's blocks share the march): fills d0 and d1 (this
-// thread's dots) and returns the p buffer read (OUT_CG_PX).
+// The march of one block of 32 x 8 threads over its `layers` node layers: fills d0 and d1
+// (this thread's dots) and returns the p buffer read (OUT_CG_PX).
 template <typename T, typename TC, int OUT, typename KP>
 __device__ __forceinline__ int walshMarch(const MatvecArgs<T>& a, const KP& kp, Scalars* S,
                                            unsigned char* smemRaw, DotAcc<TC>& d0, DotAcc<TC>& d1,
@@ -685,12 +685,14 @@ __device__ __forceinline__ int walshMarch(const MatvecArgs<T>& a, const KP& kp, 
                 // FP64: x is the caller's (vfem_apply_operator_device_noalloc) and may hold anything
                 // at unused nodes; the FP32 solver's own vectors hold 0 there and at fixed nodes
                 const bool live = std::is_same<T, float>::value || ((fl & FLAG_USED) && !fixed);
+                TC node = TC(0);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     const TC out = fixed ? TC(0) : sum[c];
                     a.y[3 * s + c] = C::out(out);
-                    if (live) dAx = fma(xo[c], out, dAx);
+                    node = c == 0 ? xo[c] * out : fma(xo[c], out, node);
                 }
+                if (live) dAx += node;
             } else if constexpr (OUT == OUT_TRUE) {
                 const bool fixed = (fl & FLAG_FIXED) != 0;
 #pragma unroll
