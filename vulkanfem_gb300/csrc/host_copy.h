@@ -10,7 +10,7 @@
 //     maps them, without changing what they hold, while the kernels run.
 //   - large arrays: from about 250 MB the GPU's translations no longer stay
 //     cached from call to call (377 MB: 2 to 48 ms for the same copy).  Above
-//     kDirectMax copies go through PinnedRing, 8 threads and the DMA overlapped,
+//     kDirectMax copies go through PinnedRing, host threads and the DMA overlapped,
 //     which takes the same time every time (377 MB: 2.9 ms in, about 6 out).
 #pragma once
 
@@ -22,12 +22,26 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <system_error>
 #include <thread>
 #include <vector>
 
 namespace vfem {
+
+// Threads that host copies and page mapping may use: 8, or VFEM_HOST_COPY_THREADS (read once),
+// and no more than the machine has.
+inline size_t hostCopyThreads() {
+    static const size_t n = [] {
+        const char* v = std::getenv("VFEM_HOST_COPY_THREADS");
+        char* end = nullptr;
+        const long long x = v && *v ? std::strtoll(v, &end, 10) : 8;
+        const long long want = end && *end ? 8 : std::max(1ll, x);
+        return (size_t)std::min<long long>(want, std::max(1u, std::thread::hardware_concurrency()));
+    }();
+    return n;
+}
 
 // Maps [p, p + bytes) writable (MADV_POPULATE_WRITE, Linux 5.14).  A kernel without it
 // leaves the pages to fault on use.
@@ -38,13 +52,12 @@ inline void populatePages(void* p, size_t bytes) {
     if (bytes) (void)madvise((void*)a, e - a, kPopulateWrite);
 }
 
-// The same on up to 8 threads of 4 MB or more, done when wait() or the destructor returns.
+// The same on up to hostCopyThreads() threads of 4 MB or more, done when wait() or the destructor returns.
 class PopulateTask {
    public:
     PopulateTask(void* p, size_t bytes) {
         constexpr size_t kSlice = (size_t)4 << 20;
-        const size_t hw = std::max(1u, std::thread::hardware_concurrency());
-        const size_t n = std::min<size_t>({8, hw, (bytes + kSlice - 1) / kSlice});
+        const size_t n = std::min(hostCopyThreads(), (bytes + kSlice - 1) / kSlice);
         if (n <= 1) {
             populatePages(p, bytes);
             return;
@@ -136,7 +149,7 @@ class PinnedRing {
 
    private:
     static constexpr size_t kChunk = (size_t)8 << 20;
-    static constexpr int kSlots = 4, kThreads = 8;
+    static constexpr int kSlots = 4;
     char* buf_ = nullptr;
     cudaEvent_t ev_[kSlots] = {};
 
@@ -158,7 +171,7 @@ class PinnedRing {
         Workers(int n, Copy copy, size_t bytes) : n_(n), copy_(copy), bytes_(bytes), done_(n) {
             for (auto& d : done_) d.store(0);
             try {
-                for (int t = 0; t < kThreads; ++t) threads_.emplace_back([this, t] { run(t); });
+                for (int t = 0; t < (int)hostCopyThreads(); ++t) threads_.emplace_back([this, t] { run(t); });
             } catch (const std::system_error&) {
             }
             count_.store(threads_.empty() ? -1 : (int)threads_.size(), std::memory_order_release);
