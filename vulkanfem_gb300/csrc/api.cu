@@ -1369,6 +1369,10 @@ vfem_status vfem_solve(vfem_problem* p, const vfem_options* opt, const double* u
     if (!p->rhsSet) return fail(VFEM_ERR_INVALID_ARGUMENT, "right-hand side not set");
     CK(cudaSetDevice(p->device));
     if (st) std::memset(st, 0, sizeof(*st));
+    if (opt) {  // before the copy of u0 is on its way
+        vfem_status s0 = checkOptions(*opt);
+        if (s0 != VFEM_OK) return s0;
+    }
     if (u0) {
         vfem_status s0 = toDenseHost(p, 0, u0, p->x64, false);
         if (s0 != VFEM_OK) return s0;
@@ -1379,6 +1383,8 @@ vfem_status vfem_solve(vfem_problem* p, const vfem_options* opt, const double* u
     if (s == VFEM_OK || s == VFEM_ERR_NOT_CONVERGED) {
         vfem_status s2 = fromDenseHost(p, 0, p->x64, u_out);
         if (s2 != VFEM_OK) return s2;
+    } else if (u0) {
+        cudaStreamSynchronize(p->stream);  // a solve that failed in its set-up: u0 may still be read
     }
     return s;
 }
