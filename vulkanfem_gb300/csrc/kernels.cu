@@ -860,6 +860,13 @@ __global__ void __launch_bounds__(NTH)
     const int64_t j1 = (nBeg + nb + CH - 1) / CH;
     double d0 = 0.0, d1 = 0.0;
     bool staged = false;
+    // sums of 2^1022 and more, which may overflow over x: the block halves every sum instead
+    bool big = false;
+    int halved = 0;
+    auto watch = [&](double s) {
+        big = big || (__double2hiint(s) & 0x7ff00000) >= (2045 << 20);
+        return s;
+    };
     for (int64_t j = nBeg / CH + threadIdx.x;; j += NTH) {
         const bool have = j < j1;
         const int64_t n0 = CH * j;
@@ -896,11 +903,19 @@ __global__ void __launch_bounds__(NTH)
             asm volatile("cp.async.wait_all;\n" ::: "memory");
             __syncthreads();
             if (zodd) {
-                for (int q = threadIdx.x; q < nstage; q += NTH) C[q] += C[nstage + q];
+                for (int q = threadIdx.x; q < nstage; q += NTH) C[q] = watch(C[q] + C[nstage + q]);
                 __syncthreads();
             }
-            for (int q = threadIdx.x; q < nsum; q += NTH) C[nstage + q] = C[q] + C[q + cw];
-            __syncthreads();
+            for (int q = threadIdx.x; q < nsum; q += NTH) C[nstage + q] = watch(C[q] + C[q + cw]);
+            halved = __syncthreads_or(big);
+            if (halved) {
+                const double* src = zc + 3 * gc.store(0, cy0, cz);
+                const int64_t up = 3 * ((int64_t)gc.nx * gc.ny);
+                for (int q = threadIdx.x; q < nstage; q += NTH) C[q] = zodd ? 0.5 * (src[q] + src[up + q]) : src[q];
+                __syncthreads();
+                for (int q = threadIdx.x; q < nsum; q += NTH) C[nstage + q] = 0.5 * (C[q] + C[q + cw]);
+                __syncthreads();
+            }
             staged = true;
         }
         if (!have) break;
@@ -919,7 +934,7 @@ __global__ void __launch_bounds__(NTH)
                 const bool used = (fl & FLAG_USED) != 0;
                 const bool zero = !used || (maskFixed && (fl & FLAG_FIXED));
                 const double* b = C + ((ly & 1) ? nstage : 0) + (ly >> 1) * cw + 3 * (fx >> 1);
-                const int k = (int)zodd + (ly & 1) + (fx & 1);
+                const int k = (halved ? 0 : (int)zodd + (ly & 1)) + (fx & 1);
                 double pv[3] = {b[0], b[1], b[2]};
                 if (fx & 1) {
 #pragma unroll
