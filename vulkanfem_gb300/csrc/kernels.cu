@@ -1476,6 +1476,15 @@ __global__ void kFill(int64_t n, T* __restrict__ y, T v) {
         y[i] = v;
 }
 
+// Values between -1 and 1 without a pattern (a multiplicative hash) at used nodes.
+__global__ void kNoise(int64_t n, const uint8_t* __restrict__ flags, double* __restrict__ y) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        unsigned h = (unsigned)i * 2654435761u;
+        h = (h ^ (h >> 15)) * 2246822519u;
+        y[i] = (flags[i / 3] & FLAG_USED) ? (double)(int)(h ^ (h >> 13)) * 0x1p-31 : 0.0;
+    }
+}
+
 template <typename T>
 __global__ void kScatterCompressed(int64_t nn, const int32_t* __restrict__ store, const double* __restrict__ comp,
                                    T* __restrict__ dense, unsigned* bad) {
@@ -1584,9 +1593,11 @@ cudaError_t setKernelAttributes() {
 
 // Node layers a product block marches: the part count with the least (layers + repeated
 // layer, prologue and epilogue) x (blocks an SM gets, at least `sat`: that many share an
-// SM without slowing each other).  FP64 at every size, about 32 layers before -> this, us:
-// 129^3 nodes 119 -> 88 (380 blocks left a fourth of them to a second wave; 285 don't),
-// 193^3 248 -> 242, 225^3 390 -> 377, 257^3 539 -> 527.
+// SM without slowing each other).  FP64 at every size, us with parts of up to 32 layers / this /
+// the best of 15 lengths from 6 to 65, boxes with voids and moduli, random vectors:
+// 65^3 nodes 68 / 45 / 47, 97^3 111 / 94 / 94, 129^3 197 / 180 / 179, 161^3 322 / 320 /
+// 311, 193^3 486 / 496 / 486, 225^3 750 / 742 / 742, 257^3 1,077 / 1,050 / 1,050; the dense form 217 /
+// 138 / 138, 466 / 386 / 385, 896 / 789 / 788, 1,480 / 1,444 / 1,435 (to 161^3).
 int marchLayers(const Grid& g, int sat) {
     const int64_t tiles = (int64_t)((g.nx + MV_TX - 2) / (MV_TX - 1)) * ((g.ny + MV_TY - 2) / (MV_TY - 1));
     int best = g.nz;
@@ -1926,6 +1937,11 @@ int launchConvert(cudaStream_t s, int64_t n, const TI* x, TO* y) {
 template <typename T>
 int launchFill(cudaStream_t s, int64_t n, T* y, T v) {
     kFill<T><<<flatBlocks(n), NT, 0, s>>>(n, y, v);
+    return 1;
+}
+
+int launchNoise(cudaStream_t s, int64_t n, const uint8_t* flags, double* y) {
+    kNoise<<<flatBlocks(n), NT, 0, s>>>(n, flags, y);
     return 1;
 }
 

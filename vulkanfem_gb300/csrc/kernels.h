@@ -249,6 +249,8 @@ template <typename TI, typename TO>
 int launchConvert(cudaStream_t s, int64_t n, const TI* x, TO* y);
 template <typename T>
 int launchFill(cudaStream_t s, int64_t n, T* y, T v);
+// noise between -1 and 1 at used nodes, 0 elsewhere
+int launchNoise(cudaStream_t s, int64_t n, const uint8_t* flags, double* y);
 
 // compressed <-> dense storage
 template <typename T>
