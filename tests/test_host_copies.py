@@ -26,3 +26,10 @@ def test_copies_and_thread_bound(program, setting, threads):
     r = subprocess.run([program], env=env, capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
     assert 1 <= int(r.stdout) <= 1 + min(threads, os.cpu_count())
+
+
+@pytest.mark.parametrize("allocations", [0, 1, 2, 3, 5, 60])
+def test_without_memory_for_threads(program, allocations):
+    """No exception leaves the copies, which are called from C entries."""
+    r = subprocess.run([program, str(allocations)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr

@@ -24,7 +24,8 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
-#include <system_error>
+#include <exception>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -68,8 +69,8 @@ class PopulateTask {
             const size_t len = std::min(each, bytes - i * each);
             try {
                 threads_.emplace_back([s, len] { populatePages(s, len); });
-            } catch (const std::system_error&) {
-                populatePages(s, len);  // no thread to be had
+            } catch (const std::exception&) {
+                populatePages(s, len);  // no thread (or no memory for one) to be had
             }
         }
     }
@@ -172,7 +173,7 @@ class PinnedRing {
             for (auto& d : done_) d.store(0);
             try {
                 for (int t = 0; t < (int)hostCopyThreads(); ++t) threads_.emplace_back([this, t] { run(t); });
-            } catch (const std::system_error&) {
+            } catch (const std::exception&) {
             }
             count_.store(threads_.empty() ? -1 : (int)threads_.size(), std::memory_order_release);
         }
@@ -217,16 +218,25 @@ class PinnedRing {
     };
 };
 
-// The caller's array to the device, ordered on the stream.
+// The caller's array to the device, ordered on the stream.  (Neither copy throws: they are called from C entries.)
 inline cudaError_t copyToDevice(PinnedRing& ring, void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    return bytes > kDirectMax ? ring.toDevice(dst, src, bytes, st)
-                              : cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    try {
+        return bytes > kDirectMax ? ring.toDevice(dst, src, bytes, st)
+                                  : cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    } catch (const std::bad_alloc&) {
+        return cudaErrorMemoryAllocation;
+    }
 }
 // Results to the caller's array; complete on return.
 inline cudaError_t copyToHost(PinnedRing& ring, void* dst, const void* src, size_t bytes, cudaStream_t st) {
     PopulateTask(dst, bytes).wait();  // while the kernels before it run
-    const cudaError_t e = bytes > kDirectMax ? ring.toHost(dst, src, bytes, st)
-                                             : cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+    cudaError_t e;
+    try {
+        e = bytes > kDirectMax ? ring.toHost(dst, src, bytes, st)
+                               : cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+    } catch (const std::bad_alloc&) {
+        return cudaErrorMemoryAllocation;
+    }
     return e != cudaSuccess ? e : cudaStreamSynchronize(st);
 }
 
