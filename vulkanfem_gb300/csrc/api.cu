@@ -850,8 +850,9 @@ int matvec(vfem_problem* p, const MatvecArgs<T>& a, bool allowTc = true) {
     return launchMatvec<T>(ctx(p), a, p->ke.structured, opc<T>(p), p->isCube ? p->cube32 : nullptr);
 }
 
-// The mixed solve's residual on FP64 vectors: the FP64 product where that runs in fixed
-// point, else double-float (257^3 nodes: 1.2 ms, 2.7; the FP64 march 8.9).
+// The mixed solve's residual on FP64 vectors: the FP64 product where that runs in fixed point
+// (257^3 nodes, a cube: 1.15 ms), else double-float (brick-shaped voxels 2.65 ms, the FP64
+// march 7.9; without the pattern 19.0 and 26.8).
 int matvecMixedResidual(vfem_problem* p, const MatvecArgs<double>& a) {
     if (fxEligible(p->fx, a.scale)) return matvec<double>(p, a);
     return launchMatvecDF(ctx(p), a, p->ke.structured, p->op64);

@@ -3,7 +3,7 @@
 // TwoSum / FastTwoSum; the product error from one FMA).  GB300 issues FP64 at about
 // 1/64 of its FP32 rate, so the mixed-precision solve evaluates its true residual
 // f - K x in df where the FP64 product is not in fixed point: relative rounding
-// ~1e-14 of the summed magnitudes, 3 times faster than the FP64 march.  Addition is
+// ~1e-14 of the summed magnitudes, 3 times faster than the FP64 march (dense Ke 1.4).  Addition is
 // the "sloppy" variant (error bounded by ~2^-44 (|a| + |b|)), ample for a residual
 // that is compared with 1e-6 |f|.  The compiler must not re-associate these
 // expressions, which nvcc does not do without fast-math flags.
