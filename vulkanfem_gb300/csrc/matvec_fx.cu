@@ -34,13 +34,16 @@
 // over e^20), where the FP64 march has 5e-16 to 4e-15; the dense form's, for the
 // matrices it takes, 5e-17 to 8e-16, where the FP64 one has 1e-16 to 2.5e-15.
 //
-// What the common grid does not keep: where one component's values are so equal, or have
-// so few bits, that FP64 sums them without rounding (a rigid translation), FP64 keeps the
-// other components' digits below it and the grid does not: x = 1e6 at every node beside
-// random y and z, 2e-12 relative against 1e-16.  With rounded values in the large
-// component FP64 loses them as well (1e6 + random: 2e-12 against 1.2e-11).  Taking such
-// elements' modes from exact differences, out of line, cost the march its registers
-// (191^3 0.49 -> 0.74 ms).
+// The common grid cuts off what components have below 2^-57 of the largest value.  FP64
+// rounds its Walsh sums there as well (x = 1e6 + random beside random y and z: 2e-12
+// relative, FP64 1.2e-11), unless that component sums without rounding, as a rigid
+// translation does (x = 1e6: 2e-12 against 1e-16).  A block with an element whose largest
+// combination is below 2^43 units (2^-18 of the grid's top) therefore looks at its elements
+// again (fxRepeat) and repeats in FP64 for such components; otherwise the cut-offs, up to 48
+// units, stay below 2^-37 of the largest combination, typically 2^-41.  191^3 492 us and
+// a 64^3 FP64 solve 117.9 ms, as without; FP64 solves of slender beams (512 x 16 x 16) 2% slower,
+// 5% with 2^-16; with 2^-14 the 64^3 solve 3%.  The march is at its 128 registers: noted in
+// another form the same test spilled there (191^3 532 us).
 //
 // No sum overflows.  Staged values are below 2^58 (S = the largest exponent), modes below
 // 2^61, sums of two below 2^62, of three below 3 x 2^61; where lz > 0 all are below 2^62.  A
@@ -65,6 +68,7 @@ constexpr int FX_EMIN = 448, FX_EMAX = 1600;  // biased exponents the integer ma
 constexpr int FX_BAD = 4000;                  // a node outside of them
 constexpr int FX_NONE = -(1 << 20);           // exponent of a zero contribution
 constexpr int FX_SLACK = 3;
+constexpr int FX_FAR = 18;                    // combinations below 2^-18 of the grid: fxRepeat looks closer
 
 // Constants times 2^f = k1 2^32 + k0, signed digits.  kb: start of a middle digit
 // sum, 2^31 (rounding) + 2^31 k1.
@@ -143,10 +147,10 @@ constexpr size_t fxSmemBytes() {
 
 // One block's march, the counterpart of walshMarch<double, double, OUT> (KA =
 // FxArgs) and denseMarch<double, double> (FxDenseArgs) with the same tile, halo
-// and pipelining.  Returns true when a value did not fit (the outputs and dots
-// are then to be recomputed).  The dense form has the 24 values themselves in
-// place of the Walsh combinations and reads both quads every layer, to keep
-// their digits in registers.
+// and pipelining.  Returns true when a value did not fit, so that the outputs and dots are to be
+// recomputed, or an element's strains were small against its grid: fxAgain finds out.  The
+// dense form has the 24 values themselves in place of the Walsh combinations and reads both
+// quads every layer, to keep their digits in registers.
 template <int OUT, int TY, typename KA>
 __device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const KA& K, int zc, unsigned char* smem,
                                         DotAcc<double>& d0, DotAcc<double>& d1) {
@@ -337,6 +341,7 @@ __device__ __forceinline__ bool fxMarch(const MatvecArgs<double>& a, const KA& K
                 unsigned mag = 0;
 #pragma unroll
                 for (int i = 0; i < 20; ++i) mag |= spread(v[i]);
+                if (mag < (1u << (29 - FX_FAR))) bad = bad || act;  // (in this form: no spills)
                 const int lz = max(__clz((int)mag) - 2, 0);
                 cO = act ? S + (eBits >> 23) + K.scaleExp - lz : FX_NONE;
                 // k_j v 2^lz in 2^64 units as a leading (A) and a middle digit sum (B)
@@ -480,6 +485,63 @@ __device__ __noinline__ void fp64March(const MatvecArgs<double>* a, const Kd<dou
     denseMarch<double, double>(*a, *kp, smem, d[0], d[1], zc);
 }
 
+// Whether the block is to repeat its march in FP64 for one of this thread's elements: a value
+// or modulus that the grid cannot take, or digits that FP64 keeps and the grid cuts off: a
+// component whose FP64 sums are exact (the same value at all corners, or values of few bits) is
+// large, and another has digits below the grid's unit.  Components that FP64 rounds at the
+// same place (the usual case) are no reason.
+__device__ __noinline__ bool fxRepeat(const MatvecArgs<double>* a, int zc) {
+    const Grid g = a->g;
+    const int ex = (int)blockIdx.x * (MV_TX - 1) + (int)threadIdx.x - 1;
+    const int ey = (int)blockIdx.y * (MV_TY - 1) + (int)threadIdx.y - 1;
+    const int z0 = blockIdx.z * zc;
+    if (ex < 0 || ex >= g.ex || ey < 0 || ey >= g.ey) return false;
+    for (int k = max(z0 - 1, 0); k < min(z0 + zc, g.ez); ++k) {
+        const float E = a->E[g.store(ex, ey, k)];
+        if (E == 0.f) continue;
+        long long first[3];
+        bool equal[3] = {true, true, true};
+        int e[3] = {0, 0, 0}, lo[3] = {1 << 20, 1 << 20, 1 << 20};  // exponents: largest value, lowest digit
+        bool zero = true;
+        for (int q = 0; q < 8; ++q) {
+            int node = 0;
+            bool any = false;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const long long v =
+                    __double_as_longlong(a->x[3 * g.store(ex + (q & 1), ey + ((q >> 1) & 1), k + (q >> 2)) + c]);
+                if (q == 0) first[c] = v;
+                equal[c] = equal[c] && v == first[c];
+                if ((v << 1) == 0) continue;
+                any = true;
+                const int ev = (int)(v >> 52) & 0x7ff;
+                node = max(node, ev);
+                e[c] = max(e[c], ev);
+                lo[c] = min(lo[c], ev - 53 + __ffsll((v & 0xfffffffffffffll) | 0x10000000000000ll));
+            }
+            if (any && (node < FX_EMIN || node > FX_EMAX)) return true;
+            zero = zero && !any;
+        }
+        if (!zero && (__float_as_int(E) >> 23) == 0) return true;
+        int top = 0, rounded = 0, low = 1 << 20;  // largest, largest that FP64 rounds, lowest digit
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            top = max(top, e[c]);
+            if (equal[c]) continue;
+            low = min(low, lo[c]);
+            if (lo[c] < e[c] - 49) rounded = max(rounded, e[c]);  // sums of 8 take more than 53 bits
+        }
+        if (low < top + FX_SLACK - 57 && rounded + 6 < top) return true;
+    }
+    return false;
+}
+
+template <int OUT, typename KP>
+__device__ __noinline__ void fxAgain(const MatvecArgs<double>* a, const KP* kp, int zc, Scalars* S,
+                                     unsigned char* smem, DotAcc<double>* d) {
+    if (__syncthreads_or(fxRepeat(a, zc))) fp64March<OUT>(a, kp, zc, S, smem, d);
+}
+
 constexpr int FX_TY = MV_TY;
 
 template <int OUT, typename KA, typename KP>
@@ -491,7 +553,7 @@ __global__ void __launch_bounds__(MV_TX* FX_TY, std::is_same<KA, FxArgs>::value 
     extern __shared__ __align__(16) unsigned char smemRaw[];
     DotAcc<double> d[2];
     if (__syncthreads_or(fxMarch<OUT, FX_TY>(a, K, zc, smemRaw, d[0], d[1])))
-        fp64March<OUT>(&a, &kp, zc, S, smemRaw, d);
+        fxAgain<OUT, KP>(&a, &kp, zc, S, smemRaw, d);
     if (a.epi != EPI_NONE) {
         double v[2] = {d[0].get(), d[1].get()}, t[2];
         if (gridReduce<MV_TX * FX_TY, 2>(v, rb, t)) applyEpi(a.epi, S, t[0], t[1]);
